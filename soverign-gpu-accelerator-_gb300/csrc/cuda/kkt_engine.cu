@@ -265,148 +265,339 @@ __global__ void k_asm_cols_dense(int M, const int* __restrict__ rp, const int* _
 // ------------------------------------------------------------------- factor
 
 // Cholesky of the 64x64 diagonal tile of step k of one front, in the front's
-// precision T, plus the explicit inverse of the factored tile (used by the panel
-// solve and by both triangular solves), stored column-major in Linv.
-// Blocked by 16 columns so that the block-wide barriers are few: warp 0 factors
-// each 16x16 diagonal block (warp-synchronous), one thread per row solves the
-// panel below it, and all threads apply the trailing update. The inverse: four
-// warps invert the four diagonal blocks, then block rows of L^{-1} follow as
-// X_ij = -X_ii (sum_k L_ik X_kj). A partial tile is padded with the identity.
+// precision. A partial tile is padded with the identity. This runs in one block on the
+// critical path of every 64-column step, by blocks of 16 columns: the 16x16 diagonal
+// block, the rows below it, the trailing update.
+constexpr int kPB = 16;
+constexpr int kPBTri = kPB * (kPB + 1) / 2;
+
+__device__ __noinline__ void report_pivot(int s, const PlanDev& pd, int* err) {
+    if ((threadIdx.x & 31) != 0) return;
+    if (atomicCAS(err, 0, 1) == 0) err[1] = s;
+    pd.lp_fail[pd.sn_lp[s]] = 1;
+}
+
+// Entry e of the lower triangle that starts at c0 + 16, less the 16 columns at c0.
 template <class T>
-__device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, T* F, T* __restrict__ Linv,
-                           const int64_t* __restrict__ inv_off, int* err, unsigned char* smraw) {
-    constexpr int B = 16;
-    T* A = reinterpret_cast<T*>(smraw);   // A[r * LDS + c], lower triangle
-    T* X = A + T64 * LDS;                 // L^{-1}, same layout
-    T* rdiag = X + T64 * LDS;             // 1 / L(c, c)
-    const int K = pd.sn_ncols[s];
-    const int LD = pd.sn_lda[s];
-    const int k0 = kstep * T64;
-    const int w = min(T64, K - k0);
-    T* Fs = F + pd.F_off[s];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-#pragma unroll 4
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256;
-        const int r = idx & 63, c = idx >> 6;
-        T x = T(0);
-        if (r < w && c < w && c <= r) x = Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD];
-        else if (r == c) x = T(1);
-        A[r * LDS + c] = x;
-        X[r * LDS + c] = T(0);
+__device__ __forceinline__ void trail_entry(T* A, int c0, int e) {
+    int i, j;
+    tri_index(e, i, j);
+    const T* a = A + (c0 + kPB + i) * LDS + c0;
+    const T* b = A + (c0 + kPB + j) * LDS + c0;
+    T v = a[kPB + j];
+#pragma unroll
+    for (int q = 0; q < kPB; ++q) v -= a[q] * b[q];
+    A[(c0 + kPB + i) * LDS + c0 + kPB + j] = v;
+}
+
+// ---- FP32 tile: L, and its explicit inverse (column-major in Linv) for the panel solve
+// and the triangular solves. Bound by the latency of the pivot chain, so warp 0 factors
+// a diagonal block from registers (shuffles, no barrier) while the other warps apply the
+// previous block's update to the rows below and form the inverse's block rows that are
+// already known. Every entry keeps its ascending sequence of fused multiply-adds, so the
+// result does not depend on the schedule. One tile: 38 -> 20 us.
+
+// The helper warps' own barrier (192 threads).
+__device__ __forceinline__ void helper_sync() { asm volatile("bar.sync 1, 192;" ::: "memory"); }
+
+// Warp 0: the diagonal block at c0; lane (r, h) holds the columns 2k + h of row r. Leaves
+// L in A and 1 / L(c, c) in rdiag. A pivot that is not positive counts as 1 (result true).
+__device__ __forceinline__ bool factor_block(float* A, float* rdiag, int c0) {
+    const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
+    bool bad = false;
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int c = 2 * k + h;
+        v[k] = r >= c ? A[(c0 + r) * LDS + c0 + c] : 0.f;
     }
-    __syncthreads();
-    for (int c0 = 0; c0 < T64; c0 += B) {
-        if (wid == 0) {            // 16x16 diagonal block, lanes 0..15 own its rows
-            const int rr = c0 + (lane & 15);
-            for (int jj = 0; jj < B; ++jj) {
-                const int c = c0 + jj;
-                if (lane == 0) {
-                    T p = A[c * LDS + c];
-                    if (!(p > T(0))) {
-                        if (atomicCAS(err, 0, 1) == 0) err[1] = s;
-                        pd.lp_fail[pd.sn_lp[s]] = 1;
-                        p = T(1);
-                    }
-                    const T d = sqrt(p);
-                    A[c * LDS + c] = d;
-                    rdiag[c] = T(1) / d;
-                }
-                __syncwarp();
-                if (lane < B && rr > c) A[rr * LDS + c] *= rdiag[c];
-                __syncwarp();
-                if (rr > c) {
-                    const T l = A[rr * LDS + c];
-                    for (int cc = c + 1 + (lane >> 4); cc <= rr; cc += 2) A[rr * LDS + cc] -= l * A[cc * LDS + c];
-                }
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        const int t0 = c0 + B, nt = T64 - t0;
-        if (tid < nt) {            // panel row r: X L_kk^T = A_r
-            const int r = t0 + tid;
-            T x[B];
 #pragma unroll
-            for (int jj = 0; jj < B; ++jj) {
-                T v = A[r * LDS + c0 + jj];
+    for (int j = 0; j < kPB; ++j) {
+        const float a = __shfl_sync(0xffffffffu, v[j >> 1], r + 16 * (j & 1));    // column j of every row
+        float p = __shfl_sync(0xffffffffu, v[j >> 1], j + 16 * (j & 1));
+        const bool ok = p > 0.f;
+        bad |= !ok;
+        p = ok ? p : 1.f;
+        const float d = sqrtf(p);
+        const float rd = 1.f / d;
+        const float l = a * rd;
+        if (h == 0 && r >= j) A[(c0 + r) * LDS + c0 + j] = r == j ? d : l;
+        if (lane == 0) rdiag[c0 + j] = rd;
 #pragma unroll
-                for (int q = 0; q < jj; ++q) v -= x[q] * A[(c0 + jj) * LDS + c0 + q];
-                x[jj] = v * rdiag[c0 + jj];
-            }
-#pragma unroll
-            for (int jj = 0; jj < B; ++jj) A[r * LDS + c0 + jj] = x[jj];
-        }
-        __syncthreads();
-        for (int e = tid; e < nt * nt; e += 256) {   // trailing lower triangle
-            const int r = t0 + e / nt, cc = t0 + e % nt;
-            if (cc > r) continue;
-            T v = A[r * LDS + cc];
-#pragma unroll
-            for (int q = 0; q < B; ++q) v -= A[r * LDS + c0 + q] * A[cc * LDS + c0 + q];
-            A[r * LDS + cc] = v;
-        }
-        __syncthreads();
-    }
-#pragma unroll 4
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256;
-        const int r = idx & 63, c = idx >> 6;
-        if (r < w && c < w && c <= r) Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD] = A[r * LDS + c];
-    }
-    // inverse of the diagonal blocks: warp b, lane = column of block b
-    if (wid < T64 / B && lane < B) {
-        const int c0 = wid * B, j = c0 + lane;
-        for (int i = j; i < c0 + B; ++i) {
-            T acc = (i == j) ? T(1) : T(0);
-            for (int q = j; q < i; ++q) acc -= A[i * LDS + q] * X[q * LDS + j];
-            X[i * LDS + j] = acc * rdiag[i];
+        for (int k = j >> 1; k < 8; ++k) {
+            if (2 * k + 1 <= j) continue;
+            const float lc = __shfl_sync(0xffffffffu, l, 2 * k + h);
+            if (2 * k + h > j) v[k] = fmaf(-l, lc, v[k]);
         }
     }
-    __syncthreads();
-    // block rows 1..3: T_ij = sum_{q < r0} L(i, q) X(q, j), then X_ij = -X_ii T_ij
-    for (int r0 = B; r0 < T64; r0 += B) {
-        const int cnt = r0 * B;            // (r0 / B) blocks of 16x16
-        for (int e = tid; e < cnt; e += 256) {
-            const int i = r0 + (e % (B * B)) / B, j = (e / (B * B)) * B + e % B;
-            T acc = T(0);
-            for (int q = (e / (B * B)) * B; q < r0; ++q) acc += A[i * LDS + q] * X[q * LDS + j];
-            X[i * LDS + j] = acc;
-        }
-        __syncthreads();
-        T out[3];
+    return bad;
+}
+
+// Rows below block c0: the block's columns of L, one thread per row.
+__device__ __forceinline__ void panel_rows(float* A, const float* rdiag, int c0, int nt) {
+    if (static_cast<int>(threadIdx.x) >= nt) return;
+    float* row = A + (c0 + kPB + threadIdx.x) * LDS + c0;
+    float x[kPB];
 #pragma unroll
-        for (int u = 0; u < 3; ++u) {
-            const int e = tid + u * 256;
-            out[u] = T(0);
-            if (e < cnt) {
-                const int rr = (e % (B * B)) / B, i = r0 + rr, j = (e / (B * B)) * B + e % B;
-                T acc = T(0);
-                for (int q = 0; q <= rr; ++q) acc += X[i * LDS + r0 + q] * X[(r0 + q) * LDS + j];
-                out[u] = -acc;
-            }
-        }
-        __syncthreads();
+    for (int c = 0; c < kPB; ++c) x[c] = row[c];
 #pragma unroll
-        for (int u = 0; u < 3; ++u) {
-            const int e = tid + u * 256;
-            if (e < cnt) {
-                const int i = r0 + (e % (B * B)) / B, j = (e / (B * B)) * B + e % B;
-                X[i * LDS + j] = out[u];
-            }
-        }
-        __syncthreads();
+    for (int q = 0; q < kPB; ++q) {
+        x[q] = x[q] * rdiag[c0 + q];
+#pragma unroll
+        for (int c = q + 1; c < kPB; ++c) x[c] = fmaf(-x[q], A[(c0 + c) * LDS + c0 + q], x[c]);
     }
-    T* Li = Linv + inv_off[s] + static_cast<int64_t>(kstep) * T64 * T64;
-#pragma unroll 4
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256;
-        const int i = idx & 63, jj = idx >> 6;
-        Li[i + jj * T64] = (i < w && jj < w) ? X[i * LDS + jj] : T(0);
+#pragma unroll
+    for (int c = 0; c < kPB; ++c) row[c] = x[c];
+}
+
+// The inverse's diagonal block at c0: thread j < 16 forms column j.
+__device__ __forceinline__ void inverse_block(const float* A, float* X, const float* rdiag, int c0, int j) {
+    if (j >= kPB) return;
+    float x[kPB];
+#pragma unroll
+    for (int i = 0; i < kPB; ++i) x[i] = i == j ? 1.f : 0.f;
+#pragma unroll
+    for (int q = 0; q < kPB; ++q) {
+        x[q] = x[q] * rdiag[c0 + q];
+#pragma unroll
+        for (int i = q + 1; i < kPB; ++i) x[i] = fmaf(-A[(c0 + i) * LDS + c0 + q], x[q], x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kPB; ++i)
+        if (i >= j) X[(c0 + i) * LDS + c0 + j] = x[i];
+}
+
+// Block row at r0 of the inverse: T(i, j) = sum_{j <= q < r0} L(i, q) X(q, j) for the
+// columns j < r0, kept transposed in X's upper triangle, then X(i, j) = -sum_q
+// X(i, r0 + q) T(r0 + q, j).
+__device__ __forceinline__ void inverse_sums(const float* A, float* X, int r0, int t, int step) {
+    for (int e = t; e < r0 * kPB; e += step) {
+        const int i = r0 + (e % (kPB * kPB)) / kPB, j = (e / (kPB * kPB)) * kPB + e % kPB;
+        float acc = 0.f;
+        for (int q = j; q < r0; ++q) acc += A[i * LDS + q] * X[q * LDS + j];
+        X[j * LDS + i] = acc;
+    }
+}
+__device__ __forceinline__ void inverse_rows(float* X, int r0, int t, int step) {
+    for (int e = t; e < r0 * kPB; e += step) {
+        const int rr = (e % (kPB * kPB)) / kPB, i = r0 + rr, j = (e / (kPB * kPB)) * kPB + e % kPB;
+        float acc = 0.f;
+        for (int q = 0; q <= rr; ++q) acc += X[i * LDS + r0 + q] * X[j * LDS + r0 + q];
+        X[i * LDS + j] = -acc;
     }
 }
 
-constexpr size_t potrf_smem(size_t elem) { return (2 * T64 * LDS + 2 * T64) * elem; }
+__device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, float* F, float* __restrict__ Linv,
+                                        const int64_t* __restrict__ inv_off, int* err, unsigned char* smraw) {
+    float* A = reinterpret_cast<float*>(smraw);   // A[r * LDS + c], lower triangle
+    float* X = A + T64 * LDS;                     // L^{-1}, same layout
+    float* rdiag = X + T64 * LDS;                 // 1 / L(c, c)
+    const int LD = pd.sn_lda[s];
+    const int k0 = kstep * T64;
+    const int w = min(T64, pd.sn_ncols[s] - k0);
+    float* Fs = F + pd.F_off[s];
+    const int tid = threadIdx.x, wid = tid >> 5;
+#pragma unroll 4
+    for (int it = 0; it < 16; ++it) {
+        const int idx = tid + it * 256;
+        const int r = idx & 63, c = idx >> 6;
+        if (c > r) continue;
+        float x = 0.f;
+        if (r < w && c < w) x = Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD];
+        else if (r == c) x = 1.f;
+        A[r * LDS + c] = x;
+    }
+    __syncthreads();
+    const int ht = (wid < 4 ? wid - 1 : wid - 2) * 32 + (tid & 31);   // helpers: warps 1-3 and 5-7
+    for (int c0 = 0; c0 < T64; c0 += kPB) {
+        const int nt = T64 - kPB - c0;
+        if (wid == 0) {
+            if (factor_block(A, rdiag, c0)) report_pivot(s, pd, err);
+        } else if (wid != 4 && c0 > 0) {
+            for (int e = kPBTri + ht; e < (nt + kPB) * (nt + kPB + 1) / 2; e += 192) trail_entry(A, c0 - kPB, e);
+            inverse_block(A, X, rdiag, c0 - kPB, ht);
+            helper_sync();
+            if (c0 > kPB) {
+                inverse_rows(X, c0 - kPB, ht, 192);
+                helper_sync();
+            }
+            inverse_sums(A, X, c0, ht, 192);
+        }
+        __syncthreads();
+        if (nt == 0) break;
+        panel_rows(A, rdiag, c0, nt);
+        __syncthreads();
+        if (tid < kPBTri) trail_entry(A, c0, tid);   // the next diagonal block
+        __syncthreads();
+    }
+    inverse_block(A, X, rdiag, T64 - kPB, tid);
+    __syncthreads();
+    inverse_rows(X, T64 - kPB, tid, 256);
+    __syncthreads();
+    float* Li = Linv + inv_off[s] + static_cast<int64_t>(kstep) * T64 * T64;
+#pragma unroll 4
+    for (int it = 0; it < 16; ++it) {
+        const int idx = tid + it * 256;
+        const int r = idx & 63, c = idx >> 6;
+        const bool in = r < w && c <= r;
+        if (in) Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD] = A[r * LDS + c];
+        Li[r + c * T64] = in ? X[r * LDS + c] : 0.f;
+    }
+}
+
+// ---- FP64 tile: L only (k_trsm_rows forms the inverse beside the panel). A warp's FP64
+// instruction takes 64 cycles of its SM quarter's pipe whatever its active lanes, a
+// dependent one follows at once, and shuffles and shared loads go through the same queue
+// (measured: sqrt 600 cycles, a division 355, a 64-bit shuffle 16). So the tile is bound
+// by the number of FP64 instructions per quarter:
+//  * elimination as a_rc -= (a_rj / p_j) a_cj: only a reciprocal sits between two pivots
+//    (seed of the approximate unit and one third-order step, folded into the product
+//    with the row); the square roots of a block are taken together, off the chain.
+//  * the diagonal block is spread over four warps, one per quarter, that exchange a
+//    column through shared memory: 6 FP64 instructions per column and quarter.
+//  * all eight warps take the rows below and the trailing update.
+// One tile: 116 -> 30 us.
+
+// p > 0 without the FP64 pipe (false for NaN).
+__device__ __forceinline__ bool is_positive(double p) {
+    const long long b = __double_as_longlong(p);
+    return b > 0 && b <= 0x7ff0000000000000LL;
+}
+
+// Threads 0..127: the diagonal block at c0. Thread (r, g) holds the columns g and g + 8
+// of row r. Leaves the Schur complement's columns (L before its scaling) in A's lower
+// triangle, the unit factor's column j in A's upper triangle (row j) and the pivots in
+// piv. col: 2 x 16 values. A pivot that is not positive counts as 1 (result true).
+__device__ __forceinline__ bool factor_block(double* A, double* piv, double* col, int c0) {
+    const int r = threadIdx.x & 15, g = threadIdx.x >> 4, wid = threadIdx.x >> 5;
+    bool bad = false;
+    double v0 = r >= g ? A[(c0 + r) * LDS + c0 + g] : 0.0;
+    double v1 = r >= g + 8 ? A[(c0 + r) * LDS + c0 + g + 8] : 0.0;
+#pragma unroll
+    for (int j = 0; j < kPB; ++j) {
+        double* cb = col + (j & 1) * kPB;
+        if (g == (j & 7)) cb[r] = j < 8 ? v0 : v1;
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        double p = cb[j];
+        const double a = cb[r], b0 = cb[g], b1 = cb[g + 8];
+        const bool ok = is_positive(p);
+        bad |= !ok;
+        p = ok ? p : 1.0;
+        // u = a / p: y0 = 1/p to about 2^-19, e = 1 - p y0, 1/p = y0 (1 + e + e^2 + O(e^3))
+        double y0;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(p));
+        const double e = fma(-p, y0, 1.0);
+        const double w = a * y0;
+        const double u = fma(w, fma(e, e, e), w);
+        if (j + 1 < 8) {
+            if (2 * wid + 1 > j && g > j) v0 = fma(-u, b0, v0);
+            v1 = fma(-u, b1, v1);
+        } else if (2 * wid + 9 > j && g + 8 > j) {
+            v1 = fma(-u, b1, v1);
+        }
+        if (g == 0) {
+            if (r >= j) A[(c0 + r) * LDS + c0 + j] = a;
+            if (r > j) A[(c0 + j) * LDS + c0 + r] = u;
+            if (r == j) piv[c0 + j] = p;
+        }
+    }
+    return bad;
+}
+
+// Rows below block c0, all eight warps: a warp takes 8 rows, lane (r, g) their columns
+// 4k + g. The update with the unit factor needs no pivot's square root, which warp 7
+// takes meanwhile; the columns are scaled after the barrier.
+__device__ __forceinline__ void panel_rows(double* A, double* piv, double* rdiag, int c0, int nt) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int r = c0 + kPB + 8 * wid + (lane & 7), g = lane >> 3;
+    const bool on = 8 * wid < nt;
+    double v[4];
+    if (on) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = A[r * LDS + c0 + 4 * k + g];
+#pragma unroll
+        for (int q = 0; q < kPB - 1; ++q) {
+            const double x = __shfl_sync(0xffffffffu, v[q >> 2], (lane & 7) + 8 * (q & 3));
+#pragma unroll
+            for (int k = q >> 2; k < 4; ++k) {
+                if (4 * k + 3 <= q) continue;
+                if (4 * k + g > q) v[k] = fma(-x, A[(c0 + q) * LDS + c0 + 4 * k + g], v[k]);
+            }
+        }
+    } else if (wid == 7 && lane < kPB) {
+        const double d = sqrt(piv[c0 + lane]);
+        piv[c0 + lane] = d;
+        rdiag[c0 + lane] = 1.0 / d;
+    }
+    __syncthreads();
+    if (on)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) A[r * LDS + c0 + 4 * k + g] = v[k] * rdiag[c0 + 4 * k + g];
+}
+
+// L's own diagonal block at c0, whose columns are still unscaled (t = 0 .. step - 1).
+__device__ __forceinline__ void scale_block(double* A, const double* piv, const double* rdiag, int c0, int t,
+                                            int step) {
+    for (int e = t; e < kPBTri; e += step) {
+        int i, j;
+        tri_index(e, i, j);
+        const int at = (c0 + i) * LDS + c0 + j;
+        A[at] = i == j ? piv[c0 + i] : A[at] * rdiag[c0 + j];
+    }
+}
+
+__device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, double* F, double*, const int64_t*, int* err,
+                                        unsigned char* smraw) {
+    double* A = reinterpret_cast<double*>(smraw);   // A[r * LDS + c]
+    double* rdiag = A + T64 * LDS;                  // 1 / L(c, c)
+    double* piv = rdiag + T64;                      // pivots, then L(c, c)
+    double* col = piv + T64;
+    const int LD = pd.sn_lda[s];
+    const int k0 = kstep * T64;
+    const int w = min(T64, pd.sn_ncols[s] - k0);
+    double* Fs = F + pd.F_off[s];
+    const int tid = threadIdx.x;
+#pragma unroll 4
+    for (int it = 0; it < 16; ++it) {
+        const int idx = tid + it * 256;
+        const int r = idx & 63, c = idx >> 6;
+        if (c > r) continue;
+        double x = 0.0;
+        if (r < w && c < w) x = Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD];
+        else if (r == c) x = 1.0;
+        A[r * LDS + c] = x;
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < T64; c0 += kPB) {
+        const int nt = T64 - kPB - c0;
+        if (tid < 128) {
+            if (factor_block(A, piv, col, c0)) report_pivot(s, pd, err);
+        } else if (c0 > 0) {
+            scale_block(A, piv, rdiag, c0 - kPB, tid - 128, 128);
+        }
+        __syncthreads();
+        panel_rows(A, piv, rdiag, c0, nt);
+        __syncthreads();
+        for (int e = tid; e < nt * (nt + 1) / 2; e += 256) trail_entry(A, c0, e);
+        __syncthreads();
+    }
+    scale_block(A, piv, rdiag, T64 - kPB, tid, 256);
+    __syncthreads();
+#pragma unroll 4
+    for (int it = 0; it < 16; ++it) {
+        const int idx = tid + it * 256;
+        const int r = idx & 63, c = idx >> 6;
+        if (r < w && c <= r) Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD] = A[r * LDS + c];
+    }
+}
+
+constexpr size_t potrf_smem(size_t elem) {
+    return elem == 4 ? (2 * T64 * LDS + T64) * elem : (T64 * LDS + 2 * T64 + 2 * kPB) * elem;
+}
+
+constexpr size_t update_smem(size_t elem) {      // two 64x64 panel tiles, then potrf_tile
+    return 2 * T64 * T64 * elem > potrf_smem(elem) ? 2 * T64 * T64 * elem : potrf_smem(elem);
+}
 
 // Diagonal-tile Cholesky of the first step of each front of a level (later steps
 // are factored at the end of the previous step's update, see k_update).
@@ -417,17 +608,16 @@ __global__ void __launch_bounds__(256) k_potrf(StepArgs a, const int* __restrict
     extern __shared__ __align__(16) unsigned char smraw[];
     const int s = items[a.item_off + blockIdx.x];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
-    potrf_tile<T>(s, a.k, pd, F, Linv, inv_off, err, smraw);
+    potrf_tile(s, a.k, pd, F, Linv, inv_off, err, smraw);
 }
 
-// Panel rows below the diagonal tile: X = B L_kk^{-T} = B Linv^T (a small GEMM).
-template <class T>
+// Panel rows below the diagonal tile: X = B L_kk^{-float} = B Linv^float (a small GEMM).
 __global__ void __launch_bounds__(256) k_trsm(StepArgs a, const int* __restrict__ items,
-                                              const int* __restrict__ prefix, PlanDev pd, T* F,
-                                              const T* __restrict__ Linv, const int64_t* __restrict__ inv_off) {
+                                              const int* __restrict__ prefix, PlanDev pd, float* F,
+                                              const float* __restrict__ Linv, const int64_t* __restrict__ inv_off) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    T* Iv = reinterpret_cast<T*>(smraw);    // Linv column-major [q + c*64]
-    T* B = Iv + T64 * T64;                   // B[c][r] (column-major)
+    float* Iv = reinterpret_cast<float*>(smraw);    // Linv column-major [q + c*64]
+    float* B = Iv + T64 * T64;                   // B[c][r] (column-major)
     const int i = find_item(prefix + a.tp_off, a.nitems, blockIdx.x);
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
@@ -438,22 +628,22 @@ __global__ void __launch_bounds__(256) k_trsm(StepArgs a, const int* __restrict_
     const int w = min(T64, K - k0);
     const int r0 = k0 + w + lt * T64;
     const int nr = min(T64, N - r0);
-    T* Fs = F + pd.F_off[s];
-    const T* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;
+    float* Fs = F + pd.F_off[s];
+    const float* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;
     const int tid = threadIdx.x;
     for (int idx = tid; idx < T64 * T64; idx += blockDim.x) Iv[idx] = Li[idx];
     for (int idx = tid; idx < T64 * T64; idx += blockDim.x) {
         const int r = idx & 63, c = idx >> 6;
-        B[c * T64 + r] = (r < nr && c < w) ? Fs[(r0 + r) + static_cast<int64_t>(k0 + c) * LD] : T(0);
+        B[c * T64 + r] = (r < nr && c < w) ? Fs[(r0 + r) + static_cast<int64_t>(k0 + c) * LD] : 0.f;
     }
     __syncthreads();
     // X[r][c] = sum_{q <= c} B[r][q] Linv[c][q]; thread: row r, 16 columns
     const int r = tid & 63, cg = tid >> 6;
-    T acc[16];
+    float acc[16];
 #pragma unroll
-    for (int t = 0; t < 16; ++t) acc[t] = T(0);
+    for (int t = 0; t < 16; ++t) acc[t] = 0.f;
     for (int q = 0; q < w; ++q) {
-        const T bq = B[q * T64 + r];
+        const float bq = B[q * T64 + r];
 #pragma unroll
         for (int t = 0; t < 16; ++t) acc[t] += bq * Iv[(cg * 16 + t) + q * T64];   // Linv[c][q], 0 when q > c
     }
@@ -463,6 +653,104 @@ __global__ void __launch_bounds__(256) k_trsm(StepArgs a, const int* __restrict_
             const int c = cg * 16 + t;
             if (c < w) Fs[(r0 + r) + static_cast<int64_t>(k0 + c) * LD] = acc[t];
         }
+}
+
+// FP64 panel rows below the diagonal tile, X L_kk^T = B by substitution, and the tile's
+// inverse, which is the same for the rows of the identity (X = L_kk^{-T}). Bound by the
+// FP64 pipe (2080 multiply-adds a row, 2 a cycle and SM), so a block takes only 16 rows:
+// two per warp, lane (row, c) their columns 16 b + c. That fills the chip from 600 rows
+// on, where 64-row tiles that multiply by the inverse left most SMs idle (69 us a step at
+// any size up to 9700 rows; now 9 us up to 1200 rows, and the inverse is off the chain of
+// the diagonal tile). Each 16-column block first takes the columns before it, then runs
+// its own substitution with shuffles. The first 4 * tiles blocks are the 16-row parts of
+// the step's 64-row tiles, the other 4 * nitems the identity's rows of each front.
+constexpr int kTrRows = 16;
+constexpr int kTrLd = T64 + 2;              // 16-byte aligned rows, no bank conflicts
+constexpr size_t kTrSmem = (T64 * kTrLd + kTrRows * kTrLd + T64) * sizeof(double);
+
+__global__ void __launch_bounds__(256) k_trsm_rows(StepArgs a, const int* __restrict__ items,
+                                                   const int* __restrict__ prefix, PlanDev pd, double* F,
+                                                   double* __restrict__ Linv, const int64_t* __restrict__ inv_off,
+                                                   int tiles) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double* L = reinterpret_cast<double*>(smraw);   // unit lower factor, L[c * kTrLd + q]
+    double* X = L + T64 * kTrLd;                    // the block's rows, X[r * kTrLd + c]
+    double* rd = X + kTrRows * kTrLd;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int sub = blockIdx.x & 3, unit = blockIdx.x >> 2;
+    const bool ident = unit >= tiles;
+    const int i = ident ? unit - tiles : find_item(prefix + a.tp_off, a.nitems, unit);
+    const int s = items[a.item_off + i];
+    if (!pd.lp_on[pd.sn_lp[s]]) return;
+    const int N = pd.sn_nrows[s], LD = pd.sn_lda[s];
+    const int k0 = a.k * T64;
+    const int w = min(T64, pd.sn_ncols[s] - k0);
+    const int r0 = ident ? sub * kTrRows : k0 + w + (unit - prefix[a.tp_off + i]) * T64 + sub * kTrRows;
+    const int nr = ident ? kTrRows : min(kTrRows, N - r0);
+    if (nr <= 0) return;
+    double* Fs = F + pd.F_off[s];
+    if (tid < T64) rd[tid] = tid < w ? 1.0 / Fs[(k0 + tid) + static_cast<int64_t>(k0 + tid) * LD] : 1.0;
+    double l[16], x[4];
+#pragma unroll
+    for (int it = 0; it < 16; ++it) {
+        const int idx = tid + it * 256, c = idx & 63, q = idx >> 6;
+        l[it] = c < w && q < c ? Fs[(k0 + c) + static_cast<int64_t>(k0 + q) * LD] : 0.0;
+    }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = tid + it * 256, r = idx & 15, c = idx >> 4;
+        if (ident) x[it] = r0 + r == c ? 1.0 : 0.0;
+        else x[it] = r < nr && c < w ? Fs[(r0 + r) + static_cast<int64_t>(k0 + c) * LD] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < 16; ++it) {
+        const int idx = tid + it * 256, c = idx & 63, q = idx >> 6;
+        if (q < c) L[c * kTrLd + q] = l[it] * rd[q];
+    }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = tid + it * 256;
+        X[(idx & 15) * kTrLd + (idx >> 4)] = x[it];
+    }
+    __syncthreads();
+    const int c = lane & 15;
+    double* xr = X + (2 * wid + (lane >> 4)) * kTrLd;
+    const int b0 = ident ? sub : 0;            // rows of the identity are 0 before their own block
+    for (int b = b0; b < T64 / 16; ++b) {
+        const double* lc = L + (16 * b + c) * kTrLd;
+        double v = xr[16 * b + c];
+        for (int q = 16 * b0; q < 16 * b; q += 4) {
+            const double2 x0 = *reinterpret_cast<const double2*>(xr + q);
+            const double2 x1 = *reinterpret_cast<const double2*>(xr + q + 2);
+            const double2 l0 = *reinterpret_cast<const double2*>(lc + q);
+            const double2 l1 = *reinterpret_cast<const double2*>(lc + q + 2);
+            v = fma(-x0.x, l0.x, v);
+            v = fma(-x0.y, l0.y, v);
+            v = fma(-x1.x, l1.x, v);
+            v = fma(-x1.y, l1.y, v);
+        }
+#pragma unroll
+        for (int q = 0; q < 15; ++q) {
+            const double y = __shfl_sync(0xffffffffu, v, (lane & 16) + q);
+            if (c > q) v = fma(-y, lc[16 * b + q], v);
+        }
+        xr[16 * b + c] = v;
+        __syncwarp();
+    }
+    __syncthreads();
+    double* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = tid + it * 256;
+        if (ident) {                           // column j of the inverse is row j of X
+            const int q = idx & 63, j = r0 + (idx >> 6);
+            Li[q + j * T64] = q < w && j <= q ? X[(idx >> 6) * kTrLd + q] * rd[q] : 0.0;
+        } else {
+            const int r = idx & 15, q = idx >> 4;
+            if (r < nr && q < w) Fs[(r0 + r) + static_cast<int64_t>(k0 + q) * LD] = X[r * kTrLd + q] * rd[q];
+        }
+    }
 }
 
 // C(64x64) -= A_i (64 x w) A_j^T; 256 threads, 4x4 outputs each. The C tile is
@@ -544,8 +832,110 @@ __global__ void __launch_bounds__(256) k_update(StepArgs a, const int* __restric
     // (step k + 1's diagonal tile), overlapping the rest of this step's update.
     if (lt == 0 && t0 < K) {
         __syncthreads();
-        potrf_tile<T>(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
+        potrf_tile(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
     }
+}
+
+// FP64 update in TS x TS parts of the 64x64 tiles (TS = 32 or 16), for steps whose tiles
+// do not fill the chip: a 64x64 tile takes 65 us of one SM's FP64 pipe, a 32x32 part 16
+// us and a 16x16 part 4 us (plus their shared loads). The same sums in the same order.
+// The next diagonal tile is spread over several blocks then: the last of them to finish
+// (cnt, per front) factors it.
+template <int TS>
+__global__ void __launch_bounds__(256) k_update_split(StepArgs a, const int* __restrict__ items,
+                                                      const int* __restrict__ prefix, PlanDev pd, double* F,
+                                                      int* __restrict__ cnt, int* err) {
+    constexpr int P = T64 / TS, E = TS / 16;        // parts per tile side, entries per thread and side
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ int last;
+    double* As = reinterpret_cast<double*>(smraw);  // [kk][r]
+    double* Bs = As + T64 * TS;                      // [kk][c]
+    const int tile = blockIdx.x / (P * P), part = blockIdx.x % (P * P);
+    const int i = find_item(prefix + a.up_off, a.nitems, tile);
+    const int s = items[a.item_off + i];
+    if (!pd.lp_on[pd.sn_lp[s]]) return;
+    const int lt = tile - prefix[a.up_off + i];
+    int ti, tj;
+    tri_index(lt, ti, tj);
+    const int N = pd.sn_nrows[s], K = pd.sn_ncols[s];
+    const int LD = pd.sn_lda[s];
+    const int k0 = a.k * T64;
+    const int w = min(T64, K - k0);
+    const int t0 = k0 + w;
+    const int si = part / P, sj = part % P;
+    const int ri0 = t0 + ti * T64 + si * TS, cj0 = t0 + tj * T64 + sj * TS;
+    const bool diag = ri0 == cj0;
+    if (ri0 >= N || cj0 >= N || ri0 < cj0) return;
+    const int nri = min(TS, N - ri0), ncj = min(TS, N - cj0);
+    double* Fs = F + pd.F_off[s];
+    const int tid = threadIdx.x;
+    const int tx = tid & 15, ty = tid >> 4;          // rows E * tx .., columns E * ty ..
+    double cv[E][E];
+#pragma unroll
+    for (int p = 0; p < E; ++p)
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const int r = tx * E + q, c = ty * E + p;
+            const bool in = r < nri && c < ncj && (!diag || r >= c);
+            cv[q][p] = in ? Fs[(ri0 + r) + static_cast<int64_t>(cj0 + c) * LD] : 0.0;
+        }
+    double va[TS / 4], vb[TS / 4];
+#pragma unroll
+    for (int it = 0; it < TS / 4; ++it) {
+        const int idx = tid + it * 256;
+        const int r = idx & (TS - 1), kk = idx / TS;
+        const int64_t cofs = static_cast<int64_t>(k0 + kk) * LD;
+        va[it] = (kk < w && r < nri) ? Fs[ri0 + r + cofs] : 0.0;
+        vb[it] = (kk < w && r < ncj) ? Fs[cj0 + r + cofs] : 0.0;
+    }
+#pragma unroll
+    for (int it = 0; it < TS / 4; ++it) {
+        const int idx = tid + it * 256;
+        As[idx] = va[it];
+        Bs[idx] = vb[it];
+    }
+    __syncthreads();
+    double acc[E][E];
+#pragma unroll
+    for (int q = 0; q < E; ++q)
+#pragma unroll
+        for (int p = 0; p < E; ++p) acc[q][p] = 0.0;
+#pragma unroll 4
+    for (int kk = 0; kk < w; ++kk) {
+        double av[E], bv[E];
+#pragma unroll
+        for (int q = 0; q < E; ++q) { av[q] = As[kk * TS + tx * E + q]; bv[q] = Bs[kk * TS + ty * E + q]; }
+#pragma unroll
+        for (int q = 0; q < E; ++q)
+#pragma unroll
+            for (int p = 0; p < E; ++p) acc[q][p] += av[q] * bv[p];
+    }
+#pragma unroll
+    for (int p = 0; p < E; ++p)
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const int r = tx * E + q, c = ty * E + p;
+            if (r < nri && c < ncj && (!diag || r >= c))
+                Fs[(ri0 + r) + static_cast<int64_t>(cj0 + c) * LD] = cv[q][p] - acc[q][p];
+        }
+    if (lt == 0 && t0 < K) {
+        __threadfence();                             // this block's C writes, before the counter
+        __syncthreads();
+        if (tid == 0) {
+            const int nb = (min(T64, N - t0) + TS - 1) / TS, parts = nb * (nb + 1) / 2;
+            const int prev = atomicAdd(cnt + s, 1);
+            last = prev == parts - 1;
+            if (last) atomicExch(cnt + s, 0);
+            __threadfence();
+        }
+        __syncthreads();
+        if (last) potrf_tile(s, a.k + 1, pd, F, nullptr, nullptr, err, smraw);
+    }
+}
+template <int TS>
+constexpr size_t split_smem() {
+    return 2 * T64 * TS * sizeof(double) > potrf_smem(sizeof(double)) ? 2 * T64 * TS * sizeof(double)
+                                                                      : potrf_smem(sizeof(double));
 }
 
 // ---- shared helpers of the tensor-core kernels (tcgen05) --------------------
@@ -922,7 +1312,7 @@ __global__ void __launch_bounds__(256, 2) k_update_oz(StepArgs a, const int* __r
             }
         }
         __syncthreads();
-        if (*last) potrf_tile<double>(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
+        if (*last) potrf_tile(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
     }
 }
 
@@ -1221,7 +1611,7 @@ __global__ void __launch_bounds__(256, 2) k_update_tcs(StepArgs a, const int* __
     // the block holding the first trailing diagonal tile factors it (as in k_update)
     if (lb == 0 && t0 < K) {
         __syncthreads();
-        potrf_tile<float>(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
+        potrf_tile(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
     }
 }
 
@@ -1625,6 +2015,13 @@ inline int blocks_for(int64_t n, int t) { return static_cast<int>((n + t - 1) / 
 
 // ------------------------------------------------------------------ engine
 
+// Steps below these numbers of 64x64 update tiles take 16x16 / 32x32 parts: 16x16 while they
+// run in about two waves of the 152 SMs, 32x32 until whole tiles lose less to their last
+// wave than the parts do to their shared loads.
+constexpr int kSplit16Tiles = 24;
+constexpr int kSplit32Tiles = 1200;
+constexpr int kTrOzTiles = 152;
+
 struct KktEngine::Prof {
     cudaStream_t st;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> ev;
@@ -1649,13 +2046,17 @@ static void set_smem_attrs() {
                                      static_cast<int>(kTsSmem)));
     SK_CUDA(cudaFuncSetAttribute(k_potrf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(potrf_smem(sizeof(T)))));
-    SK_CUDA(cudaFuncSetAttribute(k_trsm<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(2 * T64 * T64 * sizeof(T))));
     SK_CUDA(cudaFuncSetAttribute(k_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(potrf_smem(sizeof(T)))));
+                                 static_cast<int>(update_smem(sizeof(T)))));
     if (std::is_same<T, double>::value)
         SK_CUDA(cudaFuncSetAttribute(k_update_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kOzSmemU)));
+    if (std::is_same<T, double>::value) {
+        SK_CUDA(cudaFuncSetAttribute(k_trsm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(kTrSmem)));
+        SK_CUDA(cudaFuncSetAttribute(k_update_split<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(split_smem<32>())));
+    }
     if (std::is_same<T, double>::value)
         SK_CUDA(cudaFuncSetAttribute(k_trsm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kOzSmemU)));
@@ -1856,7 +2257,7 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
         k_zero_fronts<T><<<static_cast<int>(nzc_), 256, 0, st_>>>(zc_sn_.ptr, zc_len_.ptr, zc_off_.ptr, pdv, F);
     SK_CUDA(cudaMemsetAsync(err_.ptr, 0, 4 * sizeof(int), st_));
     SK_CUDA(cudaMemsetAsync(lp_fail_.ptr, 0, lp_fail_.count * sizeof(int), st_));
-    if (emulate64_ && std::is_same<T, double>::value)   // blocks of the first update tile that have finished
+    if (std::is_same<T, double>::value)   // blocks of the first update tile that have finished
         SK_CUDA(cudaMemsetAsync(oz_cnt_.ptr, 0, oz_cnt_.count * sizeof(int), st_));
     const double* theta = theta_bound_;
     run(0, [&] {
@@ -1888,26 +2289,33 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                     k_potrf<T><<<st.nitems, 256, potrf_smem(sizeof(T)), st_>>>(a, items, pdv, F, Linv,
                                                                                inv_off_.ptr, err_.ptr);
                 });
-            if (st.trsm_tiles > 0)
-                run(2, [&] {
-                    bool oz = false;
-                    if constexpr (std::is_same<T, double>::value) {
-                        if (emulate64_) {   // FP64-accurate panel solve on the tensor cores
-                            oz = true;
-                            const int64_t plane = plan_.max_digit_rows * 128, lplane = max_step_items_ * T64 * 128;
-                            k_oz_digits<<<static_cast<int>(st.trsm_tiles), 256, 0, st_>>>(
-                                a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane);
-                            k_oz_linv_digits<<<st.nitems, 256, 0, st_>>>(a, items, pdv, Linv, inv_off_.ptr,
-                                                                         ldig_.ptr, lexp_.ptr, lplane);
-                            k_trsm_oz<<<static_cast<int>(st.digit_rows / 128) * 2, 256, kOzSmemU, st_>>>(
-                                a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane, ldig_.ptr,
-                                lexp_.ptr, lplane, err_.ptr);
-                        }
-                    }
-                    if (!oz)
-                        k_trsm<T><<<static_cast<int>(st.trsm_tiles), 256, 2 * T64 * T64 * sizeof(T), st_>>>(
+            if constexpr (std::is_same<T, float>::value) {
+                if (st.trsm_tiles > 0)
+                    run(2, [&] {
+                        k_trsm<<<static_cast<int>(st.trsm_tiles), 256, 2 * T64 * T64 * sizeof(T), st_>>>(
                             a, items, prefix, pdv, F, Linv, inv_off_.ptr);
+                    });
+            } else {
+                run(2, [&] {
+                    // the panel solve on the tensor cores costs 80 us and more of digit passes and
+                    // launches but its work is small; from kTrOzTiles 64-row tiles on, the FP64
+                    // pipe (3.4 us per 152 x 64 rows) takes longer
+                    const bool oz = emulate64_ && st.trsm_tiles >= kTrOzTiles;
+                    const int tiles = oz ? 0 : static_cast<int>(st.trsm_tiles);
+                    k_trsm_rows<<<4 * (tiles + st.nitems), 256, kTrSmem, st_>>>(a, items, prefix, pdv, F, Linv,
+                                                                                inv_off_.ptr, tiles);
+                    if (oz) {
+                        const int64_t plane = plan_.max_digit_rows * 128, lplane = max_step_items_ * T64 * 128;
+                        k_oz_digits<<<static_cast<int>(st.trsm_tiles), 256, 0, st_>>>(
+                            a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane);
+                        k_oz_linv_digits<<<st.nitems, 256, 0, st_>>>(a, items, pdv, Linv, inv_off_.ptr, ldig_.ptr,
+                                                                     lexp_.ptr, lplane);
+                        k_trsm_oz<<<static_cast<int>(st.digit_rows / 128) * 2, 256, kOzSmemU, st_>>>(
+                            a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane, ldig_.ptr, lexp_.ptr, lplane,
+                            err_.ptr);
+                    }
                 });
+            }
             if (st.upd_tiles > 0) {
                 run(3, [&] {
                     bool tc = false;
@@ -1932,8 +2340,20 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                                 dexp_.ptr, plane, oz_cnt_.ptr, err_.ptr);
                         }
                     }
+                    if constexpr (std::is_same<T, double>::value) {
+                        const int tiles = static_cast<int>(st.upd_tiles);
+                        if (!tc && tiles < kSplit16Tiles) {
+                            tc = true;
+                            k_update_split<16><<<tiles * 16, 256, split_smem<16>(), st_>>>(a, items, prefix, pdv, F,
+                                                                                           oz_cnt_.ptr, err_.ptr);
+                        } else if (!tc && tiles < kSplit32Tiles) {
+                            tc = true;
+                            k_update_split<32><<<tiles * 4, 256, split_smem<32>(), st_>>>(a, items, prefix, pdv, F,
+                                                                                          oz_cnt_.ptr, err_.ptr);
+                        }
+                    }
                     if (!tc)
-                        k_update<T><<<static_cast<int>(st.upd_tiles), 256, potrf_smem(sizeof(T)), st_>>>(
+                        k_update<T><<<static_cast<int>(st.upd_tiles), 256, update_smem(sizeof(T)), st_>>>(
                             a, items, prefix, pdv, F, Linv, inv_off_.ptr, err_.ptr);
                 });
                 if (prof) {
