@@ -1644,11 +1644,28 @@ __global__ void k_extend_add(int item_off, int nitems, int prefix_off, const int
 // -------------------------------------------------------------------- solve
 // Vectors of the solve are in the front precision T; the caller's vectors are FP64.
 
+// A solution entry that is not there yet: an all-ones NaN, which no arithmetic result is
+// (publish() stores the canonical NaN instead).
+template <class T> struct Pending;
+template <> struct Pending<float> {
+    __device__ static float value() { return __uint_as_float(0xffffffffu); }
+    __device__ static bool is(float v) { return __float_as_uint(v) == 0xffffffffu; }
+};
+template <> struct Pending<double> {
+    __device__ static double value() { return __longlong_as_double(-1LL); }
+    __device__ static bool is(double v) { return __double_as_longlong(v) == -1LL; }
+};
+
+// zp = D src in elimination order; both solution vectors pending.
 template <class T>
 __global__ void k_permute_scale(int M, const int* __restrict__ perm, const double* __restrict__ D,
-                                const double* __restrict__ src, T* __restrict__ zp) {
+                                const double* __restrict__ src, T* __restrict__ zp, T* __restrict__ zsol,
+                                T* __restrict__ xp) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < M) zp[q] = static_cast<T>(D[q] * src[perm[q]]);
+    if (q >= M) return;
+    zp[q] = static_cast<T>(D[q] * src[perm[q]]);
+    zsol[q] = Pending<T>::value();
+    xp[q] = Pending<T>::value();
 }
 
 // Rows of the LPs in `own` receive D xp; rows of the LPs in `other` (the set the
@@ -1700,58 +1717,115 @@ __global__ void k_fwd_gather(int n, const int* __restrict__ dst, const int* __re
 // ---- dependency-driven triangular solves -------------------------------------
 // Each front's rows are split into 64-row blocks; block i of front s is one task.
 // Tasks of a level are handed out in dependency order by an atomic counter, so a
-// task only ever waits for tasks that have already started; results are
-// published through per-block flags. Every wait is bounded: on time-out the task
-// sets *err and returns (the host checks *err and reports an error).
+// task only ever waits for tasks that have already started. The chain from block to
+// block bounds these kernels, so a block's solution is its own signal: the entries are
+// pending (k_permute_scale) until their value is stored, and a waiting task polls the
+// values themselves. One trip through the L2 then links two blocks, where a flag took
+// four (values, fence, flag; flag, then values). Every wait is bounded: on time-out the
+// task sets *err and returns (the host checks *err and reports an error).
+// Chain of one front, per 64-row block: FP32 forward 2.2 -> 1.4 us, backward 3.2 -> 1.1
+// us; FP64 forward 4.4 -> 2.8 us, backward 8.2 -> 3.2 us (m = 1447 .. 4740).
 
 constexpr int kSpinLimit = 1 << 24;
+constexpr int kReadyBlocks = 16;   // column blocks taken per pass once they are there
 
-__device__ __forceinline__ bool wait_flag(const int* flag, int target, int* err, int* abort_sh) {
-    int spins = 0;
-    while (*reinterpret_cast<const volatile int*>(flag) < target) {
-        if (*reinterpret_cast<const volatile int*>(err) != 0 || ++spins > kSpinLimit) {
-            atomicExch(err, 1);
-            *abort_sh = 1;
-            return false;
-        }
-        // poll back to back first (the flag of the last dependency usually comes within
-        // microseconds: this wait is on the solve's critical path), then back off
-        if (spins > 512) __nanosleep(64);
-    }
-    __threadfence();
-    return true;
+__device__ __forceinline__ float peek(const float* p) {
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double peek(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void publish(float* p, float v) {
+    if (Pending<float>::is(v)) v = __uint_as_float(0x7fffffffu);
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" :: "l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void publish(double* p, double v) {
+    if (Pending<double>::is(v)) v = __longlong_as_double(0x7ff8000000000000LL);
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" :: "l"(p), "d"(v) : "memory");
 }
 
+// *p once it is there; false on time-out or when another task gave up.
 template <class T>
-__device__ __forceinline__ T ld_cg(const T* p) { return __ldcg(p); }
+__device__ __forceinline__ bool await(const T* p, T& v, int* err) {
+    for (int spins = 0;; ++spins) {
+        v = peek(p);
+        if (!Pending<T>::is(v)) return true;
+        if (spins > kSpinLimit || ((spins & 255) == 255 && *reinterpret_cast<volatile int*>(err) != 0)) {
+            atomicExch(err, 1);
+            return false;
+        }
+        // back to back first (the last dependency usually comes within microseconds: this wait is
+        // on the solve's critical path), then back off
+        if (spins > 512) __nanosleep(64);
+    }
+}
 
-constexpr int kReadyBlocks = 16;   // column blocks taken per pass once their flags are set
+struct TakeSync {
+    unsigned char ready[8];   // per warp: its four 32-entry parts that are there
+    int abort;
+};
 
-__device__ __forceinline__ int flag_now(const int* flag) { return *reinterpret_cast<const volatile int*>(flag); }
+// Solution blocks j, j + dir, ... (n of them at most; rows 64 b .. of the front's own K)
+// into out, 64 entries each: those that are there already, at least block j, which is
+// waited for. Returns how many (0: given up). Called by all 256 threads.
+template <class T>
+__device__ __forceinline__ int take_blocks(const T* sol, int j, int dir, int n, int K, T* out, TakeSync* sh,
+                                           int* err) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    n = min(n, kReadyBlocks);
+    unsigned mine = 0;
+#pragma unroll
+    for (int u = 0; u < kReadyBlocks / 4; ++u) {
+        const int b = 4 * u + (tid >> 6);            // the same for a warp
+        if (b >= n) break;
+        const int row = (j + dir * b) * T64 + (tid & 63);
+        const T v = row < K ? peek(sol + row) : T(0);
+        out[b * T64 + (tid & 63)] = v;
+        if (__all_sync(0xffffffffu, !Pending<T>::is(v))) mine |= 1u << u;
+    }
+    if (lane == 0) sh->ready[wid] = static_cast<unsigned char>(mine);
+    if (tid == 0) sh->abort = 0;
+    __syncthreads();
+    int got = 0;
+    while (got < n && (sh->ready[(2 * got) & 7] & sh->ready[(2 * got + 1) & 7] & (1u << (got >> 2)))) ++got;
+    if (got > 0) return got;
+    if (tid < T64) {
+        const int row = j * T64 + tid;
+        T v = T(0);
+        if (row < K && !await(sol + row, v, err)) sh->abort = 1;
+        out[tid] = v;
+    }
+    __syncthreads();
+    return sh->abort ? 0 : 1;
+}
+
+// Rows of a 64x64 triangular product dealt to a thread quad: warp w takes the eight rows
+// of group w or 11 - w, so that the two warps of each SM quarter share the work of a
+// triangle evenly.
+__device__ __forceinline__ int tri_group(int wid) { return wid < 4 ? wid : 11 - wid; }
 
 // Forward: task (s, i). Own block i < nb covers rows [64 i, min(64 i + 64, K));
 // external block i >= nb covers rows [K + 64 (i - nb), ...) < N. The task forms
-// f_rows - sum_{j < min(i, nb)} L(rows, block j) z_j; an own block then stores
-// z_i = Linv_i (..) in zsol and flags 1, an external block stores the parent's
-// update vector in f. Column blocks whose flags are already set are taken
-// together (up to kReadyBlocks per pass); the first block of each pass has its L
-// values loaded before the wait, so the latency-critical last dependency only
-// waits for its flag and z values.
+// f_rows - sum_{j < min(i, nb)} L(rows, block j) z_j; an own block then publishes
+// z_i = Linv_i (..) in zsol, an external block stores the parent's update vector in f.
+// Column blocks that are there already are taken together (up to kReadyBlocks per
+// pass); the first block of each pass has its L values loaded before the wait, so the
+// latency-critical last dependency only waits for its z values.
 template <class T>
 __global__ void __launch_bounds__(256, 1) k_fwd_tasks(const int2* __restrict__ tasks, int ntasks, int* counter,
                                                    PlanDev pd, const T* __restrict__ F, const T* __restrict__ Linv,
-                                                   const int64_t* __restrict__ inv_off,
-                                                   const int* __restrict__ blk_off, int* flags, T* fv, T* zsol,
-                                                   int* err) {
-    __shared__ int task_sh, abort_sh, ready_sh;
+                                                   const int64_t* __restrict__ inv_off, T* fv, T* zsol, int* err) {
+    __shared__ int task_sh;
+    __shared__ TakeSync take;
     __shared__ T zs[kReadyBlocks * T64];
     __shared__ T red[4][T64];
     __shared__ T fb[T64];
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        task_sh = atomicAdd(counter, 1);
-        abort_sh = 0;
-    }
+    if (tid == 0) task_sh = atomicAdd(counter, 1);
     __syncthreads();
     const int t = task_sh;
     if (t >= ntasks) return;
@@ -1762,7 +1836,6 @@ __global__ void __launch_bounds__(256, 1) k_fwd_tasks(const int2* __restrict__ t
     const int nb = (K + T64 - 1) / T64;
     const T* Fs = F + pd.F_off[s];
     T* f = fv + pd.f_off[s];
-    int* fl = flags + blk_off[s];
     const int r = tid & 63, cg = tid >> 6;
     const bool own = i < nb;
     const int row0 = own ? i * T64 : K + (i - nb) * T64;
@@ -1771,7 +1844,7 @@ __global__ void __launch_bounds__(256, 1) k_fwd_tasks(const int2* __restrict__ t
     const bool rv = row < rend;
     // this thread's entries of the diagonal-tile inverse (own blocks), loaded up front
     const int w = own ? min(T64, K - i * T64) : 0;
-    const int zc = tid >> 2, zpart = tid & 3;
+    const int grp = tri_group(tid >> 5), zc = 8 * grp + ((tid & 31) >> 2), zpart = tid & 3;
     T li[16];
     if (own) {
         const T* Li = Linv + inv_off[s] + static_cast<int64_t>(i) * T64 * T64;
@@ -1791,22 +1864,9 @@ __global__ void __launch_bounds__(256, 1) k_fwd_tasks(const int2* __restrict__ t
 #pragma unroll
         for (int c = 0; c < 16; ++c)
             pre[c] = (rv && colp + c < K) ? Fs[row + static_cast<int64_t>(colp + c) * LD] : T(0);
-        if (tid == 0) {
-            if (wait_flag(fl + j, 1, err, &abort_sh)) {
-                int e = j + 1;
-                while (e < jmax && e < j + kReadyBlocks && flag_now(fl + e) >= 1) ++e;
-                __threadfence();
-                ready_sh = e;
-            }
-        }
-        __syncthreads();
-        if (abort_sh) return;
-        const int e = ready_sh;
-        for (int q = tid; q < (e - j) * T64; q += 256) {
-            const int col = j * T64 + q;
-            zs[q] = col < K ? ld_cg(zsol + first + col) : T(0);
-        }
-        __syncthreads();
+        const int got = take_blocks(zsol + first, j, 1, jmax - j, K, zs, &take, err);
+        if (got == 0) return;
+        const int e = j + got;
 #pragma unroll
         for (int c = 0; c < 16; ++c) acc += pre[c] * zs[cg * 16 + c];
         if (rv) {
@@ -1818,8 +1878,8 @@ __global__ void __launch_bounds__(256, 1) k_fwd_tasks(const int2* __restrict__ t
                     if (jj * T64 + cg * 16 + c < K) acc += Lc[static_cast<int64_t>(c) * LD] * zz[c];
             }
         }
-        __syncthreads();
         j = e;
+        if (j < jmax) __syncthreads();    // zs is refilled
     }
     red[cg][r] = acc;
     __syncthreads();
@@ -1833,38 +1893,38 @@ __global__ void __launch_bounds__(256, 1) k_fwd_tasks(const int2* __restrict__ t
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             const int q = zpart + 4 * k;
+            if (k > 2 * grp + 1) break;       // beyond the diagonal for the whole warp
             if (q <= zc) z += li[k] * fb[q];
         }
         z += __shfl_xor_sync(0xffffffffu, z, 1);
         z += __shfl_xor_sync(0xffffffffu, z, 2);
-        if (zpart == 0 && zc < w) zsol[first + i * T64 + zc] = z;
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) atomicExch(fl + i, 1);
+        if (zpart == 0 && zc < w) publish(zsol + first + i * T64 + zc, z);
     } else {
         if (tid < T64 && row0 + tid < N) f[row0 + tid] = fb[tid];
     }
 }
 
 // Backward: task (s, i), i descending: x_i = Linv_i^T (z_i - sum_{rows r below
-// block i} L(r, block i)^T x_r); rows of own later blocks wait for their flag (2),
-// rows outside the front's columns come from ancestors (earlier levels). Later
-// blocks are taken oldest first (nb - 1 downwards), ready ones together, and the
-// L values of the first block of each pass are loaded before its wait.
+// block i} L(r, block i)^T x_r); rows of own later blocks are waited for, rows outside
+// the front's columns come from ancestors (earlier levels). Later blocks are taken
+// oldest first (nb - 1 downwards), those that are there together, and the L values of
+// the first block of each pass are loaded before its wait. Each lane sums its rows for
+// eight columns; the lanes' sums are added by shuffles in FP32 and through shared memory
+// in FP64, where the shuffles' forty additions per warp on the FP64 pipe (64 cycles
+// each) were a third of the chain.
 template <class T>
 __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ tasks, int ntasks, int* counter,
                                                    PlanDev pd, const T* __restrict__ F, const T* __restrict__ Linv,
-                                                   const int64_t* __restrict__ inv_off,
-                                                   const int* __restrict__ blk_off, int* flags, T* xp,
+                                                   const int64_t* __restrict__ inv_off, T* xp,
                                                    const T* __restrict__ zsol, int* err) {
-    __shared__ int task_sh, abort_sh, ready_sh;
+    constexpr bool kWide = std::is_same<T, double>::value;
+    __shared__ int task_sh;
+    __shared__ TakeSync take;
     __shared__ T xb[kReadyBlocks * T64];   // x of ready own blocks, or of a chunk of outside rows
     __shared__ T tb[T64];
+    __shared__ T lanes[kWide ? T64 * 33 : 1];
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        task_sh = atomicAdd(counter, 1);
-        abort_sh = 0;
-    }
+    if (tid == 0) task_sh = atomicAdd(counter, 1);
     __syncthreads();
     const int t = task_sh;
     if (t >= ntasks) return;
@@ -1876,7 +1936,6 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
     const int w = min(T64, K - i * T64);
     const T* Fs = F + pd.F_off[s];
     const int* R = pd.rows + pd.rows_off[s];
-    int* fl = flags + blk_off[s];
     const int lane = tid & 31, wid = tid >> 5;
     T part[8];
 #pragma unroll
@@ -1914,8 +1973,8 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
         }
         __syncthreads();
     }
-    // this thread's entries of the diagonal-tile inverse
-    const int xc = tid >> 2, xpq = tid & 3;
+    // this thread's entries of the diagonal-tile inverse and of z
+    const int grp = tri_group(wid), xc = 8 * grp + (lane >> 2), xpq = lane & 3;
     T li[16];
     {
         const T* Li = Linv + inv_off[s] + static_cast<int64_t>(i) * T64 * T64;
@@ -1925,6 +1984,8 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
             li[k] = (xc < w && q < w) ? Li[q + xc * T64] : T(0);
         }
     }
+    const int zq = kWide ? tid >> 2 : wid * 8 + (lane & 7);      // the column of tb this thread may form
+    const T zown = zq < w ? zsol[first + i * T64 + zq] : T(0);
     // rows of own later blocks
     for (int j = nb - 1; j > i;) {
         T pre[16];
@@ -1935,22 +1996,9 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
             for (int q = 0; q < 8; ++q)
                 pre[h * 8 + q] = (rr < K && c0 + q < K) ? Fs[rr + static_cast<int64_t>(c0 + q) * LD] : T(0);
         }
-        if (tid == 0) {
-            if (wait_flag(fl + j, 2, err, &abort_sh)) {
-                int e = j - 1;
-                while (e > i && e > j - kReadyBlocks && flag_now(fl + e) >= 2) --e;
-                __threadfence();
-                ready_sh = e;
-            }
-        }
-        __syncthreads();
-        if (abort_sh) return;
-        const int e = ready_sh;   // blocks j, j - 1, ..., e + 1 are ready
-        for (int q = tid; q < (j - e) * T64; q += 256) {
-            const int blk = j - q / T64, rr = blk * T64 + q % T64;
-            xb[q] = rr < K ? ld_cg(xp + first + rr) : T(0);
-        }
-        __syncthreads();
+        const int got = take_blocks(static_cast<const T*>(xp + first), j, -1, j - i, K, xb, &take, err);
+        if (got == 0) return;
+        const int e = j - got;   // blocks j, j - 1, ..., e + 1 are there
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const T xr = xb[lane + 32 * h];
@@ -1968,16 +2016,24 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
                     if (c0 + q < K) part[q] += Fs[r + static_cast<int64_t>(c0 + q) * LD] * xr;
             }
         }
-        __syncthreads();
         j = e;
+        if (j > i) __syncthreads();       // xb is refilled
     }
+    if constexpr (kWide) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        T v = part[q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) {
-            const int c = wid * 8 + q;
-            tb[c] = c < w ? zsol[first + i * T64 + c] - v : T(0);
+        for (int q = 0; q < 8; ++q) lanes[(wid * 8 + q) * 33 + lane] = part[q];
+        __syncthreads();
+        const T* v8 = lanes + (tid >> 2) * 33 + 8 * (tid & 3);
+        T v = ((v8[0] + v8[1]) + (v8[2] + v8[3])) + ((v8[4] + v8[5]) + (v8[6] + v8[7]));
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if ((tid & 3) == 0) tb[zq] = zq < w ? zown - v : T(0);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            T v = part[q];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == q) tb[zq] = zq < w ? zown - v : T(0);
         }
     }
     __syncthreads();
@@ -1986,15 +2042,13 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             const int q = xc + xpq + 4 * k;
+            if (k > 15 - 2 * grp) break;      // past the tile for the whole warp
             if (q < w) x += li[k] * tb[q];
         }
         x += __shfl_xor_sync(0xffffffffu, x, 1);
         x += __shfl_xor_sync(0xffffffffu, x, 2);
-        if (xpq == 0 && xc < w) xp[first + i * T64 + xc] = x;
+        if (xpq == 0 && xc < w) publish(xp + first + i * T64 + xc, x);
     }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) atomicExch(fl + i, 2);
 }
 
 // ------------------------------------------------------- normal-matrix apply
@@ -2073,13 +2127,7 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
         inv_size_ += static_cast<int64_t>((p.sn_ncols[s] + T64 - 1) / T64) * T64 * T64;
     }
     // solve task lists per level (forward: row blocks ascending; backward: own
-    // column blocks descending) and per-front flag offsets
-    std::vector<int> blk_off(static_cast<size_t>(p.ns), 0);
-    nflags_ = 0;
-    for (int s = 0; s < p.ns; ++s) {
-        blk_off[s] = nflags_;
-        nflags_ += (p.sn_ncols[s] + T64 - 1) / T64;
-    }
+    // column blocks descending)
     // Within a level the tasks are ordered by their position in their front's chain
     // (forward: block index; backward: distance from the last own block), fronts
     // interleaved: blocks take tasks in list order, so the first tasks of every
@@ -2169,12 +2217,11 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
     rsv(ea_off_, p.ea_off); rsv(step_items_, p.step_items); rsv(step_prefix_, p.step_prefix);
     rsv(round_items_, p.round_items); rsv(round_prefix_, p.round_prefix); rsv(level_sn_, p.level_sn);
     rsv(slot_pos_, p.slot_pos); rsv(w_ptr_, p.w_ptr); rsv(slot_i_, p.slot_i); rsv(slot_j_, p.slot_j);
-    rsv(w_col_, p.w_col); rsv(w_val_, p.w_val); rsv(inv_off_, inv_off); rsv(blk_off_, blk_off);
+    rsv(w_col_, p.w_col); rsv(w_val_, p.w_val); rsv(inv_off_, inv_off);
     rsv(fwd_tasks_, ftask); rsv(bwd_tasks_, btask);
     rsv(g_dst_, g_dst); rsv(g_zp_, g_zp); rsv(g_ptr_, g_ptr); rsv(g_src_, g_src);
     rsv(sn_lp_, sn_lp); rsv(on32_, on32_h_); rsv(on64_, on64_h_); rsv(q_lp_, q_lp);
     rsv(zc_sn_, zc_sn); rsv(zc_len_, zc_len); rsv(zc_off_, zc_off);
-    reserve(arena_, flags_, static_cast<size_t>(std::max(1, nflags_)));
     reserve(arena_, counters_, static_cast<size_t>(2 * std::max(1, p.nlevels)));
     reserve(arena_, solve_err_, 1);
     reserve(arena_, D_, static_cast<size_t>(p.M));
@@ -2197,8 +2244,8 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
     bnd(sn_first_); bnd(sn_ncols_); bnd(sn_nrows_); bnd(sn_lda_); bnd(sn_parent_); bnd(rows_); bnd(ea_map_); bnd(ch_ptr_);
     bnd(ch_list_); bnd(perm_); bnd(sn_F_off_); bnd(sn_f_off_); bnd(sn_rows_off_); bnd(ea_off_); bnd(step_items_);
     bnd(step_prefix_); bnd(round_items_); bnd(round_prefix_); bnd(level_sn_); bnd(slot_pos_); bnd(w_ptr_);
-    bnd(slot_i_); bnd(slot_j_); bnd(w_col_); bnd(w_val_); bnd(inv_off_); bnd(blk_off_); bnd(fwd_tasks_);
-    bnd(bwd_tasks_); bnd(g_dst_); bnd(g_zp_); bnd(g_ptr_); bnd(g_src_); bnd(sn_lp_); bnd(on32_); bnd(on64_); bnd(q_lp_); bnd(zc_sn_); bnd(zc_len_); bnd(zc_off_); bnd(flags_); bnd(counters_); bnd(solve_err_); bnd(D_); bnd(Mdiag_);
+    bnd(slot_i_); bnd(slot_j_); bnd(w_col_); bnd(w_val_); bnd(inv_off_); bnd(fwd_tasks_);
+    bnd(bwd_tasks_); bnd(g_dst_); bnd(g_zp_); bnd(g_ptr_); bnd(g_src_); bnd(sn_lp_); bnd(on32_); bnd(on64_); bnd(q_lp_); bnd(zc_sn_); bnd(zc_len_); bnd(zc_off_); bnd(counters_); bnd(solve_err_); bnd(D_); bnd(Mdiag_);
     bnd(zp_); bnd(xp_); bnd(zsol_); bnd(fvec_); bnd(tn_); bnd(params_); bnd(err_); bnd(lp_fail_); bnd(oz_cnt_);
     for (auto& sb : sub_) { bnd(sb.d_items); bnd(sb.d_prefix); }
     upload(sn_first_, p.sn_first, st_); upload(sn_ncols_, p.sn_ncols, st_); upload(sn_nrows_, p.sn_nrows, st_);
@@ -2210,7 +2257,7 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
     upload(round_items_, p.round_items, st_); upload(round_prefix_, p.round_prefix, st_);
     upload(level_sn_, p.level_sn, st_); upload(slot_pos_, p.slot_pos, st_); upload(w_ptr_, p.w_ptr, st_);
     upload(slot_i_, p.slot_i, st_); upload(slot_j_, p.slot_j, st_); upload(w_col_, p.w_col, st_);
-    upload(w_val_, p.w_val, st_); upload(inv_off_, inv_off, st_); upload(blk_off_, blk_off, st_);
+    upload(w_val_, p.w_val, st_); upload(inv_off_, inv_off, st_);
     upload(fwd_tasks_, ftask, st_); upload(bwd_tasks_, btask, st_);
     upload(g_dst_, g_dst, st_); upload(g_zp_, g_zp, st_); upload(g_ptr_, g_ptr, st_); upload(g_src_, g_src, st_);
     upload(sn_lp_, sn_lp, st_); upload(on32_, on32_h_, st_); upload(on64_, on64_h_, st_); upload(q_lp_, q_lp, st_);
@@ -2394,7 +2441,6 @@ void KktEngine::launch_solve(const T* F, const T* Linv, Prof* prof) {
     T* xp = reinterpret_cast<T*>(xp_.ptr);
     T* zs = reinterpret_cast<T*>(zsol_.ptr);
     T* fv = reinterpret_cast<T*>(fvec_.ptr);
-    SK_CUDA(cudaMemsetAsync(flags_.ptr, 0, sizeof(int) * static_cast<size_t>(std::max(1, nflags_)), st_));
     SK_CUDA(cudaMemsetAsync(counters_.ptr, 0, sizeof(int) * 2 * static_cast<size_t>(std::max(1, p.nlevels)), st_));
     for (int l = 0; l < p.nlevels; ++l) {
         const int nt = fwd_task_off_[l + 1] - fwd_task_off_[l];
@@ -2404,7 +2450,7 @@ void KktEngine::launch_solve(const T* F, const T* Linv, Prof* prof) {
                 k_fwd_gather<T><<<blocks_for(ng, 256), 256, 0, st_>>>(ng, g_dst_.ptr + g0, g_zp_.ptr + g0,
                                                                       g_ptr_.ptr + g0, g_src_.ptr, zp, fv);
             k_fwd_tasks<T><<<nt, 256, 0, st_>>>(fwd_tasks_.ptr + fwd_task_off_[l], nt, counters_.ptr + l, pdv, F,
-                                                Linv, inv_off_.ptr, blk_off_.ptr, flags_.ptr, fv, zs,
+                                                Linv, inv_off_.ptr, fv, zs,
                                                 solve_err_.ptr);
         });
     }
@@ -2412,7 +2458,7 @@ void KktEngine::launch_solve(const T* F, const T* Linv, Prof* prof) {
         const int nt = bwd_task_off_[l + 1] - bwd_task_off_[l];
         run(6, [&] {
             k_bwd_tasks<T><<<nt, 256, 0, st_>>>(bwd_tasks_.ptr + bwd_task_off_[l], nt, counters_.ptr + p.nlevels + l,
-                                                pdv, F, Linv, inv_off_.ptr, blk_off_.ptr, flags_.ptr, xp, zs,
+                                                pdv, F, Linv, inv_off_.ptr, xp, zs,
                                                 solve_err_.ptr);
         });
     }
@@ -2543,8 +2589,9 @@ template <class T>
 void KktEngine::solve_pass(const T* F, const T* Linv, const int* mask, bool keep, const double* d_src,
                            double* d_dst, int graph) {
     const auto& p = plan_;
-    k_permute_scale<T><<<blocks_for(p.M, 256), 256, 0, st_>>>(p.M, perm_.ptr, D_.ptr, d_src,
-                                                              reinterpret_cast<T*>(zp_.ptr));
+    k_permute_scale<T><<<blocks_for(p.M, 256), 256, 0, st_>>>(
+        p.M, perm_.ptr, D_.ptr, d_src, reinterpret_cast<T*>(zp_.ptr), reinterpret_cast<T*>(zsol_.ptr),
+        reinterpret_cast<T*>(xp_.ptr));
     if (!gsol_[graph]) {
         cudaGraph_t g;
         SK_CUDA(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
@@ -2656,14 +2703,16 @@ void KktEngine::profile(const double* d_theta, double delta, bool fp32, const do
     if (fp32) launch_factor<float>(F32_.ptr, Linv32_.ptr, &pr);
     else launch_factor<double>(F64_.ptr, Linv64_.ptr, &pr);
     if (fp32) {
-        k_permute_scale<float><<<blocks_for(plan_.M, 256), 256, 0, st_>>>(plan_.M, perm_.ptr, D_.ptr, d_rhs,
-                                                                          reinterpret_cast<float*>(zp_.ptr));
+        k_permute_scale<float><<<blocks_for(plan_.M, 256), 256, 0, st_>>>(
+            plan_.M, perm_.ptr, D_.ptr, d_rhs, reinterpret_cast<float*>(zp_.ptr), reinterpret_cast<float*>(zsol_.ptr),
+            reinterpret_cast<float*>(xp_.ptr));
         launch_solve<float>(F32_.ptr, Linv32_.ptr, &pr);
         k_unpermute_scale<float><<<blocks_for(plan_.M, 256), 256, 0, st_>>>(
             plan_.M, perm_.ptr, D_.ptr, reinterpret_cast<const float*>(xp_.ptr), lp_.row_lp, on32_.ptr, nullptr,
             d_out);
     } else {
-        k_permute_scale<double><<<blocks_for(plan_.M, 256), 256, 0, st_>>>(plan_.M, perm_.ptr, D_.ptr, d_rhs, zp_.ptr);
+        k_permute_scale<double><<<blocks_for(plan_.M, 256), 256, 0, st_>>>(plan_.M, perm_.ptr, D_.ptr, d_rhs, zp_.ptr,
+                                                                           zsol_.ptr, xp_.ptr);
         launch_solve<double>(F64_.ptr, Linv64_.ptr, &pr);
         k_unpermute_scale<double><<<blocks_for(plan_.M, 256), 256, 0, st_>>>(plan_.M, perm_.ptr, D_.ptr, xp_.ptr,
                                                                              lp_.row_lp, on64_.ptr, nullptr, d_out);
