@@ -264,12 +264,31 @@ __global__ void k_asm_cols_dense(int M, const int* __restrict__ rp, const int* _
 
 // ------------------------------------------------------------------- factor
 
-// Cholesky of the 64x64 diagonal tile of step k of one front, in the front's
-// precision. A partial tile is padded with the identity. This runs in one block on the
-// critical path of every 64-column step, by blocks of 16 columns: the 16x16 diagonal
-// block, the rows below it, the trailing update.
+// Cholesky of the 64x64 diagonal tile of step k of one front, in the front's precision T,
+// plus the explicit inverse of the factored tile (used by the panel solve and by both
+// triangular solves), stored column-major in Linv. A partial tile is padded with the
+// identity. This runs in one block on the critical path of every 64-column step, by blocks
+// of 16 columns: the 16x16 diagonal block, the rows below it, the trailing update. Every
+// entry keeps its own ascending sequence of fused multiply-adds and correctly rounded roots
+// and reciprocals, so the result does not depend on how the work is dealt out:
+//  * FP32 is bound by the latency of the pivot chain, FP64 also by the SM's FP64 pipe: a
+//    warp's FP64 instruction takes 64 cycles of its SM quarter whatever its active lanes, a
+//    dependent one follows at once, and shuffles and shared loads queue with it (measured:
+//    sqrt 600 cycles, a division 355, a 64-bit shuffle 16).
+//  * So warp 0 alone factors the diagonal block, from registers (shuffles, no barrier),
+//    while the warps of the other three quarters (helpers) apply the previous block's
+//    update to the rows below and form the inverse's block rows that are already known.
+//    Warp 0 joins them when its block is done; warp 4 shares its quarter and stays out.
+//  * The root and the reciprocal of an FP64 pivot take five dependent FP64 instructions
+//    instead of a sqrt and a division.
+// One tile: FP64 116 -> 58 us, FP32 38 -> 17 us.
 constexpr int kPB = 16;
 constexpr int kPBTri = kPB * (kPB + 1) / 2;
+
+// The helper warps' own barrier (192 threads), and the one on which warp 0 waits for them.
+__device__ __forceinline__ void helper_sync() { asm volatile("bar.sync 1, 192;" ::: "memory"); }
+__device__ __forceinline__ void inverse_arrive() { asm volatile("bar.arrive 2, 224;" ::: "memory"); }
+__device__ __forceinline__ void inverse_wait() { asm volatile("bar.sync 2, 224;" ::: "memory"); }
 
 __device__ __noinline__ void report_pivot(int s, const PlanDev& pd, int* err) {
     if ((threadIdx.x & 31) != 0) return;
@@ -277,63 +296,143 @@ __device__ __noinline__ void report_pivot(int s, const PlanDev& pd, int* err) {
     pd.lp_fail[pd.sn_lp[s]] = 1;
 }
 
-// Entry e of the lower triangle that starts at c0 + 16, less the 16 columns at c0.
-template <class T>
-__device__ __forceinline__ void trail_entry(T* A, int c0, int e) {
-    int i, j;
-    tri_index(e, i, j);
-    const T* a = A + (c0 + kPB + i) * LDS + c0;
-    const T* b = A + (c0 + kPB + j) * LDS + c0;
-    T v = a[kPB + j];
-#pragma unroll
-    for (int q = 0; q < kPB; ++q) v -= a[q] * b[q];
-    A[(c0 + kPB + i) * LDS + c0 + kPB + j] = v;
+// Pivots that pivot_root() takes: positive, in FP64 also finite and so large that the
+// residual p - d^2 is a normal number (tested without the FP64 pipe).
+__device__ __forceinline__ bool plain_pivot(float p) { return p > 0.f; }
+__device__ __forceinline__ bool plain_pivot(double p) {
+    return static_cast<unsigned>(__double2hiint(p)) - 0x08000000u < 0x7ff00000u - 0x08000000u;
 }
 
-// ---- FP32 tile: L, and its explicit inverse (column-major in Linv) for the panel solve
-// and the triangular solves. Bound by the latency of the pivot chain, so warp 0 factors
-// a diagonal block from registers (shuffles, no barrier) while the other warps apply the
-// previous block's update to the rows below and form the inverse's block rows that are
-// already known. Every entry keeps its ascending sequence of fused multiply-adds, so the
-// result does not depend on the schedule. One tile: 38 -> 20 us.
+__device__ __forceinline__ float fma_ordered(float x, float y, float z) { return fmaf(x, y, z); }
+// FP64: in program order with the other ordered ones.
+__device__ __forceinline__ double fma_ordered(double x, double y, double z) {
+    double r;
+    asm volatile("fma.rn.f64 %0, %1, %2, %3;" : "=d"(r) : "d"(x), "d"(y), "d"(z));
+    return r;
+}
 
-// The helper warps' own barrier (192 threads).
-__device__ __forceinline__ void helper_sync() { asm volatile("bar.sync 1, 192;" ::: "memory"); }
+// d = sqrt(p) and rd = 1 / d, correctly rounded (p > 0). `fill(n)` is called between the
+// parts, n = 0, 1, ..: independent work for the time they leave idle.
+template <class Fill>
+__device__ __forceinline__ void pivot_root(float p, float& d, float& rd, Fill fill) {
+    d = sqrtf(p);
+    rd = 1.f / d;
+    for (int n = 0; n < 4; ++n) fill(n);
+}
+// FP64: y ~ p^(-1/2) to about 2^-45 without the FP64 pipe: the mantissa m in [1, 4) as two
+// floats, the approximate unit's seed y0, e = 1 - m y0^2 with the square's low part, and one
+// third-order step, whose correction is added to y0's bits as an integer. Then d0 = p y, the
+// residual corrections d = d0 + (p - d0^2) y / 2 and rd = y + (1 - d y) y (Markstein 1990),
+// whose last rounding is the correct one unless the exact value lies within about 2^-90 of a
+// rounding boundary.
+template <class Fill>
+__device__ __forceinline__ void pivot_root(double p, double& d, double& rd, Fill fill) {
+    const int hi = __double2hiint(p), lo = __double2loint(p);
+    const unsigned ex = static_cast<unsigned>(hi) >> 20;
+    const int odd = (static_cast<int>(ex) - 1023) & 1, half = (static_cast<int>(ex) - 1023 - odd) >> 1;
+    const float mh = __int_as_float(((127 + odd) << 23) | ((hi & 0xfffff) << 3) |
+                                    static_cast<int>(static_cast<unsigned>(lo) >> 29));
+    const float ml = static_cast<float>(lo & 0x1fffffff) * (odd ? 0x1p-51f : 0x1p-52f);
+    float y0;
+    asm volatile("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(mh));
+    fill(0);
+    y0 = fminf(fmaxf(y0, 0.5f), 0x1.fffffep-1f);
+    const float q = y0 * y0, ql = fmaf(y0, y0, -q);
+    const float e = fmaf(-ml, q, fmaf(-mh, ql, fmaf(-mh, q, 1.f)));
+    const float f = y0 * e * fmaf(0.375f, e, 0.5f) * 0x1p53f;       // in units of y0's last FP64 bit
+    int c;
+    asm volatile("cvt.rni.s32.f32 %0, %1;" : "=r"(c) : "f"(f));
+    fill(1);
+    long long bits = (static_cast<long long>(__float_as_int(y0)) << 29) + (896LL << 52) + c;
+    bits -= static_cast<long long>(half) << 52;
+    const double y = __longlong_as_double(bits), yh = __longlong_as_double(bits - (1LL << 52));
+    const double d0 = fma_ordered(p, y, 0.0);
+    fill(2);
+    const double res = fma_ordered(__longlong_as_double(__double_as_longlong(d0) ^ (1LL << 63)), d0, p);
+    d = fma_ordered(res, yh, d0);
+    const double t = fma_ordered(__longlong_as_double(__double_as_longlong(d) ^ (1LL << 63)), y, 1.0);
+    rd = fma_ordered(t, y, y);
+    fill(3);
+}
 
-// Warp 0: the diagonal block at c0; lane (r, h) holds the columns 2k + h of row r. Leaves
-// L in A and 1 / L(c, c) in rdiag. A pivot that is not positive counts as 1 (result true).
-__device__ __forceinline__ bool factor_block(float* A, float* rdiag, int c0) {
-    const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
+// The diagonal block at c0 from its column j on, for any pivot: one that is not positive
+// counts as 1 (result true). Warp 0.
+template <class T>
+__device__ __noinline__ bool factor_rest(T* A, T* rdiag, int c0, int j) {
+    const int lane = threadIdx.x & 31, r = c0 + (lane & 15);
     bool bad = false;
-    float v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int c = 2 * k + h;
-        v[k] = r >= c ? A[(c0 + r) * LDS + c0 + c] : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < kPB; ++j) {
-        const float a = __shfl_sync(0xffffffffu, v[j >> 1], r + 16 * (j & 1));    // column j of every row
-        float p = __shfl_sync(0xffffffffu, v[j >> 1], j + 16 * (j & 1));
-        const bool ok = p > 0.f;
-        bad |= !ok;
-        p = ok ? p : 1.f;
-        const float d = sqrtf(p);
-        const float rd = 1.f / d;
-        const float l = a * rd;
-        if (h == 0 && r >= j) A[(c0 + r) * LDS + c0 + j] = r == j ? d : l;
-        if (lane == 0) rdiag[c0 + j] = rd;
-#pragma unroll
-        for (int k = j >> 1; k < 8; ++k) {
-            if (2 * k + 1 <= j) continue;
-            const float lc = __shfl_sync(0xffffffffu, l, 2 * k + h);
-            if (2 * k + h > j) v[k] = fmaf(-l, lc, v[k]);
+    for (; j < kPB; ++j) {
+        const int c = c0 + j;
+        T p = A[c * LDS + c];
+        if (!(p > T(0))) {
+            bad = true;
+            p = T(1);
         }
+        const T d = sqrt(p), rd = T(1) / d;
+        __syncwarp();
+        if (lane < kPB && r > c) A[r * LDS + c] *= rd;
+        if (lane == 0) {
+            A[c * LDS + c] = d;
+            rdiag[c] = rd;
+        }
+        __syncwarp();
+        if (r > c)
+            for (int q = c + 1 + (lane >> 4); q <= r; q += 2) A[r * LDS + q] -= A[r * LDS + c] * A[q * LDS + c];
+        __syncwarp();
     }
     return bad;
 }
 
-// Rows below block c0: the block's columns of L, one thread per row.
+// Warp 0: the diagonal block at c0; lane (r, h) holds the columns 2k + h of row r. Leaves
+// L in A and 1 / L(c, c) in rdiag. Result: a pivot was not positive (it counts as 1).
+// Column j updates column j + 1 at once and the others while the next pivot's root forms.
+template <class T>
+__device__ __forceinline__ bool factor_block(T* A, T* rdiag, int c0) {
+    const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
+    T v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int c = 2 * k + h;
+        v[k] = r >= c ? A[(c0 + r) * LDS + c0 + c] : T(0);
+    }
+    T l = T(0);
+#pragma unroll
+    for (int j = 0; j < kPB; ++j) {
+        const T a = __shfl_sync(0xffffffffu, v[j >> 1], r + 16 * (j & 1));    // column j of every row
+        const T p = __shfl_sync(0xffffffffu, v[j >> 1], j + 16 * (j & 1));
+        auto update = [&](int k, int from) {           // columns 2k, 2k + 1 by column `from`
+            const T lc = __shfl_sync(0xffffffffu, l, 2 * k + h);
+            const T t = fma_ordered(-l, lc, v[k]);
+            v[k] = 2 * k + h > from ? t : v[k];
+        };
+        T d, rd;
+        const int rest = (j >> 1) + 1;                 // column j - 1's columns still to update: 2 rest ..
+        if (!plain_pivot(p)) {
+#pragma unroll
+            for (int k = rest; k < 8; ++k)
+                if (j > 0) update(k, j - 1);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (2 * k + h >= j && r >= 2 * k + h) A[(c0 + r) * LDS + c0 + 2 * k + h] = v[k];
+            __syncwarp();
+            return factor_rest(A, rdiag, c0, j);
+        }
+        pivot_root(p, d, rd, [&](int n) {
+            if (j == 0) return;
+            if (rest + n < 8) update(rest + n, j - 1);
+            if (n == 3)
+#pragma unroll
+                for (int k = rest + 4; k < 8; ++k) update(k, j - 1);
+        });
+        l = a * rd;
+        if (j + 1 < kPB) update((j + 1) >> 1, j);
+        if (h == 0 && r >= j) A[(c0 + r) * LDS + c0 + j] = r == j ? d : l;
+        if (lane == 0) rdiag[c0 + j] = rd;
+    }
+    return false;
+}
+
+// Rows below block c0 (nt of them): the block's columns of L. FP32: one thread per row.
 __device__ __forceinline__ void panel_rows(float* A, const float* rdiag, int c0, int nt) {
     if (static_cast<int>(threadIdx.x) >= nt) return;
     float* row = A + (c0 + kPB + threadIdx.x) * LDS + c0;
@@ -349,8 +448,65 @@ __device__ __forceinline__ void panel_rows(float* A, const float* rdiag, int c0,
 #pragma unroll
     for (int c = 0; c < kPB; ++c) row[c] = x[c];
 }
+// FP64: a warp takes 8 rows, lane (r, g) their columns 4k + g.
+__device__ __forceinline__ void panel_rows(double* A, const double* rdiag, int c0, int nt) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (8 * wid >= nt) return;
+    const int r = c0 + kPB + 8 * wid + (lane & 7), g = lane >> 3;
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = A[r * LDS + c0 + 4 * k + g];
+#pragma unroll
+    for (int q = 0; q < kPB; ++q) {
+        const double t = v[q >> 2] * rdiag[c0 + q];
+        if (g == (q & 3)) v[q >> 2] = t;
+        if (q == kPB - 1) break;
+        const double x = __shfl_sync(0xffffffffu, t, (lane & 7) + 8 * (q & 3));
+#pragma unroll
+        for (int k = (q + 1) >> 2; k < 4; ++k)
+            if (4 * k + g > q) v[k] = fma(-x, A[(c0 + 4 * k + g) * LDS + c0 + q], v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) A[r * LDS + c0 + 4 * k + g] = v[k];
+}
 
-// The inverse's diagonal block at c0: thread j < 16 forms column j.
+// Entry e of the lower triangle that starts at c0 + 16, less the 16 columns at c0.
+template <class T>
+__device__ __forceinline__ void trail_entry(T* A, int c0, int e) {
+    int i, j;
+    tri_index(e, i, j);
+    const T* a = A + (c0 + kPB + i) * LDS + c0;
+    const T* b = A + (c0 + kPB + j) * LDS + c0;
+    T v = a[kPB + j];
+#pragma unroll
+    for (int q = 0; q < kPB; ++q) v -= a[q] * b[q];
+    A[(c0 + kPB + i) * LDS + c0 + kPB + j] = v;
+}
+
+// The same for a square of two rows and two columns (e: row by row).
+template <class T>
+__device__ __forceinline__ void trail_square(T* A, int c0, int e) {
+    int i, j;
+    tri_index(e, i, j);
+    const T* a = A + (c0 + kPB + 2 * i) * LDS + c0;
+    const T* b = A + (c0 + kPB + 2 * j) * LDS + c0;
+    T* out = A + (c0 + kPB + 2 * i) * LDS + c0 + kPB + 2 * j;
+    T v00 = out[0], v01 = i == j ? T(0) : out[1], v10 = out[LDS], v11 = out[LDS + 1];
+#pragma unroll
+    for (int q = 0; q < kPB; ++q) {
+        const T a0 = a[q], a1 = a[LDS + q], b0 = b[q], b1 = b[LDS + q];
+        v00 -= a0 * b0;
+        v01 -= a0 * b1;
+        v10 -= a1 * b0;
+        v11 -= a1 * b1;
+    }
+    out[0] = v00;
+    if (i != j) out[1] = v01;
+    out[LDS] = v10;
+    out[LDS + 1] = v11;
+}
+
+// The inverse's diagonal block at c0. FP32: thread j < 16 forms column j.
 __device__ __forceinline__ void inverse_block(const float* A, float* X, const float* rdiag, int c0, int j) {
     if (j >= kPB) return;
     float x[kPB];
@@ -366,62 +522,136 @@ __device__ __forceinline__ void inverse_block(const float* A, float* X, const fl
     for (int i = 0; i < kPB; ++i)
         if (i >= j) X[(c0 + i) * LDS + c0 + j] = x[i];
 }
+// FP64: warps t / 32 < 4 take four columns each, lane (c, g) the rows 8k + g of column c.
+__device__ __forceinline__ void inverse_block(const double* A, double* X, const double* rdiag, int c0, int t) {
+    if (t >= 128) return;
+    const int lane = t & 31, c = lane & 3, g = lane >> 2, j = (t >> 5) * 4 + c;
+    double x[2] = {g == j ? 1.0 : 0.0, g + 8 == j ? 1.0 : 0.0};
+#pragma unroll
+    for (int q = 0; q < kPB; ++q) {
+        const double t1 = x[q >> 3] * rdiag[c0 + q];
+        if (g == (q & 7)) x[q >> 3] = t1;
+        if (q == kPB - 1) break;
+        const double xq = __shfl_sync(0xffffffffu, t1, c + 4 * (q & 7));
+#pragma unroll
+        for (int k = (q + 1) >> 3; k < 2; ++k)
+            if (8 * k + g > q) x[k] = fma(-A[(c0 + 8 * k + g) * LDS + c0 + q], xq, x[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (8 * k + g >= j) X[(c0 + 8 * k + g) * LDS + c0 + j] = x[k];
+}
 
 // Block row at r0 of the inverse: T(i, j) = sum_{j <= q < r0} L(i, q) X(q, j) for the
-// columns j < r0, kept transposed in X's upper triangle, then X(i, j) = -sum_q
-// X(i, r0 + q) T(r0 + q, j).
-__device__ __forceinline__ void inverse_sums(const float* A, float* X, int r0, int t, int step) {
-    for (int e = t; e < r0 * kPB; e += step) {
-        const int i = r0 + (e % (kPB * kPB)) / kPB, j = (e / (kPB * kPB)) * kPB + e % kPB;
-        float acc = 0.f;
-        for (int q = j; q < r0; ++q) acc += A[i * LDS + q] * X[q * LDS + j];
-        X[j * LDS + i] = acc;
+// columns j < r0, kept transposed in X's upper triangle (e: rows i, i + 8 of kCols columns),
+// then X(i, j) = -sum_q X(i, r0 + q) T(r0 + q, j) (e: row i of kCols columns). FP32 is bound
+// by its shared loads here and takes two columns at a time, FP64 by how evenly the
+// warps' instructions are dealt out (with two columns 134k cycles a tile, with one 130k).
+template <class T> constexpr int kCols = sizeof(T) == 4 ? 2 : 1;
+
+template <class T>
+__device__ __forceinline__ void inverse_sums(const T* A, T* X, int r0, int e) {
+    constexpr int C = kCols<T>, per = kPB * kPB / (2 * C);
+    const int i = r0 + (e % per) / (kPB / C), j = (e / per) * kPB + C * (e % (kPB / C));
+    const T* a = A + i * LDS;
+    T u[C], v[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) u[c] = v[c] = T(0);
+    if (C == 2) {
+        u[0] = a[j] * X[j * LDS + j];
+        v[0] = a[8 * LDS + j] * X[j * LDS + j];
+    }
+#pragma unroll 2
+    for (int q = j + C - 1; q < r0; ++q) {
+        const T a0 = a[q], a1 = a[8 * LDS + q];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const T x = X[q * LDS + j + c];
+            u[c] += a0 * x;
+            v[c] += a1 * x;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        X[(j + c) * LDS + i] = u[c];
+        X[(j + c) * LDS + i + 8] = v[c];
     }
 }
-__device__ __forceinline__ void inverse_rows(float* X, int r0, int t, int step) {
-    for (int e = t; e < r0 * kPB; e += step) {
-        const int rr = (e % (kPB * kPB)) / kPB, i = r0 + rr, j = (e / (kPB * kPB)) * kPB + e % kPB;
-        float acc = 0.f;
-        for (int q = 0; q <= rr; ++q) acc += X[i * LDS + r0 + q] * X[j * LDS + r0 + q];
-        X[i * LDS + j] = -acc;
+template <class T>
+__device__ __forceinline__ void inverse_rows(T* X, int r0, int e) {
+    constexpr int C = kCols<T>;
+    const int nj = r0 / C, i = r0 + e / nj, j = C * (e % nj);
+    T u[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) u[c] = T(0);
+    for (int q = r0; q <= i; ++q) {
+        const T x = X[i * LDS + q];
+#pragma unroll
+        for (int c = 0; c < C; ++c) u[c] += x * X[(j + c) * LDS + q];
     }
+#pragma unroll
+    for (int c = 0; c < C; ++c) X[i * LDS + j + c] = -u[c];
 }
 
-__device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, float* F, float* __restrict__ Linv,
+template <class T>
+__device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, T* F, T* __restrict__ Linv,
                                         const int64_t* __restrict__ inv_off, int* err, unsigned char* smraw) {
-    float* A = reinterpret_cast<float*>(smraw);   // A[r * LDS + c], lower triangle
-    float* X = A + T64 * LDS;                     // L^{-1}, same layout
-    float* rdiag = X + T64 * LDS;                 // 1 / L(c, c)
+    T* A = reinterpret_cast<T*>(smraw);   // A[r * LDS + c], lower triangle
+    T* X = A + T64 * LDS;                 // L^{-1}, same layout
+    T* rdiag = X + T64 * LDS;             // 1 / L(c, c)
+    int* next = reinterpret_cast<int*>(rdiag + T64);   // per block: the next 32 of its helpers' entries
     const int LD = pd.sn_lda[s];
     const int k0 = kstep * T64;
     const int w = min(T64, pd.sn_ncols[s] - k0);
-    float* Fs = F + pd.F_off[s];
-    const int tid = threadIdx.x, wid = tid >> 5;
+    T* Fs = F + pd.F_off[s];
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
 #pragma unroll 4
     for (int it = 0; it < 16; ++it) {
         const int idx = tid + it * 256;
         const int r = idx & 63, c = idx >> 6;
         if (c > r) continue;
-        float x = 0.f;
+        T x = T(0);
         if (r < w && c < w) x = Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD];
-        else if (r == c) x = 1.f;
+        else if (r == c) x = T(1);
         A[r * LDS + c] = x;
     }
+    if (tid < 12) next[tid] = 0;
     __syncthreads();
-    const int ht = (wid < 4 ? wid - 1 : wid - 2) * 32 + (tid & 31);   // helpers: warps 1-3 and 5-7
+    const int ht = (wid < 4 ? wid - 1 : wid - 2) * 32 + lane;   // helpers: warps 1-3 and 5-7
+    // 32 entries of [0, n) at a time, to whichever helper is free
+    auto share = [&](int* counter, int n, auto&& work) {
+        for (;;) {
+            int e = 0;
+            if (lane == 0) e = atomicAdd(counter, 32);
+            e = __shfl_sync(0xffffffffu, e, 0);
+            if (e >= n) break;
+            if (e + lane < n) work(e + lane);
+            __syncwarp();
+        }
+    };
     for (int c0 = 0; c0 < T64; c0 += kPB) {
         const int nt = T64 - kPB - c0;
-        if (wid == 0) {
-            if (factor_block(A, rdiag, c0)) report_pivot(s, pd, err);
-        } else if (wid != 4 && c0 > 0) {
-            for (int e = kPBTri + ht; e < (nt + kPB) * (nt + kPB + 1) / 2; e += 192) trail_entry(A, c0 - kPB, e);
-            inverse_block(A, X, rdiag, c0 - kPB, ht);
-            helper_sync();
-            if (c0 > kPB) {
-                inverse_rows(X, c0 - kPB, ht, 192);
+        int* counter = next + (c0 / kPB) * 3;
+        const bool helper = (wid & 3) != 0;
+        if (wid == 0 && factor_block(A, rdiag, c0)) report_pivot(s, pd, err);
+        if (c0 > 0) {
+            if (helper) {
+                inverse_block(A, X, rdiag, c0 - kPB, ht);
                 helper_sync();
+                if (c0 > kPB) share(counter, (c0 - kPB) * kPB / kCols<T>, [&](int e) { inverse_rows(X, c0 - kPB, e); });
             }
-            inverse_sums(A, X, c0, ht, 192);
+            if (wid != 4) {
+                // warp 0 joins once its block is done and the inverse's last block row is there
+                if (helper) { helper_sync(); inverse_arrive(); }
+                else inverse_wait();
+                share(counter + 1, c0 * kPB / (2 * kCols<T>), [&](int e) { inverse_sums(A, X, c0, e); });
+                // less the diagonal block's entries or squares
+                constexpr int C = kCols<T>, kDone = kPB / C * (kPB / C + 1) / 2;
+                share(counter + 2, (nt + kPB) / C * ((nt + kPB) / C + 1) / 2 - kDone, [&](int e) {
+                    if constexpr (C == 2) trail_square(A, c0 - kPB, kDone + e);
+                    else trail_entry(A, c0 - kPB, kDone + e);
+                });
+            }
         }
         __syncthreads();
         if (nt == 0) break;
@@ -432,172 +662,20 @@ __device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, float* F, 
     }
     inverse_block(A, X, rdiag, T64 - kPB, tid);
     __syncthreads();
-    inverse_rows(X, T64 - kPB, tid, 256);
+    for (int e = tid; e < (T64 - kPB) * kPB / kCols<T>; e += 256) inverse_rows(X, T64 - kPB, e);
     __syncthreads();
-    float* Li = Linv + inv_off[s] + static_cast<int64_t>(kstep) * T64 * T64;
+    T* Li = Linv + inv_off[s] + static_cast<int64_t>(kstep) * T64 * T64;
 #pragma unroll 4
     for (int it = 0; it < 16; ++it) {
         const int idx = tid + it * 256;
         const int r = idx & 63, c = idx >> 6;
         const bool in = r < w && c <= r;
         if (in) Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD] = A[r * LDS + c];
-        Li[r + c * T64] = in ? X[r * LDS + c] : 0.f;
+        Li[r + c * T64] = in ? X[r * LDS + c] : T(0);
     }
 }
 
-// ---- FP64 tile: L only (k_trsm_rows forms the inverse beside the panel). A warp's FP64
-// instruction takes 64 cycles of its SM quarter's pipe whatever its active lanes, a
-// dependent one follows at once, and shuffles and shared loads go through the same queue
-// (measured: sqrt 600 cycles, a division 355, a 64-bit shuffle 16). So the tile is bound
-// by the number of FP64 instructions per quarter:
-//  * elimination as a_rc -= (a_rj / p_j) a_cj: only a reciprocal sits between two pivots
-//    (seed of the approximate unit and one third-order step, folded into the product
-//    with the row); the square roots of a block are taken together, off the chain.
-//  * the diagonal block is spread over four warps, one per quarter, that exchange a
-//    column through shared memory: 6 FP64 instructions per column and quarter.
-//  * all eight warps take the rows below and the trailing update.
-// One tile: 116 -> 30 us.
-
-// p > 0 without the FP64 pipe (false for NaN).
-__device__ __forceinline__ bool is_positive(double p) {
-    const long long b = __double_as_longlong(p);
-    return b > 0 && b <= 0x7ff0000000000000LL;
-}
-
-// Threads 0..127: the diagonal block at c0. Thread (r, g) holds the columns g and g + 8
-// of row r. Leaves the Schur complement's columns (L before its scaling) in A's lower
-// triangle, the unit factor's column j in A's upper triangle (row j) and the pivots in
-// piv. col: 2 x 16 values. A pivot that is not positive counts as 1 (result true).
-__device__ __forceinline__ bool factor_block(double* A, double* piv, double* col, int c0) {
-    const int r = threadIdx.x & 15, g = threadIdx.x >> 4, wid = threadIdx.x >> 5;
-    bool bad = false;
-    double v0 = r >= g ? A[(c0 + r) * LDS + c0 + g] : 0.0;
-    double v1 = r >= g + 8 ? A[(c0 + r) * LDS + c0 + g + 8] : 0.0;
-#pragma unroll
-    for (int j = 0; j < kPB; ++j) {
-        double* cb = col + (j & 1) * kPB;
-        if (g == (j & 7)) cb[r] = j < 8 ? v0 : v1;
-        asm volatile("bar.sync 2, 128;" ::: "memory");
-        double p = cb[j];
-        const double a = cb[r], b0 = cb[g], b1 = cb[g + 8];
-        const bool ok = is_positive(p);
-        bad |= !ok;
-        p = ok ? p : 1.0;
-        // u = a / p: y0 = 1/p to about 2^-19, e = 1 - p y0, 1/p = y0 (1 + e + e^2 + O(e^3))
-        double y0;
-        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(p));
-        const double e = fma(-p, y0, 1.0);
-        const double w = a * y0;
-        const double u = fma(w, fma(e, e, e), w);
-        if (j + 1 < 8) {
-            if (2 * wid + 1 > j && g > j) v0 = fma(-u, b0, v0);
-            v1 = fma(-u, b1, v1);
-        } else if (2 * wid + 9 > j && g + 8 > j) {
-            v1 = fma(-u, b1, v1);
-        }
-        if (g == 0) {
-            if (r >= j) A[(c0 + r) * LDS + c0 + j] = a;
-            if (r > j) A[(c0 + j) * LDS + c0 + r] = u;
-            if (r == j) piv[c0 + j] = p;
-        }
-    }
-    return bad;
-}
-
-// Rows below block c0, all eight warps: a warp takes 8 rows, lane (r, g) their columns
-// 4k + g. The update with the unit factor needs no pivot's square root, which warp 7
-// takes meanwhile; the columns are scaled after the barrier.
-__device__ __forceinline__ void panel_rows(double* A, double* piv, double* rdiag, int c0, int nt) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int r = c0 + kPB + 8 * wid + (lane & 7), g = lane >> 3;
-    const bool on = 8 * wid < nt;
-    double v[4];
-    if (on) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = A[r * LDS + c0 + 4 * k + g];
-#pragma unroll
-        for (int q = 0; q < kPB - 1; ++q) {
-            const double x = __shfl_sync(0xffffffffu, v[q >> 2], (lane & 7) + 8 * (q & 3));
-#pragma unroll
-            for (int k = q >> 2; k < 4; ++k) {
-                if (4 * k + 3 <= q) continue;
-                if (4 * k + g > q) v[k] = fma(-x, A[(c0 + q) * LDS + c0 + 4 * k + g], v[k]);
-            }
-        }
-    } else if (wid == 7 && lane < kPB) {
-        const double d = sqrt(piv[c0 + lane]);
-        piv[c0 + lane] = d;
-        rdiag[c0 + lane] = 1.0 / d;
-    }
-    __syncthreads();
-    if (on)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) A[r * LDS + c0 + 4 * k + g] = v[k] * rdiag[c0 + 4 * k + g];
-}
-
-// L's own diagonal block at c0, whose columns are still unscaled (t = 0 .. step - 1).
-__device__ __forceinline__ void scale_block(double* A, const double* piv, const double* rdiag, int c0, int t,
-                                            int step) {
-    for (int e = t; e < kPBTri; e += step) {
-        int i, j;
-        tri_index(e, i, j);
-        const int at = (c0 + i) * LDS + c0 + j;
-        A[at] = i == j ? piv[c0 + i] : A[at] * rdiag[c0 + j];
-    }
-}
-
-__device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, double* F, double*, const int64_t*, int* err,
-                                        unsigned char* smraw) {
-    double* A = reinterpret_cast<double*>(smraw);   // A[r * LDS + c]
-    double* rdiag = A + T64 * LDS;                  // 1 / L(c, c)
-    double* piv = rdiag + T64;                      // pivots, then L(c, c)
-    double* col = piv + T64;
-    const int LD = pd.sn_lda[s];
-    const int k0 = kstep * T64;
-    const int w = min(T64, pd.sn_ncols[s] - k0);
-    double* Fs = F + pd.F_off[s];
-    const int tid = threadIdx.x;
-#pragma unroll 4
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256;
-        const int r = idx & 63, c = idx >> 6;
-        if (c > r) continue;
-        double x = 0.0;
-        if (r < w && c < w) x = Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD];
-        else if (r == c) x = 1.0;
-        A[r * LDS + c] = x;
-    }
-    __syncthreads();
-    for (int c0 = 0; c0 < T64; c0 += kPB) {
-        const int nt = T64 - kPB - c0;
-        if (tid < 128) {
-            if (factor_block(A, piv, col, c0)) report_pivot(s, pd, err);
-        } else if (c0 > 0) {
-            scale_block(A, piv, rdiag, c0 - kPB, tid - 128, 128);
-        }
-        __syncthreads();
-        panel_rows(A, piv, rdiag, c0, nt);
-        __syncthreads();
-        for (int e = tid; e < nt * (nt + 1) / 2; e += 256) trail_entry(A, c0, e);
-        __syncthreads();
-    }
-    scale_block(A, piv, rdiag, T64 - kPB, tid, 256);
-    __syncthreads();
-#pragma unroll 4
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256;
-        const int r = idx & 63, c = idx >> 6;
-        if (r < w && c <= r) Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD] = A[r * LDS + c];
-    }
-}
-
-constexpr size_t potrf_smem(size_t elem) {
-    return elem == 4 ? (2 * T64 * LDS + T64) * elem : (T64 * LDS + 2 * T64 + 2 * kPB) * elem;
-}
-
-constexpr size_t update_smem(size_t elem) {      // two 64x64 panel tiles, then potrf_tile
-    return 2 * T64 * T64 * elem > potrf_smem(elem) ? 2 * T64 * T64 * elem : potrf_smem(elem);
-}
+constexpr size_t potrf_smem(size_t elem) { return (2 * T64 * LDS + T64) * elem + 12 * sizeof(int); }
 
 // Diagonal-tile Cholesky of the first step of each front of a level (later steps
 // are factored at the end of the previous step's update, see k_update).
@@ -655,115 +733,96 @@ __global__ void __launch_bounds__(256) k_trsm(StepArgs a, const int* __restrict_
         }
 }
 
-// FP64 panel rows below the diagonal tile, X L_kk^T = B by substitution, and the tile's
-// inverse, which is the same for the rows of the identity (X = L_kk^{-T}). Bound by the
-// FP64 pipe (2080 multiply-adds a row, 2 a cycle and SM), so a block takes only 16 rows:
-// two per warp, lane (row, c) their columns 16 b + c. That fills the chip from 600 rows
-// on, where 64-row tiles that multiply by the inverse left most SMs idle (69 us a step at
-// any size up to 9700 rows; now 9 us up to 1200 rows, and the inverse is off the chain of
-// the diagonal tile). Each 16-column block first takes the columns before it, then runs
-// its own substitution with shuffles. The first 4 * tiles blocks are the 16-row parts of
-// the step's 64-row tiles, the other 4 * nitems the identity's rows of each front.
-constexpr int kTrRows = 16;
+// FP64 panel rows below the diagonal tile, X = B Linv^T. Bound by the FP64 pipe (2560
+// multiply-adds a row, 2 a cycle and SM), so a block takes only 2 W rows: two per warp, lane
+// (row, c) their columns 16 b + c, each an ascending sum over the columns up to its own
+// block's end (the inverse is 0 beyond its diagonal). With 64-row tiles a step took 69 us at
+// any size up to 9700 rows; now 10 us up to 1200 rows and 26 us at 4700.
 constexpr int kTrLd = T64 + 2;              // 16-byte aligned rows, no bank conflicts
-constexpr size_t kTrSmem = (T64 * kTrLd + kTrRows * kTrLd + T64) * sizeof(double);
+constexpr size_t tr_smem(int warps) { return (T64 + 2 * warps) * kTrLd * sizeof(double); }
 
-__global__ void __launch_bounds__(256) k_trsm_rows(StepArgs a, const int* __restrict__ items,
-                                                   const int* __restrict__ prefix, PlanDev pd, double* F,
-                                                   double* __restrict__ Linv, const int64_t* __restrict__ inv_off,
-                                                   int tiles) {
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_trsm_rows(StepArgs a, const int* __restrict__ items,
+                                                      const int* __restrict__ prefix, PlanDev pd, double* F,
+                                                      const double* __restrict__ Linv,
+                                                      const int64_t* __restrict__ inv_off) {
+    constexpr int kRows = 2 * W, kParts = T64 / kRows, kT = 32 * W;
     extern __shared__ __align__(16) unsigned char smraw[];
-    double* L = reinterpret_cast<double*>(smraw);   // unit lower factor, L[c * kTrLd + q]
+    double* L = reinterpret_cast<double*>(smraw);   // the tile's inverse, L[c * kTrLd + q]
     double* X = L + T64 * kTrLd;                    // the block's rows, X[r * kTrLd + c]
-    double* rd = X + kTrRows * kTrLd;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int sub = blockIdx.x & 3, unit = blockIdx.x >> 2;
-    const bool ident = unit >= tiles;
-    const int i = ident ? unit - tiles : find_item(prefix + a.tp_off, a.nitems, unit);
+    const int sub = blockIdx.x % kParts, unit = blockIdx.x / kParts;
+    const int i = find_item(prefix + a.tp_off, a.nitems, unit);
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
     const int N = pd.sn_nrows[s], LD = pd.sn_lda[s];
     const int k0 = a.k * T64;
     const int w = min(T64, pd.sn_ncols[s] - k0);
-    const int r0 = ident ? sub * kTrRows : k0 + w + (unit - prefix[a.tp_off + i]) * T64 + sub * kTrRows;
-    const int nr = ident ? kTrRows : min(kTrRows, N - r0);
+    const int r0 = k0 + w + (unit - prefix[a.tp_off + i]) * T64 + sub * kRows;
+    const int nr = min(kRows, N - r0);
     if (nr <= 0) return;
     double* Fs = F + pd.F_off[s];
-    if (tid < T64) rd[tid] = tid < w ? 1.0 / Fs[(k0 + tid) + static_cast<int64_t>(k0 + tid) * LD] : 1.0;
-    double l[16], x[4];
+    const double* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;
+    double l[T64 * T64 / kT], x[4];
 #pragma unroll
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256, c = idx & 63, q = idx >> 6;
-        l[it] = c < w && q < c ? Fs[(k0 + c) + static_cast<int64_t>(k0 + q) * LD] : 0.0;
+    for (int it = 0; it < T64 * T64 / kT; ++it) l[it] = Li[tid + it * kT];
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+        const int idx = tid + it * kT, r = idx % kRows, c = idx / kRows;
+        x[it] = r < nr && c < w ? Fs[(r0 + r) + static_cast<int64_t>(k0 + c) * LD] : 0.0;
+    }
+#pragma unroll
+    for (int it = 0; it < T64 * T64 / kT; ++it) {
+        const int idx = tid + it * kT;
+        L[(idx & 63) * kTrLd + (idx >> 6)] = l[it];
     }
 #pragma unroll
     for (int it = 0; it < 4; ++it) {
-        const int idx = tid + it * 256, r = idx & 15, c = idx >> 4;
-        if (ident) x[it] = r0 + r == c ? 1.0 : 0.0;
-        else x[it] = r < nr && c < w ? Fs[(r0 + r) + static_cast<int64_t>(k0 + c) * LD] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256, c = idx & 63, q = idx >> 6;
-        if (q < c) L[c * kTrLd + q] = l[it] * rd[q];
-    }
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const int idx = tid + it * 256;
-        X[(idx & 15) * kTrLd + (idx >> 4)] = x[it];
+        const int idx = tid + it * kT;
+        X[(idx % kRows) * kTrLd + idx / kRows] = x[it];
     }
     __syncthreads();
     const int c = lane & 15;
     double* xr = X + (2 * wid + (lane >> 4)) * kTrLd;
-    const int b0 = ident ? sub : 0;            // rows of the identity are 0 before their own block
-    for (int b = b0; b < T64 / 16; ++b) {
+    double out[T64 / 16];
+#pragma unroll
+    for (int b = 0; b < T64 / 16; ++b) {
         const double* lc = L + (16 * b + c) * kTrLd;
-        double v = xr[16 * b + c];
-        for (int q = 16 * b0; q < 16 * b; q += 4) {
+        double v = 0.0;
+#pragma unroll 2
+        for (int q = 0; q < 16 * (b + 1); q += 4) {
             const double2 x0 = *reinterpret_cast<const double2*>(xr + q);
             const double2 x1 = *reinterpret_cast<const double2*>(xr + q + 2);
             const double2 l0 = *reinterpret_cast<const double2*>(lc + q);
             const double2 l1 = *reinterpret_cast<const double2*>(lc + q + 2);
-            v = fma(-x0.x, l0.x, v);
-            v = fma(-x0.y, l0.y, v);
-            v = fma(-x1.x, l1.x, v);
-            v = fma(-x1.y, l1.y, v);
+            v = fma(x0.x, l0.x, v);
+            v = fma(x0.y, l0.y, v);
+            v = fma(x1.x, l1.x, v);
+            v = fma(x1.y, l1.y, v);
         }
-#pragma unroll
-        for (int q = 0; q < 15; ++q) {
-            const double y = __shfl_sync(0xffffffffu, v, (lane & 16) + q);
-            if (c > q) v = fma(-y, lc[16 * b + q], v);
-        }
-        xr[16 * b + c] = v;
-        __syncwarp();
+        out[b] = v;
     }
+    __syncwarp();
+#pragma unroll
+    for (int b = 0; b < T64 / 16; ++b) xr[16 * b + c] = out[b];
     __syncthreads();
-    double* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;
 #pragma unroll
     for (int it = 0; it < 4; ++it) {
-        const int idx = tid + it * 256;
-        if (ident) {                           // column j of the inverse is row j of X
-            const int q = idx & 63, j = r0 + (idx >> 6);
-            Li[q + j * T64] = q < w && j <= q ? X[(idx >> 6) * kTrLd + q] * rd[q] : 0.0;
-        } else {
-            const int r = idx & 15, q = idx >> 4;
-            if (r < nr && q < w) Fs[(r0 + r) + static_cast<int64_t>(k0 + q) * LD] = X[r * kTrLd + q] * rd[q];
-        }
+        const int idx = tid + it * kT, r = idx % kRows, q = idx / kRows;
+        if (r < nr && q < w) Fs[(r0 + r) + static_cast<int64_t>(k0 + q) * LD] = X[r * kTrLd + q];
     }
 }
 
-// C(64x64) -= A_i (64 x w) A_j^T; 256 threads, 4x4 outputs each. The C tile is
+// FP32 update without the tensor cores, C(64x64) -= A_i (64 x w) A_j^T; 256 threads, 4x4 outputs each. The C tile is
 // read into registers and both panel tiles are staged with fully unrolled loads
 // before any arithmetic, so every global load of a thread is in flight at once.
-template <class T>
 __global__ void __launch_bounds__(256) k_update(StepArgs a, const int* __restrict__ items,
-                                                const int* __restrict__ prefix, PlanDev pd, T* F,
-                                                T* __restrict__ Linv, const int64_t* __restrict__ inv_off,
+                                                const int* __restrict__ prefix, PlanDev pd, float* F,
+                                                float* __restrict__ Linv, const int64_t* __restrict__ inv_off,
                                                 int* err) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    T* As = reinterpret_cast<T*>(smraw);     // [kk][r]
-    T* Bs = As + T64 * T64;                  // [kk][c]
+    float* As = reinterpret_cast<float*>(smraw);     // [kk][r]
+    float* Bs = As + T64 * T64;                  // [kk][c]
     const int i = find_item(prefix + a.up_off, a.nitems, blockIdx.x);
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
@@ -777,26 +836,26 @@ __global__ void __launch_bounds__(256) k_update(StepArgs a, const int* __restric
     const int t0 = k0 + w;
     const int ri0 = t0 + ti * T64, cj0 = t0 + tj * T64;
     const int nri = min(T64, N - ri0), ncj = min(T64, N - cj0);
-    T* Fs = F + pd.F_off[s];
+    float* Fs = F + pd.F_off[s];
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
-    T cv[4][4];
+    float cv[4][4];
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int r = ty * 4 + q, c = tx * 4 + p;
             const bool in = r < nri && c < ncj && (ti != tj || r >= c);
-            cv[q][p] = in ? Fs[(ri0 + r) + static_cast<int64_t>(cj0 + c) * LD] : T(0);
+            cv[q][p] = in ? Fs[(ri0 + r) + static_cast<int64_t>(cj0 + c) * LD] : 0.f;
         }
-    T va[16], vb[16];
+    float va[16], vb[16];
 #pragma unroll
     for (int it = 0; it < 16; ++it) {
         const int idx = tid + it * 256;
         const int r = idx & (T64 - 1), kk = idx >> 6;
         const int64_t cofs = static_cast<int64_t>(k0 + kk) * LD;
-        va[it] = (kk < w && r < nri) ? Fs[ri0 + r + cofs] : T(0);
-        vb[it] = (kk < w && r < ncj) ? Fs[cj0 + r + cofs] : T(0);
+        va[it] = (kk < w && r < nri) ? Fs[ri0 + r + cofs] : 0.f;
+        vb[it] = (kk < w && r < ncj) ? Fs[cj0 + r + cofs] : 0.f;
     }
 #pragma unroll
     for (int it = 0; it < 16; ++it) {
@@ -805,14 +864,14 @@ __global__ void __launch_bounds__(256) k_update(StepArgs a, const int* __restric
         Bs[idx] = vb[it];
     }
     __syncthreads();
-    T acc[4][4];
+    float acc[4][4];
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int p = 0; p < 4; ++p) acc[q][p] = T(0);
+        for (int p = 0; p < 4; ++p) acc[q][p] = 0.f;
 #pragma unroll 4
     for (int kk = 0; kk < w; ++kk) {
-        T av[4], bv[4];
+        float av[4], bv[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) { av[q] = As[kk * T64 + ty * 4 + q]; bv[q] = Bs[kk * T64 + tx * 4 + q]; }
 #pragma unroll
@@ -836,14 +895,18 @@ __global__ void __launch_bounds__(256) k_update(StepArgs a, const int* __restric
     }
 }
 
-// FP64 update in TS x TS parts of the 64x64 tiles (TS = 32 or 16), for steps whose tiles
-// do not fill the chip: a 64x64 tile takes 65 us of one SM's FP64 pipe, a 32x32 part 16
-// us and a 16x16 part 4 us (plus their shared loads). The same sums in the same order.
-// The next diagonal tile is spread over several blocks then: the last of them to finish
-// (cnt, per front) factors it.
+// FP64 update on the FP64 pipe, in TS x TS parts of the 64x64 tiles. Bound by the pipe (two
+// multiply-adds a cycle and SM): a 64x64 tile takes 65 us of one SM, a 32x32 part 16 us
+// and a 16x16 part 4 us (plus its shared loads, two per product instead of one), so small
+// trailing parts need the small parts to fill the chip, and large ones lose less in their
+// last wave (m = 4001: update 23.2 ms with 64x64 tiles, 18.5 ms with 32x32 parts). The next
+// diagonal tile is spread over several blocks: the last of them to finish (cnt, per front)
+// factors it. Its FP64 work shares the pipe with the SM's other blocks, so while that tile
+// decides the step's time a block asks for more than half of the SM's shared memory.
 template <int TS>
 __global__ void __launch_bounds__(256) k_update_split(StepArgs a, const int* __restrict__ items,
                                                       const int* __restrict__ prefix, PlanDev pd, double* F,
+                                                      double* __restrict__ Linv, const int64_t* __restrict__ inv_off,
                                                       int* __restrict__ cnt, int* err) {
     constexpr int P = T64 / TS, E = TS / 16;        // parts per tile side, entries per thread and side
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -929,9 +992,10 @@ __global__ void __launch_bounds__(256) k_update_split(StepArgs a, const int* __r
             __threadfence();
         }
         __syncthreads();
-        if (last) potrf_tile(s, a.k + 1, pd, F, nullptr, nullptr, err, smraw);
+        if (last) potrf_tile(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
     }
 }
+constexpr size_t kSplitAlone = 120 * 1024;          // leaves room for one block per SM
 template <int TS>
 constexpr size_t split_smem() {
     return 2 * T64 * TS * sizeof(double) > potrf_smem(sizeof(double)) ? 2 * T64 * TS * sizeof(double)
@@ -2023,10 +2087,11 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
 #pragma unroll
         for (int q = 0; q < 8; ++q) lanes[(wid * 8 + q) * 33 + lane] = part[q];
         __syncthreads();
-        const T* v8 = lanes + (tid >> 2) * 33 + 8 * (tid & 3);
-        T v = ((v8[0] + v8[1]) + (v8[2] + v8[3])) + ((v8[4] + v8[5]) + (v8[6] + v8[7]));
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        // the sum tree of the shuffles below: lanes 16, 8, 4, 2, 1 apart
+        const T* v4 = lanes + (tid >> 2) * 33 + (tid & 3);
+        T v = ((v4[0] + v4[16]) + (v4[8] + v4[24])) + ((v4[4] + v4[20]) + (v4[12] + v4[28]));
         v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
         if ((tid & 3) == 0) tb[zq] = zq < w ? zown - v : T(0);
     } else {
 #pragma unroll
@@ -2069,13 +2134,16 @@ inline int blocks_for(int64_t n, int t) { return static_cast<int>((n + t - 1) / 
 
 // ------------------------------------------------------------------ engine
 
-// Steps below these numbers of 64x64 update tiles take 16x16 / 32x32 parts: 16x16 while they
-// run in about two waves of the 152 SMs, 32x32 until whole tiles lose less to their last
-// wave than the parts do to their shared loads.
+// FP64 updates of fewer 64x64 tiles than this take 16x16 parts (about two waves of the 152
+// SMs): m = 500 LP 16.5 ms, with 32x32 parts from 12 tiles on 16.8 ms.
 constexpr int kSplit16Tiles = 24;
-constexpr int kSplit32Tiles = 1200;
-constexpr int kTrOzTiles = 152;
-
+// Fewer tiles than this run one block per SM, so that the next diagonal tile has an SM to
+// itself: m = 1447 3.12 -> 2.89 ms; with 800 here m = 4001 loses 1 %.
+constexpr int kAloneTiles = 300;
+// Panel solves of fewer 64-row units than this take 8 rows a block instead of 16: m = 500
+// LP 17.5 -> 16.0 ms, one warp then has an SM quarter to itself; more blocks than SMs only
+// load the diagonal tile more often.
+constexpr int kTr4Tiles = 76;
 struct KktEngine::Prof {
     cudaStream_t st;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> ev;
@@ -2100,16 +2168,14 @@ static void set_smem_attrs() {
                                      static_cast<int>(kTsSmem)));
     SK_CUDA(cudaFuncSetAttribute(k_potrf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(potrf_smem(sizeof(T)))));
-    SK_CUDA(cudaFuncSetAttribute(k_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(update_smem(sizeof(T)))));
     if (std::is_same<T, double>::value)
         SK_CUDA(cudaFuncSetAttribute(k_update_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kOzSmemU)));
     if (std::is_same<T, double>::value) {
-        SK_CUDA(cudaFuncSetAttribute(k_trsm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kTrSmem)));
+        SK_CUDA(cudaFuncSetAttribute(k_update_split<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(split_smem<16>())));
         SK_CUDA(cudaFuncSetAttribute(k_update_split<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(split_smem<32>())));
+                                     static_cast<int>(kSplitAlone)));
     }
     if (std::is_same<T, double>::value)
         SK_CUDA(cudaFuncSetAttribute(k_trsm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2336,33 +2402,28 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                     k_potrf<T><<<st.nitems, 256, potrf_smem(sizeof(T)), st_>>>(a, items, pdv, F, Linv,
                                                                                inv_off_.ptr, err_.ptr);
                 });
-            if constexpr (std::is_same<T, float>::value) {
-                if (st.trsm_tiles > 0)
-                    run(2, [&] {
-                        k_trsm<<<static_cast<int>(st.trsm_tiles), 256, 2 * T64 * T64 * sizeof(T), st_>>>(
-                            a, items, prefix, pdv, F, Linv, inv_off_.ptr);
-                    });
-            } else {
+            if (st.trsm_tiles > 0)
                 run(2, [&] {
-                    // the panel solve on the tensor cores costs 80 us and more of digit passes and
-                    // launches but its work is small; from kTrOzTiles 64-row tiles on, the FP64
-                    // pipe (3.4 us per 152 x 64 rows) takes longer
-                    const bool oz = emulate64_ && st.trsm_tiles >= kTrOzTiles;
-                    const int tiles = oz ? 0 : static_cast<int>(st.trsm_tiles);
-                    k_trsm_rows<<<4 * (tiles + st.nitems), 256, kTrSmem, st_>>>(a, items, prefix, pdv, F, Linv,
-                                                                                inv_off_.ptr, tiles);
-                    if (oz) {
+                    const int tiles = static_cast<int>(st.trsm_tiles);
+                    if constexpr (std::is_same<T, float>::value) {
+                        k_trsm<<<tiles, 256, 2 * T64 * T64 * sizeof(T), st_>>>(a, items, prefix, pdv, F, Linv,
+                                                                              inv_off_.ptr);
+                    } else if (emulate64_) {   // FP64-accurate panel solve on the tensor cores
                         const int64_t plane = plan_.max_digit_rows * 128, lplane = max_step_items_ * T64 * 128;
-                        k_oz_digits<<<static_cast<int>(st.trsm_tiles), 256, 0, st_>>>(
-                            a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane);
+                        k_oz_digits<<<tiles, 256, 0, st_>>>(a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane);
                         k_oz_linv_digits<<<st.nitems, 256, 0, st_>>>(a, items, pdv, Linv, inv_off_.ptr, ldig_.ptr,
                                                                      lexp_.ptr, lplane);
                         k_trsm_oz<<<static_cast<int>(st.digit_rows / 128) * 2, 256, kOzSmemU, st_>>>(
                             a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane, ldig_.ptr, lexp_.ptr, lplane,
                             err_.ptr);
+                    } else if (tiles < kTr4Tiles) {
+                        k_trsm_rows<4><<<8 * tiles, 128, tr_smem(4), st_>>>(a, items, prefix, pdv, F, Linv,
+                                                                            inv_off_.ptr);
+                    } else {
+                        k_trsm_rows<8><<<4 * tiles, 256, tr_smem(8), st_>>>(a, items, prefix, pdv, F, Linv,
+                                                                            inv_off_.ptr);
                     }
                 });
-            }
             if (st.upd_tiles > 0) {
                 run(3, [&] {
                     bool tc = false;
@@ -2387,21 +2448,17 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                                 dexp_.ptr, plane, oz_cnt_.ptr, err_.ptr);
                         }
                     }
-                    if constexpr (std::is_same<T, double>::value) {
-                        const int tiles = static_cast<int>(st.upd_tiles);
-                        if (!tc && tiles < kSplit16Tiles) {
-                            tc = true;
-                            k_update_split<16><<<tiles * 16, 256, split_smem<16>(), st_>>>(a, items, prefix, pdv, F,
-                                                                                           oz_cnt_.ptr, err_.ptr);
-                        } else if (!tc && tiles < kSplit32Tiles) {
-                            tc = true;
-                            k_update_split<32><<<tiles * 4, 256, split_smem<32>(), st_>>>(a, items, prefix, pdv, F,
-                                                                                          oz_cnt_.ptr, err_.ptr);
-                        }
-                    }
-                    if (!tc)
-                        k_update<T><<<static_cast<int>(st.upd_tiles), 256, update_smem(sizeof(T)), st_>>>(
-                            a, items, prefix, pdv, F, Linv, inv_off_.ptr, err_.ptr);
+                    if (tc) return;
+                    const int tiles = static_cast<int>(st.upd_tiles);
+                    if constexpr (std::is_same<T, float>::value)
+                        k_update<<<tiles, 256, potrf_smem(sizeof(T)), st_>>>(a, items, prefix, pdv, F, Linv,
+                                                                             inv_off_.ptr, err_.ptr);
+                    else if (tiles < kSplit16Tiles)
+                        k_update_split<16><<<tiles * 16, 256, split_smem<16>(), st_>>>(a, items, prefix, pdv, F, Linv,
+                                                                                       inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
+                    else
+                        k_update_split<32><<<tiles * 4, 256, tiles < kAloneTiles ? kSplitAlone : split_smem<32>(),
+                                             st_>>>(a, items, prefix, pdv, F, Linv, inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
                 });
                 if (prof) {
                     for (int it = 0; it < st.nitems; ++it) {
