@@ -545,7 +545,7 @@ def run_ours(args):
                        "k_fwd_tasks<double> + k_bwd_tasks<double> (triangular solves)"),
         solve_roofline(prof, nnz_factor, 4, hbm, src, wl + ", FP32 factor",
                        "k_fwd_tasks<float> + k_bwd_tasks<float> (triangular solves)"),
-        update_roofline(prof64, "k_oz_digits + k_update_oz (FP64-accurate trailing update on the tensor cores, "
+        update_roofline(prof64, "k_update_oz (FP64-accurate trailing update on the tensor cores, "
                         "BF16 digit products; FP64 flops counted)", bf16, src, wl + ", FP64 fronts"),
         update_roofline(prof, "k_update_tc (FP32 trailing update, tcgen05 TF32 x3; FP32 flops counted once)", bf16,
                         src, wl + ", FP32 fronts"),

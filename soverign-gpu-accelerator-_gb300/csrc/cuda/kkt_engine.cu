@@ -1031,7 +1031,7 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 //     a_k = sum_{i=0..6} d_ik 2^(E - 7 - 8 i),   E = floor(log2 max_k |a_k|),
 // with balanced base-256 digits (d_0 in [-256, 256], d_i in [-128, 127] for
 // i >= 1): 56 bits, the row to 2^-56 of its largest entry. Every digit is an
-// integer of at most 8 significant bits, exact in BF16 (k_oz_digits, once per
+// integer of at most 8 significant bits, exact in BF16 (k_panel_oz, once per
 // panel row). C -= A B^T is then the sum over digit pairs (i, j); the pairs of
 // one level L = i + j share the scale 2^(E_a + E_b - 14 - 8 L) and accumulate in
 // one FP32 TMEM accumulator. With K <= 64 each level sum is an integer below
@@ -1040,7 +1040,7 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 // 0..6 (28 pairs; the pairs beyond level 6 weigh below 2^-56 and are left out)
 // are combined in 64-bit integers, hi = levels 0..2 and lo = levels 3..6, folded
 // into u = hi 2^22 + round(lo 2^-10) (below 2^62 in magnitude) and applied with
-// one conversion and one FP64 FMA per entry: C - u 2^(Ea+Eb-52) (GB300's FP64 pipe
+// one FP64 subtraction per entry: C - u 2^(Ea+Eb-52) (GB300's FP64 pipe
 // is the scarce resource of this epilogue).
 // This is the error-free splitting of Ozaki, Ogita, Oishi and Rump (2012) with
 // BF16 digits, exact FP32 tensor-core sums and an integer epilogue; the result
@@ -1058,9 +1058,7 @@ constexpr uint32_t kOzLbo = 128;                       // bytes between K-adjace
 constexpr uint32_t kOzSbo = 512;                       // bytes between 8-row groups (32 bf16 per row and half)
 constexpr size_t kOzA = 128 * 64;                      // 128 rows of one plane and half: 8 KB
 constexpr size_t kOzBu = 32 * 64;                      // 32 rows (update tiles): 2 KB
-constexpr size_t kOzBt = 64 * 64;                      // 64 rows (Linv rows of the panel solve): 4 KB
 constexpr size_t kOzSmemU = kOzDigits * (kOzA + kOzBu) + 64;   // 70 KB: two blocks per SM
-constexpr size_t kOzSmemT = kOzDigits * (kOzA + kOzBt) + 64;   // 84 KB
 constexpr int kOzSpin = 1 << 22;
 // instruction descriptors (kind::f16): D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1),
 // both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28 (M = 128; N = 64 or 32)
@@ -1078,9 +1076,6 @@ __device__ __forceinline__ double oz_pow2(int p) {       // 2^p, 0 below the nor
     if (p < -1022) return 0.0;
     return __longlong_as_double(static_cast<long long>(p + 1023) << 52);
 }
-__device__ __forceinline__ uint32_t oz_bf16(int d) {     // |d| <= 256: exact
-    return __float_as_uint(static_cast<float>(d)) >> 16;
-}
 __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity = 0) {
     uint32_t done = 0;
     for (int spin = 0; spin < kOzSpin && !done; ++spin) {
@@ -1093,37 +1088,76 @@ __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity = 0) {
     return done != 0;
 }
 
-// The 7 balanced base-256 digits of 16 entries v of row q (columns 16 cg .. 16 cg + 15)
-// with row exponent E, as BF16 into the digit planes (layout above).
+// v 2^(55 - E) rounded to an integer (to nearest, ties to even; |v| < 2^(E + 1)), and u 2^e
+// with u rounded to FP64, on the integer pipe: an FP64 instruction takes 64 cycles of its SM
+// quarter here, and these conversions were most of the FP64 work of the digit kernels.
+__device__ __forceinline__ long long oz_fixed(double v, int E) {
+    const long long b = __double_as_longlong(v);
+    const int ex = static_cast<int>(b >> 52) & 0x7ff;
+    const long long m = ((b & 0xfffffffffffffLL) | (ex ? 1LL << 52 : 0LL)) << 3;
+    const int n = min(max(E + 1023 - max(ex, 1), 0), 60);           // |v| = m 2^-n 2^(E - 55)
+    const long long half = (1LL << n) >> 1, odd = n > 0 ? (m >> n) & 1 : 1;
+    const long long f = (m + half - 1 + odd) >> n;
+    return b < 0 ? -f : f;
+}
+__device__ __noinline__ double oz_value_slow(long long u, int e) {   // beyond the normal range
+    return static_cast<double>(u) * oz_pow2(e);
+}
+__device__ __forceinline__ double oz_value(long long u, int e) {
+    const long long a = u < 0 ? -u : u;                              // below 2^62
+    const int n = __clzll(a) - 1;
+    const long long t = a << n;                                      // its highest bit at 62
+    const long long m = (t + 511 + ((t >> 10) & 1)) >> 10;           // 53 bits; 2^53 carries over
+    const int ex = 1084 - n + e;
+    if (a == 0) return 0.0;
+    if (ex < 1 || ex > 2044 || e < -1022) return oz_value_slow(u, e);
+    return __longlong_as_double((static_cast<long long>(ex) << 52) + m + (u & (1LL << 63)));
+}
+// |v| for an integer maximum (a NaN counts as 0), and the exponent E of a row's largest one:
+// at -968 or above, so that 2^(55 - E) stays a normal double (rows whose largest entry is
+// below 2^-967 keep fewer digits; they do not matter next to 1); 0 for a row of zeros.
+__device__ __forceinline__ long long oz_abs(double v) {
+    const long long b = __double_as_longlong(v) & 0x7fffffffffffffffLL;
+    return b <= 0x7ff0000000000000LL ? b : 0;
+}
+__device__ __forceinline__ int oz_exponent(long long mx) {
+    return mx > 0 ? max(static_cast<int>(mx >> 52) - 1023, -968) : 0;
+}
+
+// The 7 balanced base-256 digits of NV entries v of row q (columns NV cg .., NV = 8 or 16)
+// with row exponent E, as BF16 into the digit planes (layout above). With 128 added to each
+// digit below the first they are the bytes of one integer; a byte in the last mantissa bits
+// of 2^23 less 2^23 + 128 is the digit as a float, whose upper half is its BF16.
+template <int NV>
 __device__ __forceinline__ void oz_store_digits(const double* v, int E, int q, int cg, unsigned char* dig,
                                                 int64_t plane) {
-    const double mul = oz_pow2(55 - E);             // |v mul| < 2^56
-    uint32_t pk[kOzDigits][8];                      // 16 BF16 digits per plane, packed in pairs
+    uint32_t pk[kOzDigits][NV / 2];                 // BF16 digits per plane, packed in pairs
 #pragma unroll
-    for (int t = 0; t < 16; t += 2) {
-        int d0[kOzDigits], d1[kOzDigits];
-        long long f0 = llrint(v[t] * mul), f1 = llrint(v[t + 1] * mul);
+    for (int t = 0; t < NV; t += 2) {
+        uint32_t w[2][kOzDigits];                   // the digits as float bits
 #pragma unroll
-        for (int j = kOzDigits - 1; j >= 1; --j) {
-            int l0 = static_cast<int>(f0 & 255), l1 = static_cast<int>(f1 & 255);
-            f0 >>= 8;
-            f1 >>= 8;
-            if (l0 >= 128) { l0 -= 256; f0 += 1; }
-            if (l1 >= 128) { l1 -= 256; f1 += 1; }
-            d0[j] = l0;
-            d1[j] = l1;
+        for (int x = 0; x < 2; ++x) {
+            const long long f = oz_fixed(v[t + x], E) + 0x808080808080LL;
+            const uint32_t lo = static_cast<uint32_t>(f), hi = static_cast<uint32_t>(f >> 32);
+            w[x][0] = __float_as_uint(__uint_as_float(0x4B000000u + ((static_cast<int>(hi) >> 16) + 512)) - 8389120.f);
+#pragma unroll
+            for (int j = 1; j < kOzDigits; ++j) {
+                const uint32_t word = j < 3 ? hi : lo;
+                const int byte = j < 3 ? 2 - j : 6 - j;
+                const uint32_t m = __byte_perm(word, 0x4B000000u, 0x7440u | byte);   // 2^23 + that byte
+                w[x][j] = __float_as_uint(__uint_as_float(m) - 8388736.f);
+            }
         }
-        d0[0] = static_cast<int>(f0);
-        d1[0] = static_cast<int>(f1);
 #pragma unroll
-        for (int j = 0; j < kOzDigits; ++j) pk[j][t >> 1] = oz_bf16(d0[j]) | (oz_bf16(d1[j]) << 16);
+        for (int j = 0; j < kOzDigits; ++j) pk[j][t >> 1] = __byte_perm(w[0][j], w[1][j], 0x7632u);
     }
-    unsigned char* base = dig + (cg >> 1) * (plane >> 1) + static_cast<int64_t>(q >> 3) * kOzSbo + (q & 7) * 16;
+    constexpr int G = 32 / NV;                      // column groups of a K half
+    unsigned char* base = dig + (cg / G) * (plane >> 1) + static_cast<int64_t>(q >> 3) * kOzSbo + (q & 7) * 16;
 #pragma unroll
     for (int j = 0; j < kOzDigits; ++j)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-            *reinterpret_cast<uint4*>(base + j * plane + ((cg & 1) * 2 + h) * kOzLbo) =
+        for (int h = 0; h < NV / 8; ++h)
+            *reinterpret_cast<uint4*>(base + j * plane + ((cg % G) * (NV / 8) + h) * kOzLbo) =
                 make_uint4(pk[j][4 * h], pk[j][4 * h + 1], pk[j][4 * h + 2], pk[j][4 * h + 3]);
 }
 
@@ -1194,6 +1228,7 @@ __device__ __forceinline__ bool oz_products(uint64_t* bar, uint32_t tmem, unsign
 // thread's lane, combined into the integers u with sum = u 2^(Ea+Eb-52):
 // hi 2^(E-30) + lo 2^(E-62) = 2^(E-52) (hi 2^22 + lo 2^-10), one integer below 2^62
 // (lo rounded to 2^(E-53)).
+template <int LevelCols>
 __device__ __forceinline__ void oz_read8(uint32_t taddr, long long* u) {
     uint32_t v[kOzDigits][8];
 #pragma unroll
@@ -1201,7 +1236,7 @@ __device__ __forceinline__ void oz_read8(uint32_t taddr, long long* u) {
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                      : "=r"(v[L][0]), "=r"(v[L][1]), "=r"(v[L][2]), "=r"(v[L][3]), "=r"(v[L][4]),
                        "=r"(v[L][5]), "=r"(v[L][6]), "=r"(v[L][7])
-                     : "r"(taddr + static_cast<uint32_t>(32 * L)));
+                     : "r"(taddr + static_cast<uint32_t>(LevelCols * L)));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -1214,8 +1249,6 @@ __device__ __forceinline__ void oz_read8(uint32_t taddr, long long* u) {
     }
 }
 
-// Digits of the step's trailing panel rows: one block per 64-row tile (the trsm
-// tiles), four threads per row with 16 columns each.
 // Row block bi of block lb in a list where row block bi holds 2 bi + 2 blocks
 // (bi (bi + 1) <= lb < (bi + 1)(bi + 2)); FP32 estimate corrected in integers (the
 // FP64 pipe is kept for the epilogues).
@@ -1224,42 +1257,6 @@ __device__ __forceinline__ int block_row_of(int lb) {
     while ((bi + 1) * (bi + 2) <= lb) ++bi;
     while (bi > 0 && bi * (bi + 1) > lb) --bi;
     return bi;
-}
-
-__global__ void __launch_bounds__(256) k_oz_digits(StepArgs a, const int* __restrict__ items,
-                                                   const int* __restrict__ prefix, PlanDev pd,
-                                                   const double* __restrict__ F, unsigned char* __restrict__ dig,
-                                                   int* __restrict__ dexp, int64_t plane) {
-    __shared__ double smax[4][64];
-    const int i = find_item(prefix + a.tp_off, a.nitems, blockIdx.x);
-    const int s = items[a.item_off + i];
-    if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const int lt = blockIdx.x - prefix[a.tp_off + i];
-    const int N = pd.sn_nrows[s], K = pd.sn_ncols[s], LD = pd.sn_lda[s];
-    const int k0 = a.k * T64;
-    const int w = min(T64, K - k0);
-    const int t0 = k0 + w;
-    const int r = threadIdx.x & 63, cg = threadIdx.x >> 6;
-    const int row = t0 + lt * T64 + r;
-    const bool rin = row < N;
-    const double* Fs = F + pd.F_off[s];
-    double v[16];
-    double mx = 0.0;
-#pragma unroll
-    for (int t = 0; t < 16; ++t) {
-        const int k = cg * 16 + t;
-        v[t] = (rin && k < w) ? Fs[row + static_cast<int64_t>(k0 + k) * LD] : 0.0;
-        mx = fmax(mx, fabs(v[t]));
-    }
-    smax[cg][r] = mx;
-    __syncthreads();
-    mx = fmax(fmax(smax[0][r], smax[1][r]), fmax(smax[2][r], smax[3][r]));
-    // E is held at -968 or above so that 2^(55 - E) stays a normal double (rows whose
-    // largest entry is below 2^-967 keep fewer digits; they do not matter next to 1)
-    const int E = mx > 0.0 ? max(ilogb(mx), -968) : 0;
-    const int q = prefix[a.dr_off + i] + lt * T64 + r;
-    oz_store_digits(v, E, q, cg, dig, plane);
-    if (cg == 0) dexp[q] = E;
 }
 
 // C(128 x 32) -= A B^T from the digit planes: two blocks per 128-row x 64-column
@@ -1342,14 +1339,13 @@ __global__ void __launch_bounds__(256, 2) k_update_oz(StepArgs a, const int* __r
 #pragma unroll
         for (int c8 = 0; c8 < 2; ++c8) {
             long long u[8];
-            oz_read8(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
+            oz_read8<32>(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int j = 8 * c8 + q, col = ch + j;
-                // one conversion and one FP64 FMA on the slow FP64 pipe per entry
                 if (rok && col < ncb && r0 + row >= c0 + col)
                     Fs[(r0 + row) + static_cast<int64_t>(c0 + col) * LD] =
-                        fma(-static_cast<double>(u[q]), oz_pow2(ea + dexp[qb + col] - 52), cv[j]);
+                        cv[j] - oz_value(u[q], ea + dexp[qb + col] - 52);
             }
         }
     }
@@ -1381,109 +1377,149 @@ __global__ void __launch_bounds__(256, 2) k_update_oz(StepArgs a, const int* __r
 }
 
 // ---- FP64 panel solve on the tensor cores (the same digit products) ----------
-// X = B Linv^T for the step's panel rows below the diagonal tile (B = their current
-// values, Linv = the inverse of the factored diagonal tile): k_oz_digits writes the
-// digits of B before the solve, k_oz_linv_digits those of the 64 rows of Linv of
-// every item of the step (one block per item, rows i * 64 .. in a buffer of its own),
-// and k_trsm_oz forms X = u 2^(Ea+Eb-52) with the MMAs of k_update_oz and no C
-// operand: two blocks per 128 panel rows, each taking 32 of the 64 Linv rows (N = 32).
-__global__ void __launch_bounds__(256) k_oz_linv_digits(StepArgs a, const int* __restrict__ items, PlanDev pd,
-                                                        const double* __restrict__ Linv,
-                                                        const int64_t* __restrict__ inv_off,
-                                                        unsigned char* __restrict__ dig, int* __restrict__ dexp,
-                                                        int64_t plane) {
-    __shared__ double smax[4][64];
-    const int i = blockIdx.x;
-    const int s = items[a.item_off + i];
-    if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const double* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;   // column-major 64 x 64
-    const int r = threadIdx.x & 63, cg = threadIdx.x >> 6;
-    double v[16];
-    double mx = 0.0;
-#pragma unroll
-    for (int t = 0; t < 16; ++t) {
-        v[t] = Li[r + (cg * 16 + t) * T64];
-        mx = fmax(mx, fabs(v[t]));
-    }
-    smax[cg][r] = mx;
-    __syncthreads();
-    mx = fmax(fmax(smax[0][r], smax[1][r]), fmax(smax[2][r], smax[3][r]));
-    const int E = mx > 0.0 ? max(ilogb(mx), -968) : 0;
-    const int q = i * T64 + r;
-    oz_store_digits(v, E, q, cg, dig, plane);
-    if (cg == 0) dexp[q] = E;
-}
+// X = B Linv^T for 128 of the step's panel rows below the diagonal tile (B = their current
+// values, Linv = the inverse of the factored diagonal tile), and the digits of X for the
+// update. One block forms the digits of its rows of B and of the 64 rows of Linv in shared
+// memory, runs the 28 digit pairs of both K halves as MMAs with M = 128, N = 64 (level L in
+// TMEM columns 64 L ..), and takes X = u 2^(Ea+Eb-52) from the accumulators through the
+// registers to the front and to the digit planes. Bound by the integer work of the digits
+// and of the 64-bit sums (half of its 48,000 cycles; the MMAs take 7,700). As separate
+// kernels (digits of B, of Linv, MMAs, digits of X, each through memory) a step took 33 us
+// at m = 4740 and 112 us at 54,000 rows; now 25 and 95 us. Every wait is bounded: on a
+// time-out the block records err[2], waits once more for what it issued and frees its TMEM.
+constexpr size_t kOzPanelA = 128 * 128, kOzPanelB = 64 * 128;       // one plane, both K halves
+constexpr size_t kOzPanelSmem = kOzDigits * (kOzPanelA + kOzPanelB) + 8 * 128 * sizeof(long long) +
+                                (128 + 64) * sizeof(int) + 64;
 
-__global__ void __launch_bounds__(256, 2) k_trsm_oz(StepArgs a, const int* __restrict__ items,
-                                                    const int* __restrict__ prefix, PlanDev pd, double* F,
-                                                    const unsigned char* __restrict__ dig,
-                                                    const int* __restrict__ dexp, int64_t plane,
-                                                    const unsigned char* __restrict__ ldig,
-                                                    const int* __restrict__ lexp, int64_t lplane, int* err) {
+__global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __restrict__ items,
+                                                     const int* __restrict__ prefix, PlanDev pd, double* F,
+                                                     const double* __restrict__ Linv,
+                                                     const int64_t* __restrict__ inv_off,
+                                                     unsigned char* __restrict__ dig, int* __restrict__ dexp,
+                                                     int64_t plane, int* err) {
     extern __shared__ __align__(1024) unsigned char smraw[];
     unsigned char* As = smraw;
-    unsigned char* Bs = smraw + kOzDigits * kOzA;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(Bs + kOzDigits * kOzBu);   // [0] planes loaded, [1] MMAs done
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
-    int* fail = reinterpret_cast<int*>(bar + 3);
-    const int unit = blockIdx.x >> 1, hc = blockIdx.x & 1;   // 128 panel rows, 32 of the 64 columns
-    const int i = find_item(prefix + a.dr_off, a.nitems, unit * 128);
+    unsigned char* Bs = As + kOzDigits * kOzPanelA;
+    long long* rmax = reinterpret_cast<long long*>(Bs + kOzDigits * kOzPanelB);   // [4][128], then [8][64]
+    int* ea = reinterpret_cast<int*>(rmax + 8 * 128);
+    int* eb = ea + 128;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(eb + 64);                         // MMAs done
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
+    int* fail = reinterpret_cast<int*>(tslot + 1);
+    const int i = find_item(prefix + a.dr_off, a.nitems, blockIdx.x * 128);
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const int blk = unit - prefix[a.dr_off + i] / 128;
+    const int blk = blockIdx.x - prefix[a.dr_off + i] / 128;
     const int N = pd.sn_nrows[s], K = pd.sn_ncols[s], LD = pd.sn_lda[s];
     const int k0 = a.k * T64;
     const int w = min(T64, K - k0);
     const int r0 = k0 + w + blk * 128;
-    if (r0 >= N || hc * 32 >= w) return;              // a padded block of the digit rows, or no columns
+    if (r0 >= N) return;                               // a padded block of the digit rows
     const int nra = min(128, N - r0);
-    const int qa = prefix[a.dr_off + i] + blk * 128, qb = i * T64 + hc * 32;
+    const int qa = prefix[a.dr_off + i] + blk * 128;
     double* Fs = F + pd.F_off[s];
+    const double* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;   // column-major 64 x 64
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    if (tid == 0) {                                    // the copies first, then TMEM allocation
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(bar)));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(bar + 1)));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *fail = 0;
-        oz_copy_half(0, smem_addr(bar), As, Bs, dig, plane, qa, ldig, lplane, qb);
-    }
     if (wid == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" :: "r"(smem_addr(tslot)));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_addr(tslot)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(bar)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        *fail = 0;
+    }
+    // B: row `brow`, columns 16 bg ..; Linv: row `lrow`, columns 8 lg ..
+    const int brow = tid & 127, bg = tid >> 7, lrow = tid & 63, lg = tid >> 6;
+    double v[16];
+    {
+        double l[8];
+        long long ml = 0, mb = 0;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) l[t] = Li[lrow + (lg * 8 + t) * T64];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const int k = 16 * bg + t;
+            v[t] = brow < nra && k < w ? Fs[(r0 + brow) + static_cast<int64_t>(k0 + k) * LD] : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) ml = max(ml, oz_abs(l[t]));
+#pragma unroll
+        for (int t = 0; t < 16; ++t) mb = max(mb, oz_abs(v[t]));
+        rmax[bg * 128 + brow] = mb;
+        rmax[512 + lg * 64 + lrow] = ml;
+        __syncthreads();
+        mb = max(max(rmax[brow], rmax[128 + brow]), max(rmax[256 + brow], rmax[384 + brow]));
+#pragma unroll
+        for (int g = 0; g < 8; ++g) ml = max(ml, rmax[512 + g * 64 + lrow]);
+        const int eB = oz_exponent(mb), eL = oz_exponent(ml);
+        if (bg == 0) ea[brow] = eB;
+        if (lg == 0) eb[lrow] = eL;
+        oz_store_digits<8>(l, eL, lrow, lg, Bs, static_cast<int64_t>(kOzPanelB));
+        oz_store_digits<16>(v, eB, brow, bg, As, static_cast<int64_t>(kOzPanelA));
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
-    if (tid == 0 && !oz_products(bar, tmem, As, Bs, dig, plane, qa, ldig, lplane, qb)) {
-        *fail = 1;
-        atomicExch(err + 2, 1);
+    if (tid == 0) {
+        const uint32_t sa = smem_addr(As), sb = smem_addr(Bs), b0 = smem_addr(bar);
+        for (int L = 0; L < kOzDigits; ++L)
+            for (int da = 0; da <= L; ++da)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {       // K half kk / 2, 16 columns each
+                    const uint32_t acc = (da > 0 || kk > 0) ? 1u : 0u;
+                    const uint32_t ko = (kk & 1) * 2 * kOzLbo;
+                    const uint64_t adesc = oz_sdesc(sa + da * static_cast<uint32_t>(kOzPanelA) +
+                                                    (kk >> 1) * static_cast<uint32_t>(kOzPanelA / 2) + ko);
+                    const uint64_t bdesc = oz_sdesc(sb + (L - da) * static_cast<uint32_t>(kOzPanelB) +
+                                                    (kk >> 1) * static_cast<uint32_t>(kOzPanelB / 2) + ko);
+                    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                                 :: "r"(tmem + static_cast<uint32_t>(64 * L)), "l"(adesc), "l"(bdesc),
+                                    "r"(kOzIdesc64), "r"(acc));
+                }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                     :: "r"(b0) : "memory");
+        if (!oz_wait(b0)) {
+            oz_wait(b0);                               // a second bounded wait before TMEM is freed
+            *fail = 1;
+            atomicExch(err + 2, 1);
+        }
     }
-    const int row = 32 * (wid & 3) + lane, ch = 16 * (wid >> 2);
-    const bool rok = row < nra;
-    const int ea = rok ? dexp[qa + row] : 0;
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (*fail == 0) {
+    const bool ok = *fail == 0;
+    // X: row `row` (TMEM lane), columns ch ..
+    const int row = 32 * (wid & 3) + lane, ch = 16 * (wid >> 2);
+    long long mx = 0;
+    if (ok) {
+        const int er = ea[row];
 #pragma unroll
         for (int c8 = 0; c8 < 2; ++c8) {
             long long u[8];
-            oz_read8(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
+            oz_read8<64>(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                const int col = hc * 32 + ch + 8 * c8 + q;
-                if (rok && col < w)
-                    Fs[(r0 + row) + static_cast<int64_t>(k0 + col) * LD] =
-                        static_cast<double>(u[q]) * oz_pow2(ea + lexp[i * T64 + col] - 52);
+                const int j = 8 * c8 + q, col = ch + j;
+                v[j] = row < nra && col < w ? oz_value(u[q], er + eb[col] - 52) : 0.0;
+                if (row < nra && col < w) Fs[(r0 + row) + static_cast<int64_t>(k0 + col) * LD] = v[j];
+                mx = max(mx, oz_abs(v[j]));
             }
         }
+        rmax[(wid >> 2) * 128 + row] = mx;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (wid == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" :: "r"(tmem));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" :: "r"(tmem));
     }
+    if (!ok) return;
+    const int E = oz_exponent(max(max(rmax[row], rmax[128 + row]), max(rmax[256 + row], rmax[384 + row])));
+    oz_store_digits<16>(v, E, qa + row, ch / 16, dig, plane);
+    if (ch == 0) dexp[qa + row] = E;
 }
 
 // ---- FP32 trailing update on the tensor cores from pre-split panels -----------
@@ -2178,8 +2214,8 @@ static void set_smem_attrs() {
                                      static_cast<int>(kSplitAlone)));
     }
     if (std::is_same<T, double>::value)
-        SK_CUDA(cudaFuncSetAttribute(k_trsm_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kOzSmemU)));
+        SK_CUDA(cudaFuncSetAttribute(k_panel_oz, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(kOzPanelSmem)));
 }
 
 KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_t stream)
@@ -2409,13 +2445,9 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                         k_trsm<<<tiles, 256, 2 * T64 * T64 * sizeof(T), st_>>>(a, items, prefix, pdv, F, Linv,
                                                                               inv_off_.ptr);
                     } else if (emulate64_) {   // FP64-accurate panel solve on the tensor cores
-                        const int64_t plane = plan_.max_digit_rows * 128, lplane = max_step_items_ * T64 * 128;
-                        k_oz_digits<<<tiles, 256, 0, st_>>>(a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane);
-                        k_oz_linv_digits<<<st.nitems, 256, 0, st_>>>(a, items, pdv, Linv, inv_off_.ptr, ldig_.ptr,
-                                                                     lexp_.ptr, lplane);
-                        k_trsm_oz<<<static_cast<int>(st.digit_rows / 128) * 2, 256, kOzSmemU, st_>>>(
-                            a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane, ldig_.ptr, lexp_.ptr, lplane,
-                            err_.ptr);
+                        k_panel_oz<<<static_cast<int>(st.digit_rows / 128), 512, kOzPanelSmem, st_>>>(
+                            a, items, prefix, pdv, F, Linv, inv_off_.ptr, dig_.ptr, dexp_.ptr,
+                            plan_.max_digit_rows * 128, err_.ptr);
                     } else if (tiles < kTr4Tiles) {
                         k_trsm_rows<4><<<8 * tiles, 128, tr_smem(4), st_>>>(a, items, prefix, pdv, F, Linv,
                                                                             inv_off_.ptr);
@@ -2441,8 +2473,6 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                         if (emulate64_) {
                             tc = true;
                             const int64_t plane = plan_.max_digit_rows * 128;
-                            k_oz_digits<<<static_cast<int>(st.trsm_tiles), 256, 0, st_>>>(
-                                a, items, prefix, pdv, F, dig_.ptr, dexp_.ptr, plane);
                             k_update_oz<<<static_cast<int>(st.upd3_blocks) * 2, 256, kOzSmemU, st_>>>(
                                 a, items, prefix, pdv, F, Linv, inv_off_.ptr, dig_.ptr,
                                 dexp_.ptr, plane, oz_cnt_.ptr, err_.ptr);
@@ -2550,18 +2580,12 @@ void KktEngine::ensure_fronts(bool fp32) {
 
 void KktEngine::ensure_digits() {
     if (dig_.ptr || plan_.max_digit_rows <= 0) return;
-    max_step_items_ = 1;
-    for (const auto& st : plan_.steps) max_step_items_ = std::max(max_step_items_, static_cast<int64_t>(st.nitems));
     dig_arena_.reset();
     reserve(dig_arena_, dig_, static_cast<size_t>(kOzDigits) * static_cast<size_t>(plan_.max_digit_rows) * 128);
     reserve(dig_arena_, dexp_, static_cast<size_t>(plan_.max_digit_rows));
-    reserve(dig_arena_, ldig_, static_cast<size_t>(kOzDigits) * static_cast<size_t>(max_step_items_) * T64 * 128);
-    reserve(dig_arena_, lexp_, static_cast<size_t>(max_step_items_) * T64);
     dig_arena_.commit();
     bind(dig_arena_, dig_);
     bind(dig_arena_, dexp_);
-    bind(dig_arena_, ldig_);
-    bind(dig_arena_, lexp_);
 }
 
 // The step lists for a factorisation of the LPs of this precision's mask: the
