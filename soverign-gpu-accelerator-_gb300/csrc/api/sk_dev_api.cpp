@@ -934,9 +934,9 @@ int sk_gnn_loss_grad(sk_gnn* g, sk_gnn_batch* bt, double* loss, float* grad) {
     if (!g || !bt) return SK_ERR_INVALID;
     if (!bt->has_targets) { api::set_error("batch has no targets"); return SK_ERR_INVALID; }
     try {
-        const double l = g->net->forward(bt->lp, g->st, nullptr, nullptr, nullptr, bt->tlx.ptr, bt->tls.ptr, bt->ty.ptr);
-        if (loss) *loss = l;
+        g->net->forward(bt->lp, g->st, nullptr, nullptr, nullptr, bt->tlx.ptr, bt->tls.ptr, bt->ty.ptr);
         g->net->backward(bt->lp, g->st, grad);
+        if (loss) *loss = g->net->loss();
         SK_CUDA(cudaStreamSynchronize(g->st));
         return SK_OK;
     } catch (...) {
@@ -949,10 +949,11 @@ int sk_gnn_train_step(sk_gnn* g, sk_gnn_batch* bt, float lr, double* loss) {
     if (!g || !bt || !(lr > 0.f)) return SK_ERR_INVALID;
     if (!bt->has_targets) { api::set_error("batch has no targets"); return SK_ERR_INVALID; }
     try {
-        const double l = g->net->forward(bt->lp, g->st, nullptr, nullptr, nullptr, bt->tlx.ptr, bt->tls.ptr, bt->ty.ptr);
-        if (loss) *loss = l;
+        g->net->forward(bt->lp, g->st, nullptr, nullptr, nullptr, bt->tlx.ptr, bt->tls.ptr, bt->ty.ptr);
         g->net->backward(bt->lp, g->st, nullptr);
         g->net->adam_step(g->st, lr);
+        const double l = g->net->loss();       // the gradient and the step still run
+        if (loss) *loss = l;
         return SK_OK;
     } catch (...) {
         return api::status_of_current_exception();

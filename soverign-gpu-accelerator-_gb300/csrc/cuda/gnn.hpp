@@ -33,10 +33,12 @@ public:
     void get_params(float* out) const;
     void set_params(const float* in);
     // Forward on the LP batch; writes log x, log s (n) and y (m) predictions into
-    // out_logx, out_logs, out_y (device, scaled space). If targets are given,
-    // returns the loss and keeps activations for backward().
-    double forward(const DeviceLP& lp, cudaStream_t st, double* out_logx, double* out_logs, double* out_y,
-                   const double* t_logx = nullptr, const double* t_logs = nullptr, const double* t_y = nullptr);
+    // out_logx, out_logs, out_y (device, scaled space; may be null). If targets are
+    // given, also forms the loss (see loss()) and keeps activations for backward().
+    void forward(const DeviceLP& lp, cudaStream_t st, double* out_logx, double* out_logs, double* out_y,
+                 const double* t_logx = nullptr, const double* t_logs = nullptr, const double* t_y = nullptr);
+    // Loss of the last forward with targets; waits for that forward alone.
+    double loss() const;
     // Gradient of the last forward's loss into grad_ (FP32); optional copy-out.
     void backward(const DeviceLP& lp, cudaStream_t st, float* grad_host = nullptr);
     void adam_step(cudaStream_t st, float lr);
@@ -59,7 +61,8 @@ private:
     float *dc_ = nullptr, *dr_ = nullptr, *dm_ = nullptr, *dt_ = nullptr;  // gradient work
     float *inv_deg_r_ = nullptr, *inv_deg_c_ = nullptr;
     double* loss_ = nullptr;
-    const double *t_logx_ = nullptr, *t_logs_ = nullptr, *t_y_ = nullptr;
+    double* loss_host_ = nullptr;     // pinned
+    cudaEvent_t loss_ready_ = nullptr;
 };
 
 }  // namespace dev
