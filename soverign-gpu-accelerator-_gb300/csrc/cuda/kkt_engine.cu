@@ -1823,8 +1823,11 @@ __global__ void k_fwd_gather(int n, const int* __restrict__ dst, const int* __re
 // values themselves. One trip through the L2 then links two blocks, where a flag took
 // four (values, fence, flag; flag, then values). Every wait is bounded: on time-out the
 // task sets *err and returns (the host checks *err and reports an error).
-// Chain of one front, per 64-row block: FP32 forward 2.2 -> 1.4 us, backward 3.2 -> 1.1
-// us; FP64 forward 4.4 -> 2.8 us, backward 8.2 -> 3.2 us (m = 1447 .. 4740).
+// Chain of one front, per 64-row block: FP32 forward 2.2 -> 1.0 us, backward 3.2 -> 1.0
+// us; FP64 forward 4.4 -> 2.6 us, backward 8.2 -> 3.2 us (m = 1447 .. 4740). In a batch a
+// task starts behind its chain and is bound by how fast it takes in the blocks that are
+// there: with two of them in registers the FP32 solves of 40 LPs take 206 -> 110 us forward
+// and 133 -> 93 us backward.
 
 constexpr int kSpinLimit = 1 << 24;
 constexpr int kReadyBlocks = 16;   // column blocks taken per pass once they are there
@@ -1969,13 +1972,23 @@ __global__ void __launch_bounds__(256, 1) k_fwd_tasks(const int2* __restrict__ t
         const int e = j + got;
 #pragma unroll
         for (int c = 0; c < 16; ++c) acc += pre[c] * zs[cg * 16 + c];
-        if (rv) {
-            for (int jj = j + 1; jj < e; ++jj) {
+        if (rv && got > 1) {              // behind: the next block's L is loaded while one is summed
+            auto load = [&](T* l, int jj) {
                 const T* Lc = Fs + row + static_cast<int64_t>(jj * T64 + cg * 16) * LD;
-                const T* zz = zs + (jj - j) * T64 + cg * 16;
 #pragma unroll
                 for (int c = 0; c < 16; ++c)
-                    if (jj * T64 + cg * 16 + c < K) acc += Lc[static_cast<int64_t>(c) * LD] * zz[c];
+                    l[c] = jj * T64 + cg * 16 + c < K ? Lc[static_cast<int64_t>(c) * LD] : T(0);
+            };
+            T cur[16];
+            load(cur, j + 1);
+            for (int jj = j + 1; jj < e; ++jj) {
+                T nxt[16];
+                if (jj + 1 < e) load(nxt, jj + 1);
+                const T* zz = zs + (jj - j) * T64 + cg * 16;
+#pragma unroll
+                for (int c = 0; c < 16; ++c) acc += cur[c] * zz[c];
+#pragma unroll
+                for (int c = 0; c < 16; ++c) cur[c] = nxt[c];
             }
         }
         j = e;
@@ -2105,15 +2118,39 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
 #pragma unroll
             for (int q = 0; q < 8; ++q) part[q] += pre[h * 8 + q] * xr;
         }
-        for (int blk = j - 1; blk > e; --blk) {
-            const T* xx = xb + (j - blk) * T64;
-            for (int rr = lane; rr < T64; rr += 32) {
-                const int r = blk * T64 + rr;
-                if (r >= K) break;
-                const T xr = xx[rr];
+        if constexpr (kWide) {            // a second block of L in registers would not leave room for two
+            for (int blk = j - 1; blk > e; --blk) {                  // blocks on an SM (77 -> 93 us at m = 1447)
+                const T* xx = xb + (j - blk) * T64;
+                for (int rr = lane; rr < T64; rr += 32) {
+                    const T xr = xx[rr];
 #pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    if (c0 + q < K) part[q] += Fs[r + static_cast<int64_t>(c0 + q) * LD] * xr;
+                    for (int q = 0; q < 8; ++q)
+                        if (c0 + q < K) part[q] += Fs[blk * T64 + rr + static_cast<int64_t>(c0 + q) * LD] * xr;
+                }
+            }
+        } else if (got > 1) {             // behind: the next block's L is loaded while one is summed
+            auto load = [&](T* l, int blk) {         // a block before the last: all its rows are there
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        l[h * 8 + q] = c0 + q < K ? Fs[blk * T64 + lane + 32 * h + static_cast<int64_t>(c0 + q) * LD]
+                                                  : T(0);
+            };
+            T cur[16];
+            load(cur, j - 1);
+            for (int blk = j - 1; blk > e; --blk) {
+                T nxt[16];
+                if (blk - 1 > e) load(nxt, blk - 1);
+                const T* xx = xb + (j - blk) * T64;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const T xr = xx[lane + 32 * h];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) part[q] += cur[h * 8 + q] * xr;
+                }
+#pragma unroll
+                for (int q = 0; q < 16; ++q) cur[q] = nxt[q];
             }
         }
         j = e;
