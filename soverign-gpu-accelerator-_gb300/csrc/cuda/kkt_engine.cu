@@ -77,6 +77,17 @@ __device__ __forceinline__ int find_item(const int* prefix, int n, int b) {
     return lo;
 }
 
+// Item i and tile of update unit u in a grid of nitems + prefix[nitems] units: the first
+// tile of every item comes first, because the block that finishes it goes on to factor the
+// next diagonal tile, which takes longer than a whole tile of update; in the list's order
+// the last front's factorisation was the kernel's tail. Result -1: nothing to do.
+__device__ __forceinline__ int update_unit(const int* prefix, int nitems, int u, int& i) {
+    const bool first = u < nitems;
+    i = first ? u : find_item(prefix, nitems, u - nitems);
+    const int lt = first ? 0 : u - nitems - prefix[i];
+    return first ? (prefix[i + 1] > prefix[i] ? 0 : -1) : (lt > 0 ? lt : -1);
+}
+
 __device__ __forceinline__ void tri_index(int lt, int& ti, int& tj) {
     int t = static_cast<int>((sqrtf(8.0f * static_cast<float>(lt) + 1.0f) - 1.0f) * 0.5f);
     while ((t + 1) * (t + 2) / 2 <= lt) ++t;
@@ -823,10 +834,11 @@ __global__ void __launch_bounds__(256) k_update(StepArgs a, const int* __restric
     extern __shared__ __align__(16) unsigned char smraw[];
     float* As = reinterpret_cast<float*>(smraw);     // [kk][r]
     float* Bs = As + T64 * T64;                  // [kk][c]
-    const int i = find_item(prefix + a.up_off, a.nitems, blockIdx.x);
+    int i;
+    const int lt = update_unit(prefix + a.up_off, a.nitems, blockIdx.x, i);
+    if (lt < 0) return;
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const int lt = blockIdx.x - prefix[a.up_off + i];
     int ti, tj;
     tri_index(lt, ti, tj);
     const int N = pd.sn_nrows[s], K = pd.sn_ncols[s];
@@ -913,11 +925,12 @@ __global__ void __launch_bounds__(256) k_update_split(StepArgs a, const int* __r
     __shared__ int last;
     double* As = reinterpret_cast<double*>(smraw);  // [kk][r]
     double* Bs = As + T64 * TS;                      // [kk][c]
-    const int tile = blockIdx.x / (P * P), part = blockIdx.x % (P * P);
-    const int i = find_item(prefix + a.up_off, a.nitems, tile);
+    const int part = blockIdx.x % (P * P);
+    int i;
+    const int lt = update_unit(prefix + a.up_off, a.nitems, blockIdx.x / (P * P), i);
+    if (lt < 0) return;
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const int lt = tile - prefix[a.up_off + i];
     int ti, tj;
     tri_index(lt, ti, tj);
     const int N = pd.sn_nrows[s], K = pd.sn_ncols[s];
@@ -1283,11 +1296,12 @@ __global__ void __launch_bounds__(256, 2) k_update_oz(StepArgs a, const int* __r
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
     int* fail = reinterpret_cast<int*>(bar + 3);
     int* last = fail + 1;
-    const int unit = blockIdx.x >> 1, hc = blockIdx.x & 1;
-    const int i = find_item(prefix + a.up3_off, a.nitems, unit);
+    const int hc = blockIdx.x & 1;
+    int i;
+    const int lb = update_unit(prefix + a.up3_off, a.nitems, blockIdx.x >> 1, i);
+    if (lb < 0) return;
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const int lb = unit - prefix[a.up3_off + i];
     const int bi = block_row_of(lb);
     const int bj = lb - bi * (bi + 1);
     const int N = pd.sn_nrows[s], K = pd.sn_ncols[s], LD = pd.sn_lda[s];
@@ -1593,10 +1607,11 @@ __global__ void __launch_bounds__(256, 2) k_update_tcs(StepArgs a, const int* __
     uint64_t* bar = reinterpret_cast<uint64_t*>(Bl + kTsB);   // [0] parts loaded, [1] MMAs done
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
     int* fail = reinterpret_cast<int*>(bar + 3);
-    const int i = find_item(prefix + a.up3_off, a.nitems, blockIdx.x);
+    int i;
+    const int lb = update_unit(prefix + a.up3_off, a.nitems, blockIdx.x, i);
+    if (lb < 0) return;
     const int s = items[a.item_off + i];
     if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const int lb = blockIdx.x - prefix[a.up3_off + i];
     int bi = block_row_of(lb);
     const int bj = lb - bi * (bi + 1);
     const int N = pd.sn_nrows[s], K = pd.sn_ncols[s], LD = pd.sn_lda[s];
@@ -2502,7 +2517,7 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                             const int64_t plane = plan_.max_digit_rows * 256;
                             k_tc_split<<<static_cast<int>(st.trsm_tiles), 256, 0, st_>>>(
                                 a, items, prefix, pdv, F, dig_.ptr, plane);
-                            k_update_tcs<<<static_cast<int>(st.upd3_blocks), 256, kTsSmem, st_>>>(
+                            k_update_tcs<<<st.nitems + static_cast<int>(st.upd3_blocks), 256, kTsSmem, st_>>>(
                                 a, items, prefix, pdv, F, Linv, inv_off_.ptr, dig_.ptr, plane,
                                 err_.ptr);
                         }
@@ -2510,7 +2525,7 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                         if (emulate64_) {
                             tc = true;
                             const int64_t plane = plan_.max_digit_rows * 128;
-                            k_update_oz<<<static_cast<int>(st.upd3_blocks) * 2, 256, kOzSmemU, st_>>>(
+                            k_update_oz<<<(st.nitems + static_cast<int>(st.upd3_blocks)) * 2, 256, kOzSmemU, st_>>>(
                                 a, items, prefix, pdv, F, Linv, inv_off_.ptr, dig_.ptr,
                                 dexp_.ptr, plane, oz_cnt_.ptr, err_.ptr);
                         }
@@ -2518,13 +2533,13 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                     if (tc) return;
                     const int tiles = static_cast<int>(st.upd_tiles);
                     if constexpr (std::is_same<T, float>::value)
-                        k_update<<<tiles, 256, potrf_smem(sizeof(T)), st_>>>(a, items, prefix, pdv, F, Linv,
+                        k_update<<<st.nitems + tiles, 256, potrf_smem(sizeof(T)), st_>>>(a, items, prefix, pdv, F, Linv,
                                                                              inv_off_.ptr, err_.ptr);
                     else if (tiles < kSplit16Tiles)
-                        k_update_split<16><<<tiles * 16, 256, split_smem<16>(), st_>>>(a, items, prefix, pdv, F, Linv,
+                        k_update_split<16><<<(st.nitems + tiles) * 16, 256, split_smem<16>(), st_>>>(a, items, prefix, pdv, F, Linv,
                                                                                        inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
                     else
-                        k_update_split<32><<<tiles * 4, 256, tiles < kAloneTiles ? kSplitAlone : split_smem<32>(),
+                        k_update_split<32><<<(st.nitems + tiles) * 4, 256, tiles < kAloneTiles ? kSplitAlone : split_smem<32>(),
                                              st_>>>(a, items, prefix, pdv, F, Linv, inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
                 });
                 if (prof) {
