@@ -301,6 +301,9 @@ __device__ __forceinline__ void helper_sync() { asm volatile("bar.sync 1, 192;" 
 __device__ __forceinline__ void inverse_arrive() { asm volatile("bar.arrive 2, 224;" ::: "memory"); }
 __device__ __forceinline__ void inverse_wait() { asm volatile("bar.sync 2, 224;" ::: "memory"); }
 
+// The 256 threads of a diagonal tile (the update's block has one more warp).
+__device__ __forceinline__ void tile_sync() { asm volatile("bar.sync 3, 256;" ::: "memory"); }
+
 __device__ __noinline__ void report_pivot(int s, const PlanDev& pd, int* err) {
     if ((threadIdx.x & 31) != 0) return;
     if (atomicCAS(err, 0, 1) == 0) err[1] = s;
@@ -627,7 +630,7 @@ __device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, T* F, T* _
         A[r * LDS + c] = x;
     }
     if (tid < 12) next[tid] = 0;
-    __syncthreads();
+    tile_sync();
     const int ht = (wid < 4 ? wid - 1 : wid - 2) * 32 + lane;   // helpers: warps 1-3 and 5-7
     // 32 entries of [0, n) at a time, to whichever helper is free
     auto share = [&](int* counter, int n, auto&& work) {
@@ -664,17 +667,17 @@ __device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, T* F, T* _
                 });
             }
         }
-        __syncthreads();
+        tile_sync();
         if (nt == 0) break;
         panel_rows(A, rdiag, c0, nt);
-        __syncthreads();
+        tile_sync();
         if (tid < kPBTri) trail_entry(A, c0, tid);   // the next diagonal block
-        __syncthreads();
+        tile_sync();
     }
     inverse_block(A, X, rdiag, T64 - kPB, tid);
-    __syncthreads();
+    tile_sync();
     for (int e = tid; e < (T64 - kPB) * kPB / kCols<T>; e += 256) inverse_rows(X, T64 - kPB, e);
-    __syncthreads();
+    tile_sync();
     T* Li = Linv + inv_off[s] + static_cast<int64_t>(kstep) * T64 * T64;
 #pragma unroll 4
     for (int it = 0; it < 16; ++it) {
@@ -1070,13 +1073,11 @@ constexpr int kOzDigits = 7;
 constexpr uint32_t kOzLbo = 128;                       // bytes between K-adjacent core matrices
 constexpr uint32_t kOzSbo = 512;                       // bytes between 8-row groups (32 bf16 per row and half)
 constexpr size_t kOzA = 128 * 64;                      // 128 rows of one plane and half: 8 KB
-constexpr size_t kOzBu = 32 * 64;                      // 32 rows (update tiles): 2 KB
-constexpr size_t kOzSmemU = kOzDigits * (kOzA + kOzBu) + 64;   // 70 KB: two blocks per SM
+constexpr size_t kOzB = 64 * 64;                       // 64 rows: 4 KB
 constexpr int kOzSpin = 1 << 22;
 // instruction descriptors (kind::f16): D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1),
-// both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28 (M = 128; N = 64 or 32)
-constexpr uint32_t kOzIdesc64 = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-constexpr uint32_t kOzIdesc32 = (1u << 4) | (1u << 7) | (1u << 10) | ((32u >> 3) << 17) | ((128u >> 4) << 24);
+// both K-major, N >> 3 at bits 17-22 (added per product), M >> 4 at bits 24-28 (M = 128)
+constexpr uint32_t kOzIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
 
 __device__ __forceinline__ uint64_t oz_sdesc(uint32_t saddr) {
     uint64_t d = static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
@@ -1089,14 +1090,15 @@ __device__ __forceinline__ double oz_pow2(int p) {       // 2^p, 0 below the nor
     if (p < -1022) return 0.0;
     return __longlong_as_double(static_cast<long long>(p + 1023) << 52);
 }
-__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity = 0) {
+__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity = 0, int limit = kOzSpin,
+                                        int polls = 4096) {
     uint32_t done = 0;
-    for (int spin = 0; spin < kOzSpin && !done; ++spin) {
+    for (int spin = 0; spin < limit && !done; ++spin) {
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         // back-to-back polls first: a copy or an MMA batch of one tile completes within
         // microseconds, and a sleep per poll adds its own latency to every tile
-        if (!done && spin >= 4096) __nanosleep(32);
+        if (!done && spin >= polls) __nanosleep(polls ? 32 : 1000);
     }
     return done != 0;
 }
@@ -1113,18 +1115,26 @@ __device__ __forceinline__ long long oz_fixed(double v, int E) {
     const long long f = (m + half - 1 + odd) >> n;
     return b < 0 ? -f : f;
 }
-__device__ __noinline__ double oz_value_slow(long long u, int e) {   // beyond the normal range
-    return static_cast<double>(u) * oz_pow2(e);
+__device__ __noinline__ double oz_value_any(long long u, int e) {
+    return u == 0 ? 0.0 : static_cast<double>(u) * oz_pow2(e);
 }
-__device__ __forceinline__ double oz_value(long long u, int e) {
-    const long long a = u < 0 ? -u : u;                              // below 2^62
-    const int n = __clzll(a) - 1;
-    const long long t = a << n;                                      // its highest bit at 62
-    const long long m = (t + 511 + ((t >> 10) & 1)) >> 10;           // 53 bits; 2^53 carries over
-    const int ex = 1084 - n + e;
-    if (a == 0) return 0.0;
-    if (ex < 1 || ex > 2044 || e < -1022) return oz_value_slow(u, e);
-    return __longlong_as_double((static_cast<long long>(ex) << 52) + m + (u & (1LL << 63)));
+// e for which every u below 2^62 gives zero or a normal number
+__device__ __forceinline__ bool oz_plain(int e) { return e >= -1000 && e <= 900; }
+// The same for |u| of 2^32 or more (else `small` is set and the result is nothing) and plain e, without a
+// branch.
+__device__ __forceinline__ double oz_value(long long u, int e, bool& small) {
+    const int s = static_cast<int>(u >> 32) >> 31;
+    const unsigned long long a = (u ^ s) - s;                        // |u|, below 2^62
+    const unsigned ah = static_cast<unsigned>(a >> 32);
+    small |= ah == 0;
+    const int n = __clz(static_cast<int>(ah)) - 1;
+    const unsigned tl = static_cast<unsigned>(a) << n;               // its highest bit at 62
+    const unsigned th = __funnelshift_l(static_cast<unsigned>(a), ah, n);
+    const unsigned long long t = (static_cast<unsigned long long>(th) << 32) | tl;
+    // 53 bits, ties to even; 2^53 carries over into the exponent
+    const unsigned long long m = (t + 511 + ((tl >> 10) & 1)) >> 10;
+    const unsigned hi = static_cast<unsigned>(m >> 32) + (static_cast<unsigned>(1084 - n + e) << 20);
+    return __hiloint2double(static_cast<int>(hi | (static_cast<unsigned>(s) & 0x80000000u)), static_cast<int>(m));
 }
 // |v| for an integer maximum (a NaN counts as 0), and the exponent E of a row's largest one:
 // at -968 or above, so that 2^(55 - E) stays a normal double (rows whose largest entry is
@@ -1143,7 +1153,7 @@ __device__ __forceinline__ int oz_exponent(long long mx) {
 // of 2^23 less 2^23 + 128 is the digit as a float, whose upper half is its BF16.
 template <int NV>
 __device__ __forceinline__ void oz_store_digits(const double* v, int E, int q, int cg, unsigned char* dig,
-                                                int64_t plane) {
+                                                int64_t plane, int64_t half) {
     uint32_t pk[kOzDigits][NV / 2];                 // BF16 digits per plane, packed in pairs
 #pragma unroll
     for (int t = 0; t < NV; t += 2) {
@@ -1165,7 +1175,7 @@ __device__ __forceinline__ void oz_store_digits(const double* v, int E, int q, i
         for (int j = 0; j < kOzDigits; ++j) pk[j][t >> 1] = __byte_perm(w[0][j], w[1][j], 0x7632u);
     }
     constexpr int G = 32 / NV;                      // column groups of a K half
-    unsigned char* base = dig + (cg / G) * (plane >> 1) + static_cast<int64_t>(q >> 3) * kOzSbo + (q & 7) * 16;
+    unsigned char* base = dig + (cg / G) * half + static_cast<int64_t>(q >> 3) * kOzSbo + (q & 7) * 16;
 #pragma unroll
     for (int j = 0; j < kOzDigits; ++j)
 #pragma unroll
@@ -1174,92 +1184,108 @@ __device__ __forceinline__ void oz_store_digits(const double* v, int E, int q, i
                 make_uint4(pk[j][4 * h], pk[j][4 * h + 1], pk[j][4 * h + 2], pk[j][4 * h + 3]);
 }
 
-// Thread 0 of a digit-product block: start the bulk copies of K half h of the 7
-// planes of A (128 rows from row qa of adig) and B (32 rows from row qb of bdig)
-// into As / Bs, completing on the mbarrier at b0.
-__device__ __forceinline__ void oz_copy_half(int h, uint32_t b0, unsigned char* As, unsigned char* Bs,
-                                             const unsigned char* adig, int64_t aplane, int qa,
-                                             const unsigned char* bdig, int64_t bplane, int qb) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                 :: "r"(b0), "r"(static_cast<uint32_t>(kOzDigits * (kOzA + kOzBu))) : "memory");
-    for (int j = 0; j < kOzDigits; ++j) {
-        const unsigned char* ga = adig + j * aplane + h * (aplane >> 1) + static_cast<int64_t>(qa >> 3) * kOzSbo;
-        const unsigned char* gb = bdig + j * bplane + h * (bplane >> 1) + static_cast<int64_t>(qb >> 3) * kOzSbo;
+// Lanes 0..6 of a warp: bulk copies of K half h of the 7 planes of `rows` digit rows from
+// row q on into dst (plane after plane), completing on the mbarrier at bar.
+__device__ __forceinline__ void oz_copy_rows(int h, uint32_t bar, unsigned char* dst, const unsigned char* dig,
+                                             int64_t plane, int q, int rows) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t bytes = static_cast<uint32_t>(rows) * 64;
+    if (lane == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                     :: "r"(bar), "r"(kOzDigits * bytes) : "memory");
+    __syncwarp();
+    if (lane < kOzDigits) {
+        const unsigned char* src = dig + lane * plane + h * (plane >> 1) + static_cast<int64_t>(q >> 3) * kOzSbo;
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     :: "r"(smem_addr(As + j * kOzA)), "l"(ga), "r"(static_cast<uint32_t>(kOzA)), "r"(b0)
-                     : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     :: "r"(smem_addr(Bs + j * kOzBu)), "l"(gb), "r"(static_cast<uint32_t>(kOzBu)), "r"(b0)
-                     : "memory");
+                     :: "r"(smem_addr(dst + lane * bytes)), "l"(src), "r"(bytes), "r"(bar) : "memory");
     }
+    __syncwarp();
 }
 
-// Thread 0, after oz_copy_half(0, ...): for each K half wait for its planes, issue
-// the 28 digit pairs x 2 K-steps of MMAs (M=128, N=32, K=16; level L into TMEM
-// columns 32L..32L+31), wait for them to finish with the buffer and start the next
-// half's copies. bar[0] counts the copies (phase h), bar[1] the MMA batches. Every
-// wait is bounded; on a time-out it waits once more for what is in flight and
-// returns false.
-__device__ __forceinline__ bool oz_products(uint64_t* bar, uint32_t tmem, unsigned char* As, unsigned char* Bs,
-                                            const unsigned char* adig, int64_t aplane, int qa,
-                                            const unsigned char* bdig, int64_t bplane, int qb) {
-    const uint32_t b0 = smem_addr(bar), b1 = smem_addr(bar + 1);
-    const uint32_t sa = smem_addr(As), sb = smem_addr(Bs);
-    for (int h = 0; h < 2; ++h) {
-        if (!oz_wait(b0, h)) {
-            oz_wait(b0, h);                            // copies still in flight: a second bounded wait
-            return false;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int L = 0; L < kOzDigits; ++L) {
-            for (int da = 0; da <= L; ++da) {
-                const int db = L - da;
+// One thread: the products of levels l0..l1-1 (at most four) over K half h, whose planes are
+// at sa and sb; level L into TMEM columns 64 L .. 64 L + 63. Plane da of A meets the planes
+// db of B with da + db in l0..l1-1; these follow one another in shared memory and their
+// levels in TMEM, so that they are one product with N = 64 per plane: 20 instead of 56 MMAs
+// a half, and A is read once for up to four planes (pair by pair a tile took 7,700 cycles,
+// twice what its multiplications need).
+__device__ __forceinline__ void oz_products(uint32_t tmem, uint32_t sa, uint32_t sb, int h, int l0, int l1) {
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) {
-                    const uint32_t acc = (h > 0 || da > 0 || ks > 0) ? 1u : 0u;
-                    const uint64_t adesc = oz_sdesc(sa + da * static_cast<uint32_t>(kOzA) + ks * 2 * kOzLbo);
-                    const uint64_t bdesc = oz_sdesc(sb + db * static_cast<uint32_t>(kOzBu) + ks * 2 * kOzLbo);
-                    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                                 :: "r"(tmem + static_cast<uint32_t>(32 * L)), "l"(adesc), "l"(bdesc),
-                                    "r"(kOzIdesc32), "r"(acc));
-                }
-            }
+    for (int ks = 0; ks < 2; ++ks)
+        for (int da = 0; da < l1; ++da) {
+            const int L = max(l0, da);
+            const uint32_t acc = (h > 0 || da > 0 || ks > 0) ? 1u : 0u;
+            const uint32_t idesc = kOzIdesc | (static_cast<uint32_t>((l1 - L) * 64) >> 3 << 17);
+            const uint64_t adesc = oz_sdesc(sa + da * static_cast<uint32_t>(kOzA) + ks * 2 * kOzLbo);
+            const uint64_t bdesc = oz_sdesc(sb + (L - da) * static_cast<uint32_t>(kOzB) + ks * 2 * kOzLbo);
+            asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                         :: "r"(tmem + static_cast<uint32_t>(64 * L)), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                     :: "r"(b1) : "memory");
-        if (!oz_wait(b1, h)) {
-            oz_wait(b1, h);                            // a second bounded wait before TMEM is freed
-            return false;
-        }
-        if (h == 0) oz_copy_half(1, b0, As, Bs, adig, aplane, qa, bdig, bplane, qb);
-    }
-    return true;
+}
+__device__ __forceinline__ void oz_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
 }
 
-// Row accumulators of 8 TMEM columns (from column c) of the 7 levels for this
-// thread's lane, combined into the integers u with sum = u 2^(Ea+Eb-52):
-// hi 2^(E-30) + lo 2^(E-62) = 2^(E-52) (hi 2^22 + lo 2^-10), one integer below 2^62
-// (lo rounded to 2^(E-53)).
-template <int LevelCols>
+// One entry's sum from its level accumulators, in units of 2^(Ea+Eb-52): hi 2^(E-30) from the
+// levels 0..2 plus lo 2^(E-62) from 3..6, lo rounded to 2^(E-53) (hi below 2^39.2, lo below
+// 2^47.2). The multiply-adds are 32-bit as long as the levels' bounds (4, 4, 5, 6, 7, 8 and
+// 9 * 2^20) allow it: every integer instruction takes two cycles here, a conversion eight.
+__device__ __forceinline__ long long mad_wide(int x, int y, long long z) {
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(x), "r"(y), "l"(z));
+    return d;
+}
+__device__ __forceinline__ int oz_int(uint32_t v) {           // in program order with sub_ordered
+    int i;
+    asm volatile("cvt.rni.s32.f32 %0, %1;" : "=r"(i) : "f"(__uint_as_float(v)));
+    return i;
+}
+__device__ __forceinline__ double sub_ordered(double x, double y) {
+    double d;
+    asm volatile("sub.rn.f64 %0, %1, %2;" : "=d"(d) : "d"(x), "d"(y));
+    return d;
+}
+// |v| <= 2^22: the last bits of 1.5 * 2^23 + v, less 0x4B400000
+__device__ __forceinline__ uint32_t oz_int_biased(uint32_t v) {
+    return __float_as_uint(__uint_as_float(v) + 12582912.f);
+}
+__device__ __forceinline__ long long oz_lower(const uint32_t* v, int stride) {
+    const int b = oz_int(v[0]) * 256 + oz_int(v[stride]);
+    const long long c = mad_wide(oz_int(v[2 * stride]), 256, static_cast<long long>(oz_int(v[3 * stride]) + 512));
+    return mad_wide(b, 65536, c) >> 10;
+}
+__device__ __forceinline__ long long oz_sum(const uint32_t* v, int stride, long long lower) {
+    const uint32_t a = oz_int_biased(v[stride]) * 256u + (static_cast<uint32_t>(oz_int(v[2 * stride])) - 0x40000000u);
+    const long long u = mad_wide(static_cast<int>(a), 4194304, lower);
+    const uint32_t hi = static_cast<uint32_t>(u >> 32) + (oz_int_biased(v[0]) << 6) - 0xD0000000u;
+    return (static_cast<long long>(hi) << 32) | static_cast<uint32_t>(u);
+}
+
+__device__ __forceinline__ void tmem_load8(uint32_t* v, uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_load16(uint32_t* v, uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                   "=r"(v[15])
+                 : "r"(addr));
+}
+
+// The integers u (sum = u 2^(Ea+Eb-52), below 2^62) of 8 columns from TMEM column c on, for
+// this thread's lane.
 __device__ __forceinline__ void oz_read8(uint32_t taddr, long long* u) {
-    uint32_t v[kOzDigits][8];
+    uint32_t v[kOzDigits * 8];
 #pragma unroll
-    for (int L = 0; L < kOzDigits; ++L)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(v[L][0]), "=r"(v[L][1]), "=r"(v[L][2]), "=r"(v[L][3]), "=r"(v[L][4]),
-                       "=r"(v[L][5]), "=r"(v[L][6]), "=r"(v[L][7])
-                     : "r"(taddr + static_cast<uint32_t>(LevelCols * L)));
+    for (int L = 0; L < kOzDigits; ++L) tmem_load8(v + 8 * L, taddr + static_cast<uint32_t>(64 * L));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        long long lv[kOzDigits];
-#pragma unroll
-        for (int L = 0; L < kOzDigits; ++L) lv[L] = __float2int_rn(__uint_as_float(v[L][q]));
-        const long long hi = lv[0] * 65536LL + lv[1] * 256LL + lv[2];   // |hi| < 2^39.2
-        const long long lo = lv[3] * 16777216LL + lv[4] * 65536LL + lv[5] * 256LL + lv[6];  // < 2^47.2
-        u[q] = hi * 4194304LL + ((lo + 512) >> 10);
-    }
+    for (int q = 0; q < 8; ++q) u[q] = oz_sum(v + q, 8, oz_lower(v + 24 + q, 8));
 }
 
 // Row block bi of block lb in a list where row block bi holds 2 bi + 2 blocks
@@ -1272,121 +1298,265 @@ __device__ __forceinline__ int block_row_of(int lb) {
     return bi;
 }
 
-// C(128 x 32) -= A B^T from the digit planes: two blocks per 128-row x 64-column
-// block of the trailing lower part (row block bi holds column blocks 0..2bi+1), each
-// taking 32 of its columns, so that two blocks fit an SM (70 KB of shared memory, 256
-// TMEM columns, at most 128 registers). Thread 0 streams the two K halves of the 14
-// planes through one buffer with bulk copies and issues 28 digit pairs x 2 K-steps of
-// MMAs (M=128, N=32, K=16) per half; level L accumulates in TMEM columns 32L..32L+31.
-// Every thread loads its 16 C values meanwhile, then reads its row's 7 accumulators
-// and applies them. The diagonal tile of the next step lies in both blocks of the
-// first 128 x 64 block: the one of the two that finishes second (a per-front counter,
-// no waiting) factors it. Every wait is bounded: on a time-out the block records
-// err[2], waits once more for what it issued, frees its TMEM and leaves C untouched.
-__global__ void __launch_bounds__(256, 2) k_update_oz(StepArgs a, const int* __restrict__ items,
+// C(128 x 64) -= A B^T from the digit planes, over the 128 x 64 blocks of the trailing lower
+// part (row block bi holds column blocks 0..2bi+1). One block per SM stays for the whole step
+// and takes runs of tiles from a counter, long ones first, so that the next tiles of a run find
+// their 128 rows of A in shared memory (7 planes, 112 KB) and load only 64 rows of B (56 KB,
+// two buffers). Warp 9 fetches tiles and copies, warp 8 issues the MMAs, warps 0..7 take the
+// sums from TMEM (448 columns) to C, 32 columns a thread. The lower levels are multiplied
+// first: their accumulators are free for the next tile as soon as they are in registers, while
+// the upper levels' products run. Bound by the epilogue: of an SM quarter 5,500 cycles of
+// integer instructions a tile, 4,100 of FP64 subtractions, 3,700 of conversions, so these are
+// kept apart in neighbouring groups of columns and have no branch between them. The block
+// with a front's first tile factors the next diagonal tile and waits for it without polling.
+// As 128 x 32 tiles of blocks that copied, multiplied and subtracted in turn, two on an SM, a
+// tile's half took 29,000 cycles: mean step at m = 4740 85 -> 78 us (there the diagonal tile's
+// 64 us are the limit), of 40 LPs (54,000 rows) 161 -> 115 us. Waits are bounded: on a
+// time-out the block records err[2], takes no further tile, waits once more for what it issued
+// and frees its TMEM.
+constexpr size_t kOzSmemU = kOzDigits * (2 * kOzA + 4 * kOzB) + 512;
+
+struct OzTile {
+    int s, r0, c0, qa, qb, N, LD;             // s < 0: no more tiles
+    bool first, fresh;                        // factors the next diagonal tile; its rows of A are copied
+    int64_t F;
+};
+
+__global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __restrict__ items,
                                                       const int* __restrict__ prefix, PlanDev pd, double* F,
                                                       double* __restrict__ Linv, const int64_t* __restrict__ inv_off,
                                                       const unsigned char* __restrict__ dig,
-                                                      const int* __restrict__ dexp, int64_t plane, int* cnt,
-                                                      int* err) {
+                                                      const int* __restrict__ dexp, int64_t plane,
+                                                      int* __restrict__ next, int* err) {
     extern __shared__ __align__(1024) unsigned char smraw[];
-    unsigned char* As = smraw;
-    unsigned char* Bs = smraw + kOzDigits * kOzA;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(Bs + kOzDigits * kOzBu);   // [0] planes loaded, [1] MMAs done
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
-    int* fail = reinterpret_cast<int*>(bar + 3);
-    int* last = fail + 1;
-    const int hc = blockIdx.x & 1;
-    int i;
-    const int lb = update_unit(prefix + a.up3_off, a.nitems, blockIdx.x >> 1, i);
-    if (lb < 0) return;
-    const int s = items[a.item_off + i];
-    if (!pd.lp_on[pd.sn_lp[s]]) return;
-    const int bi = block_row_of(lb);
-    const int bj = lb - bi * (bi + 1);
-    const int N = pd.sn_nrows[s], K = pd.sn_ncols[s], LD = pd.sn_lda[s];
-    const int k0 = a.k * T64;
-    const int w = min(T64, K - k0);
-    const int t0 = k0 + w;
-    const int r0 = t0 + bi * 128, c0 = t0 + bj * T64 + hc * 32;
-    if (c0 >= N) return;                              // the whole block: columns past the front
-    const int nra = min(128, N - r0), ncb = min(32, N - c0);
-    const int qa = prefix[a.dr_off + i] + bi * 128, qb = prefix[a.dr_off + i] + bj * T64 + hc * 32;
-    double* Fs = F + pd.F_off[s];
+    constexpr int kA = kOzDigits * static_cast<int>(kOzA), kB = kOzDigits * static_cast<int>(kOzB);   // a K half
+    unsigned char* As = smraw;                        // [half][plane]
+    unsigned char* Bs = smraw + 2 * kA;               // [buffer][half][plane]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(Bs + 4 * kB);
+    OzTile* slot = reinterpret_cast<OzTile*>(bars + 16);              // [4]
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(slot + 4);
+    volatile int* fail = reinterpret_cast<volatile int*>(tslot + 1);
+    int* go = reinterpret_cast<int*>(tslot + 2);
+    // A's halves, B's buffers and halves, the slots' descriptions; a tile's lower sums done, an
+    // even and an odd tile's upper ones (the copying warp may look after the next is done too),
+    // their accumulators free again, the diagonal tile factored
+    const uint32_t bA = smem_addr(bars), bB = bA + 16, bTile = bA + 48, bLo = bA + 80, bHi = bA + 88,
+                   bLoFree = bA + 104, bHiFree = bA + 112, bTri = bA + 120;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    // thread 0 starts the first half's copies; TMEM allocation and every thread's C
-    // loads then overlap them
+    constexpr int kLimit = 2 * kOzSpin;   // waits for other warps, whose own waits end before
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(bar)));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(bar + 1)));
+        for (int b = 0; b < 16; ++b)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bA + 8 * b), "r"(b < 13 ? 1 : 8));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *fail = 0;
-        oz_copy_half(0, smem_addr(bar), As, Bs, dig, plane, qa, dig, plane, qb);
     }
-    if (wid == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" :: "r"(smem_addr(tslot)));
+    if (wid == 8) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_addr(tslot)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    // this thread's row (TMEM lane) and 16 columns, and its C values
-    const int row = 32 * (wid & 3) + lane, ch = 16 * (wid >> 2);
-    const bool rok = row < nra;
-    double cv[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const int col = ch + j;
-        const bool in = rok && col < ncb && r0 + row >= c0 + col;
-        cv[j] = in ? Fs[(r0 + row) + static_cast<int64_t>(c0 + col) * LD] : 0.0;
-    }
-    const int ea = rok ? dexp[qa + row] : 0;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
-    if (tid == 0 && !oz_products(bar, tmem, As, Bs, dig, plane, qa, dig, plane, qb)) {
-        *fail = 1;
-        atomicExch(err + 2, 1);
-    }
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const bool ok = *fail == 0;
-    if (ok) {
+    // a copy or an MMA batch that does not complete
+    auto wait_async = [&](uint32_t bar, int n) {      // the n-th phase of a barrier
+        bool done = *fail == 0 && oz_wait(bar, n & 1);
+        done = __all_sync(0xffffffffu, done);
+        if (!done && lane == 0) {
+            *fail = 1;
+            atomicExch(err + 2, 1);
+        }
+        return done;
+    };
+    if (wid == 9) {
+        const int* up = prefix + a.up3_off;
+        const int grid = gridDim.x, total = a.nitems + up[a.nitems];
+        int u = blockIdx.x, end = u + 1, last = grid;
+        int item = -1, rows = -1;                     // whose rows are in As
+        int tri = 0;
+        bool first = false;                           // the tile before was a first one
+        for (int t = 0;; ++t) {
+            // the diagonal tile needs the SM's issue slots: no polling beside it
+            if (first) oz_wait(bTri, tri++ & 1, kLimit, 0);
+            OzTile w;
+            w.s = -1;
+            while (u < total && w.s < 0) {
+                if (u >= end) {
+                    // runs of half the block's share of what is left; first tiles one by one
+                    const int run = last < a.nitems ? 1 : max(1, min(8, (total - last) / (2 * grid)));
+                    if (lane == 0) u = grid + atomicAdd(next, run);
+                    u = __shfl_sync(0xffffffffu, u, 0);
+                    end = min(u + run, total);
+                    last = u;
+                    continue;
+                }
+                int i;
+                const int lb = update_unit(up, a.nitems, u++, i);
+                if (lb < 0) continue;
+                const int s = items[a.item_off + i];
+                if (!pd.lp_on[pd.sn_lp[s]]) continue;
+                const int bi = block_row_of(lb), bj = lb - bi * (bi + 1);
+                const int K = pd.sn_ncols[s], t0 = min(K, (a.k + 1) * T64);
+                w.N = pd.sn_nrows[s];
+                w.r0 = t0 + bi * 128;
+                w.c0 = t0 + bj * T64;
+                if (w.c0 >= w.N) continue;            // a column block past the front
+                w.s = s;
+                w.LD = pd.sn_lda[s];
+                w.F = pd.F_off[s];
+                w.qa = prefix[a.dr_off + i] + bi * 128;
+                w.qb = prefix[a.dr_off + i] + bj * T64;
+                w.first = lb == 0 && t0 < K;
+                w.fresh = first || i != item || bi != rows;
+                item = i;
+                rows = bi;
+            }
+            const int buf = t & 1;
+            bool ok = w.s >= 0;
+            if (ok && t > 1) ok = wait_async(bHi + 8 * buf, (t - 2) >> 1);              // B's buffer is no longer read
+            if (ok)
+                for (int h = 0; h < 2; ++h)
+                    oz_copy_rows(h, bB + 16 * buf + 8 * h, Bs + (2 * buf + h) * kB, dig, plane, w.qb, 64);
+            if (ok && w.fresh) {
+                if (t > 0) ok = wait_async(bHi + 8 * (buf ^ 1), (t - 1) >> 1);                // nor are A's rows
+                if (ok)
+                    for (int h = 0; h < 2; ++h)
+                        oz_copy_rows(h, bA + 8 * h, As + h * kA, dig, plane, w.qa, 128);
+            }
+            if (!ok) w.s = -1;
+            first = w.first;
+            if (lane == 0) {
+                slot[t & 3] = w;
+                mbar_arrive(bTile + 8 * (t & 3));
+            }
+            if (!ok) break;
+        }
+        if (*fail != 0)                               // what may still be in flight
+            for (int b = 0; b < 6; ++b) oz_wait(bA + 8 * b, 0, 1 << 12);
+    } else if (wid == 8) {
+        const uint32_t sa = smem_addr(As);
+        int na = 0;
+        for (int t = 0;; ++t) {
+            if (!oz_wait(bTile + 8 * (t & 3), (t >> 2) & 1, kLimit, t > 0 && slot[(t - 1) & 3].first ? 0 : 4096) ||
+                slot[t & 3].s < 0) break;
+            na += slot[t & 3].fresh;
+            if (t > 0) oz_wait(bLoFree, (t - 1) & 1, kLimit);
+            const uint32_t sb = smem_addr(Bs) + (t & 1) * 2 * kB;
+            bool ok = true;
+            for (int h = 0; h < 2; ++h) {
+                ok = ok && wait_async(bA + 8 * h, na - 1) && wait_async(bB + 16 * (t & 1) + 8 * h, t >> 1);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (ok && lane == 0) oz_products(tmem, sa + h * kA, sb + h * kB, h, 3, kOzDigits);
+            }
+            if (lane == 0) oz_commit(bLo);
+            if (t > 0) oz_wait(bHiFree, (t - 1) & 1, kLimit);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (lane == 0) {
+                if (ok)
+                    for (int h = 0; h < 2; ++h) oz_products(tmem, sa + h * kA, sb + h * kB, h, 0, 3);
+                oz_commit(bHi + 8 * (t & 1));
+            }
+            __syncwarp();
+        }
+    } else {
+        const int row = 32 * (wid & 3) + lane, ch = 32 * (wid >> 2);      // this thread's row and columns
+        const uint32_t tl = tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch);
+        for (int t = 0;; ++t) {
+            if (!oz_wait(bTile + 8 * (t & 3), (t >> 2) & 1, kLimit)) break;
+            const OzTile w = slot[t & 3];
+            if (w.s < 0) break;
+            const int r = w.r0 + row;
+            // columns c0 + ch + j of row r for j < nj
+            const int nj = r < w.N ? min(32, min(w.N, r + 1) - (w.c0 + ch)) : 0;
+            double* C = F + w.F + r + static_cast<int64_t>(w.c0 + ch) * w.LD;
+            const int ea = dexp[w.qa + row] - 52, eb = dexp[w.qb + ch + lane];
+            const bool plain = oz_plain(ea + __reduce_min_sync(0xffffffffu, eb)) &&
+                               oz_plain(ea + __reduce_max_sync(0xffffffffu, eb));
+            double cv[2][16];
+            auto load_c = [&](int h) {
 #pragma unroll
-        for (int c8 = 0; c8 < 2; ++c8) {
-            long long u[8];
-            oz_read8<32>(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
+                for (int j = 0; j < 16; ++j)
+                    cv[h][j] = 16 * h + j < nj ? C[static_cast<int64_t>(16 * h + j) * w.LD] : 0.0;
+            };
+            load_c(0);
+            oz_wait(bLo, t & 1, kLimit);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            long long lo[32];
+            {
+                uint32_t v[4 * 32];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int j = 8 * c8 + q, col = ch + j;
-                if (rok && col < ncb && r0 + row >= c0 + col)
-                    Fs[(r0 + row) + static_cast<int64_t>(c0 + col) * LD] =
-                        cv[j] - oz_value(u[q], ea + dexp[qb + col] - 52);
+                for (int L = 0; L < 4; ++L) {
+                    tmem_load16(v + 32 * L, tl + static_cast<uint32_t>(64 * (3 + L)));
+                    tmem_load16(v + 32 * L + 16, tl + static_cast<uint32_t>(64 * (3 + L) + 16));
+                }
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bLoFree);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) lo[j] = oz_lower(v + j, 32);
+            }
+            oz_wait(bHi + 8 * (t & 1), (t >> 1) & 1, kLimit);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int last = *fail == 0 ? nj : 0;
+            // Eight columns at a time; their subtractions are issued between the integer work of
+            // the next eight, which they would otherwise wait for and hold up.
+            double x[2][8];
+            auto store = [&](int g) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (8 * g + q < last) C[static_cast<int64_t>(8 * g + q) * w.LD] = x[g & 1][q];
+            };
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                uint32_t v[3 * 8];
+#pragma unroll
+                for (int L = 0; L < 3; ++L) tmem_load8(v + 8 * L, tl + static_cast<uint32_t>(64 * L + 8 * g));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (g == 3) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bHiFree);
+                }
+                long long u[8];
+                bool any = !plain;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    u[q] = oz_sum(v + q, 8, lo[8 * g + q]);
+                    if (g > 0)
+                        x[(g - 1) & 1][q] = sub_ordered(cv[(g - 1) >> 1][(8 * (g - 1) + q) & 15], x[(g - 1) & 1][q]);
+                    x[g & 1][q] = oz_value(u[q], ea + __shfl_sync(0xffffffffu, eb, 8 * g + q), any);
+                }
+                if (g > 0) store(g - 1);
+                if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int e = ea + __shfl_sync(0xffffffffu, eb, 8 * g + q);
+                        if (any) x[g & 1][q] = oz_value_any(u[q], e);
+                    }
+                }
+                if (g == 0) load_c(1);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) x[1][q] = cv[1][8 + q] - x[1][q];
+            store(3);
+            if (w.first) {
+                __threadfence();                      // C, before the other warps read it
+                tile_sync();
+                if (tid == 0) *go = *fail == 0;
+                tile_sync();
+                if (*go) potrf_tile(w.s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before A is copied there again
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bTri);
             }
         }
     }
-    __threadfence();                                   // this block's C writes, before the counter below
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (wid == 0) {
+    if (wid == 8) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" :: "r"(tmem));
-    }
-    if (!ok) return;
-    // the next diagonal tile spans both blocks of the first 128 x 64 block: the second
-    // of the two to get here factors it (when the front ends within the first 32
-    // columns the first block is alone) and resets the counter for the next step
-    if (lb == 0 && t0 < K) {
-        if (tid == 0) {
-            if (t0 + 32 >= N) {
-                *last = 1;
-            } else {
-                const int prev = atomicAdd(cnt + s, 1);
-                *last = prev == 1;
-                if (prev == 1) atomicExch(cnt + s, 0);
-                __threadfence();
-            }
-        }
-        __syncthreads();
-        if (*last) potrf_tile(s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" :: "r"(tmem));
     }
 }
 
@@ -1397,12 +1567,11 @@ __global__ void __launch_bounds__(256, 2) k_update_oz(StepArgs a, const int* __r
 // memory, runs the 28 digit pairs of both K halves as MMAs with M = 128, N = 64 (level L in
 // TMEM columns 64 L ..), and takes X = u 2^(Ea+Eb-52) from the accumulators through the
 // registers to the front and to the digit planes. Bound by the integer work of the digits
-// and of the 64-bit sums (half of its 48,000 cycles; the MMAs take 7,700). As separate
+// and of the 64-bit sums (half of its 45,000 cycles; the MMAs take 4,000). As separate
 // kernels (digits of B, of Linv, MMAs, digits of X, each through memory) a step took 33 us
-// at m = 4740 and 112 us at 54,000 rows; now 25 and 95 us. Every wait is bounded: on a
+// at m = 4740 and 112 us at 54,000 rows; now 24 and 90 us. Every wait is bounded: on a
 // time-out the block records err[2], waits once more for what it issued and frees its TMEM.
-constexpr size_t kOzPanelA = 128 * 128, kOzPanelB = 64 * 128;       // one plane, both K halves
-constexpr size_t kOzPanelSmem = kOzDigits * (kOzPanelA + kOzPanelB) + 8 * 128 * sizeof(long long) +
+constexpr size_t kOzPanelSmem = 2 * kOzDigits * (kOzA + kOzB) + 8 * 128 * sizeof(long long) +
                                 (128 + 64) * sizeof(int) + 64;
 
 __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __restrict__ items,
@@ -1410,11 +1579,12 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
                                                      const double* __restrict__ Linv,
                                                      const int64_t* __restrict__ inv_off,
                                                      unsigned char* __restrict__ dig, int* __restrict__ dexp,
-                                                     int64_t plane, int* err) {
+                                                     int64_t plane, int* __restrict__ next, int* err) {
     extern __shared__ __align__(1024) unsigned char smraw[];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;        // the update's tile counter
     unsigned char* As = smraw;
-    unsigned char* Bs = As + kOzDigits * kOzPanelA;
-    long long* rmax = reinterpret_cast<long long*>(Bs + kOzDigits * kOzPanelB);   // [4][128], then [8][64]
+    unsigned char* Bs = As + 2 * kOzDigits * kOzA;                               // both [half][plane]
+    long long* rmax = reinterpret_cast<long long*>(Bs + 2 * kOzDigits * kOzB);   // [4][128], then [8][64]
     int* ea = reinterpret_cast<int*>(rmax + 8 * 128);
     int* eb = ea + 128;
     uint64_t* bar = reinterpret_cast<uint64_t*>(eb + 64);                         // MMAs done
@@ -1469,8 +1639,8 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
         const int eB = oz_exponent(mb), eL = oz_exponent(ml);
         if (bg == 0) ea[brow] = eB;
         if (lg == 0) eb[lrow] = eL;
-        oz_store_digits<8>(l, eL, lrow, lg, Bs, static_cast<int64_t>(kOzPanelB));
-        oz_store_digits<16>(v, eB, brow, bg, As, static_cast<int64_t>(kOzPanelA));
+        oz_store_digits<8>(l, eL, lrow, lg, Bs, kOzB, kOzDigits * kOzB);
+        oz_store_digits<16>(v, eB, brow, bg, As, kOzA, kOzDigits * kOzA);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1479,21 +1649,12 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
     const uint32_t tmem = *tslot;
     if (tid == 0) {
         const uint32_t sa = smem_addr(As), sb = smem_addr(Bs), b0 = smem_addr(bar);
-        for (int L = 0; L < kOzDigits; ++L)
-            for (int da = 0; da <= L; ++da)
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {       // K half kk / 2, 16 columns each
-                    const uint32_t acc = (da > 0 || kk > 0) ? 1u : 0u;
-                    const uint32_t ko = (kk & 1) * 2 * kOzLbo;
-                    const uint64_t adesc = oz_sdesc(sa + da * static_cast<uint32_t>(kOzPanelA) +
-                                                    (kk >> 1) * static_cast<uint32_t>(kOzPanelA / 2) + ko);
-                    const uint64_t bdesc = oz_sdesc(sb + (L - da) * static_cast<uint32_t>(kOzPanelB) +
-                                                    (kk >> 1) * static_cast<uint32_t>(kOzPanelB / 2) + ko);
-                    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                                 :: "r"(tmem + static_cast<uint32_t>(64 * L)), "l"(adesc), "l"(bdesc),
-                                    "r"(kOzIdesc64), "r"(acc));
-                }
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t ah = sa + h * static_cast<uint32_t>(kOzDigits * kOzA);
+            const uint32_t bh = sb + h * static_cast<uint32_t>(kOzDigits * kOzB);
+            oz_products(tmem, ah, bh, h, 0, 3);
+            oz_products(tmem, ah, bh, h, 3, kOzDigits);
+        }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                      :: "r"(b0) : "memory");
         if (!oz_wait(b0)) {
@@ -1513,11 +1674,21 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
 #pragma unroll
         for (int c8 = 0; c8 < 2; ++c8) {
             long long u[8];
-            oz_read8<64>(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
+            oz_read8(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
+            bool any = false;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int e = er + eb[ch + 8 * c8 + q] - 52;
+                any |= !oz_plain(e);
+                v[8 * c8 + q] = oz_value(u[q], e, any);
+            }
+            if (any)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[8 * c8 + q] = oz_value_any(u[q], er + eb[ch + 8 * c8 + q] - 52);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int j = 8 * c8 + q, col = ch + j;
-                v[j] = row < nra && col < w ? oz_value(u[q], er + eb[col] - 52) : 0.0;
+                v[j] = row < nra && col < w ? v[j] : 0.0;
                 if (row < nra && col < w) Fs[(r0 + row) + static_cast<int64_t>(k0 + col) * LD] = v[j];
                 mx = max(mx, oz_abs(v[j]));
             }
@@ -1532,7 +1703,7 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
     }
     if (!ok) return;
     const int E = oz_exponent(max(max(rmax[row], rmax[128 + row]), max(rmax[256 + row], rmax[384 + row])));
-    oz_store_digits<16>(v, E, qa + row, ch / 16, dig, plane);
+    oz_store_digits<16>(v, E, qa + row, ch / 16, dig, plane, plane >> 1);
     if (ch == 0) dexp[qa + row] = E;
 }
 
@@ -2273,6 +2444,9 @@ static void set_smem_attrs() {
 KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_t stream)
     : plan_(plan), lp_(lp), st_(stream) {
     const auto& p = plan_;
+    int dev = 0;
+    SK_CUDA(cudaGetDevice(&dev));
+    SK_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
     // tile-inverse offsets and per-level column-block prefixes of the backward pass
     std::vector<int64_t> inv_off(static_cast<size_t>(p.ns), 0);
     inv_size_ = 0;
@@ -2387,7 +2561,7 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
     reserve(arena_, tn_, static_cast<size_t>(std::max(1, p.N)));
     reserve(arena_, params_, 4);
     reserve(arena_, err_, 4);
-    reserve(arena_, oz_cnt_, std::max<size_t>(1, p.sn_ncols.size()));
+    reserve(arena_, oz_cnt_, p.sn_ncols.size() + 1);
     reserve(arena_, lp_fail_, std::max<size_t>(1, static_cast<size_t>(p.nlp)));
     for (auto& sb : sub_) {
         reserve(arena_, sb.d_items, std::max<size_t>(1, p.step_items.size()));
@@ -2499,7 +2673,7 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                     } else if (emulate64_) {   // FP64-accurate panel solve on the tensor cores
                         k_panel_oz<<<static_cast<int>(st.digit_rows / 128), 512, kOzPanelSmem, st_>>>(
                             a, items, prefix, pdv, F, Linv, inv_off_.ptr, dig_.ptr, dexp_.ptr,
-                            plan_.max_digit_rows * 128, err_.ptr);
+                            plan_.max_digit_rows * 128, oz_cnt_.ptr + plan_.ns, err_.ptr);
                     } else if (tiles < kTr4Tiles) {
                         k_trsm_rows<4><<<8 * tiles, 128, tr_smem(4), st_>>>(a, items, prefix, pdv, F, Linv,
                                                                             inv_off_.ptr);
@@ -2525,9 +2699,10 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                         if (emulate64_) {
                             tc = true;
                             const int64_t plane = plan_.max_digit_rows * 128;
-                            k_update_oz<<<(st.nitems + static_cast<int>(st.upd3_blocks)) * 2, 256, kOzSmemU, st_>>>(
+                            const int64_t units = st.nitems + st.upd3_blocks;
+                            k_update_oz<<<static_cast<int>(std::min<int64_t>(units, sms_)), 320, kOzSmemU, st_>>>(
                                 a, items, prefix, pdv, F, Linv, inv_off_.ptr, dig_.ptr,
-                                dexp_.ptr, plane, oz_cnt_.ptr, err_.ptr);
+                                dexp_.ptr, plane, oz_cnt_.ptr + plan_.ns, err_.ptr);
                         }
                     }
                     if (tc) return;

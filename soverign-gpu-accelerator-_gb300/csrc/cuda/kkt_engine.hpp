@@ -122,6 +122,7 @@ private:
     ipm::FrontPlan plan_;
     const DeviceLP& lp_;
     cudaStream_t st_;
+    int sms_ = 0;                               // of this device
     Arena arena_;
     Arena f32_arena_, f64_arena_;
     Slot<float> F32_, Linv32_;
@@ -150,7 +151,7 @@ private:
     // numeric work
     Slot<double> D_, Mdiag_, zp_, xp_, zsol_, fvec_, tn_, params_;
     Slot<int> err_;
-    Slot<int> oz_cnt_;                          // per front: blocks of the first update tile done (fused potrf)
+    Slot<int> oz_cnt_;                          // per front: parts of the next diagonal tile updated; then the tile counter
     bool fp32_ = false;
     int failed_sn_ = -1;
     std::vector<int> failed_lps_;
