@@ -288,16 +288,18 @@ __global__ void k_asm_cols_dense(int M, const int* __restrict__ rp, const int* _
 //    sqrt 600 cycles, a division 355, a 64-bit shuffle 16).
 //  * So warp 0 alone factors the diagonal block, from registers (shuffles, no barrier),
 //    while the warps of the other three quarters (helpers) apply the previous block's
-//    update to the rows below and form the inverse's block rows that are already known.
-//    Warp 0 joins them when its block is done; warp 4 shares its quarter and stays out.
+//    update to the rows below (two of them first) and form the inverse's block rows that
+//    are already known (four of them, in the last block all). Warp 0 joins them when its
+//    block is done; warp 4 shares its quarter and stays out.
 //  * The root and the reciprocal of an FP64 pivot take five dependent FP64 instructions
 //    instead of a sqrt and a division.
-// One tile: FP64 116 -> 58 us, FP32 38 -> 17 us.
+// One tile: FP64 116 -> 53 us, FP32 38 -> 15 us.
 constexpr int kPB = 16;
 constexpr int kPBTri = kPB * (kPB + 1) / 2;
 
-// The helper warps' own barrier (192 threads), and the one on which warp 0 waits for them.
-__device__ __forceinline__ void helper_sync() { asm volatile("bar.sync 1, 192;" ::: "memory"); }
+// The barrier of the warps that extend the inverse, and the one on which the others wait for
+// its block row.
+__device__ __forceinline__ void inverse_sync(int threads) { asm volatile("bar.sync 1, %0;" :: "r"(threads) : "memory"); }
 __device__ __forceinline__ void inverse_arrive() { asm volatile("bar.arrive 2, 224;" ::: "memory"); }
 __device__ __forceinline__ void inverse_wait() { asm volatile("bar.sync 2, 224;" ::: "memory"); }
 
@@ -397,29 +399,27 @@ __device__ __noinline__ bool factor_rest(T* A, T* rdiag, int c0, int j) {
     return bad;
 }
 
-// Warp 0: the diagonal block at c0; lane (r, h) holds the columns 2k + h of row r. Leaves
-// L in A and 1 / L(c, c) in rdiag. Result: a pivot was not positive (it counts as 1).
-// Column j updates column j + 1 at once and the others while the next pivot's root forms.
-template <class T>
-__device__ __forceinline__ bool factor_block(T* A, T* rdiag, int c0) {
+// Warp 0: the diagonal block at c0. Leaves L in A and 1 / L(c, c) in rdiag. Result: a pivot was
+// not positive (it counts as 1). FP32: lane (r, h) holds the columns 2k + h of row r. Column j updates column j + 1 at once and the others while the next pivot's root forms.
+__device__ __forceinline__ bool factor_block(float* A, float* rdiag, int c0) {
     const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
-    T v[8];
+    float v[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const int c = 2 * k + h;
-        v[k] = r >= c ? A[(c0 + r) * LDS + c0 + c] : T(0);
+        v[k] = r >= c ? A[(c0 + r) * LDS + c0 + c] : 0.f;
     }
-    T l = T(0);
+    float l = 0.f;
 #pragma unroll
     for (int j = 0; j < kPB; ++j) {
-        const T a = __shfl_sync(0xffffffffu, v[j >> 1], r + 16 * (j & 1));    // column j of every row
-        const T p = __shfl_sync(0xffffffffu, v[j >> 1], j + 16 * (j & 1));
+        const float a = __shfl_sync(0xffffffffu, v[j >> 1], r + 16 * (j & 1));    // column j of every row
+        const float p = __shfl_sync(0xffffffffu, v[j >> 1], j + 16 * (j & 1));
         auto update = [&](int k, int from) {           // columns 2k, 2k + 1 by column `from`
-            const T lc = __shfl_sync(0xffffffffu, l, 2 * k + h);
-            const T t = fma_ordered(-l, lc, v[k]);
+            const float lc = __shfl_sync(0xffffffffu, l, 2 * k + h);
+            const float t = fmaf(-l, lc, v[k]);
             v[k] = 2 * k + h > from ? t : v[k];
         };
-        T d, rd;
+        float d, rd;
         const int rest = (j >> 1) + 1;                 // column j - 1's columns still to update: 2 rest ..
         if (!plain_pivot(p)) {
 #pragma unroll
@@ -442,6 +442,71 @@ __device__ __forceinline__ bool factor_block(T* A, T* rdiag, int c0) {
         if (j + 1 < kPB) update((j + 1) >> 1, j);
         if (h == 0 && r >= j) A[(c0 + r) * LDS + c0 + j] = r == j ? d : l;
         if (lane == 0) rdiag[c0 + j] = rd;
+    }
+    return false;
+}
+
+// FP64: lane r (and r + 16) holds row r of the column that is to be factored; the columns
+// after it are packed into four registers a lane, the last column first, so that the entries
+// still to be updated fill whole warps: a column costs its 7 dependent FP64 instructions and
+// 1.7 for the others (as two columns a register 4.5: 1240 cycles a column, now 810). Column
+// j - 1 updates them while column j's root forms, then column j + 1 leaves them.
+__device__ __forceinline__ bool factor_block(double* A, double* rdiag, int c0) {
+    const int lane = threadIdx.x & 31, r = lane & 15;
+    constexpr int kSlots = 4;
+    auto live = [](int j) { return (15 - j) * (16 - j) / 2; };       // entries in the columns after j
+    double v[kSlots];
+    double* at[kSlots];                                 // the entry's place
+    int ri[kSlots], rq[kSlots];                         // its row and column of A, as offsets of their rows
+    double* Ac = A + c0 * LDS + c0;
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) {
+        int n, i;                                       // entry i of the n-th column from the last
+        tri_index(min(lane + 32 * k, 119), n, i);
+        const int q = 15 - n;
+        ri[k] = (q + i) * LDS;
+        rq[k] = q * LDS;
+        at[k] = Ac + ri[k] + q;
+        v[k] = *at[k];
+    }
+    double a = Ac[r * LDS], l = 0.0;
+#pragma unroll
+    for (int j = 0; j < kPB; ++j) {
+        const double p = __shfl_sync(0xffffffffu, a, j);
+        auto update = [&](int k) {                      // slot k by column j - 1
+            v[k] = fma_ordered(-Ac[ri[k] + j - 1], Ac[rq[k] + j - 1], v[k]);
+        };
+        const int slots = (live(j) + 31) / 32;          // with columns after j
+        if (!plain_pivot(p)) {
+#pragma unroll
+            for (int k = 0; k < kSlots; ++k)
+                if (k < slots && j > 0) update(k);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < kSlots; ++k)
+                if (lane + 32 * k < live(j)) *at[k] = v[k];
+            if (lane < kPB && r >= j) Ac[r * LDS + j] = a;
+            __syncwarp();
+            return factor_rest(A, rdiag, c0, j);
+        }
+        double d, rd, b = 0.0;
+        pivot_root(p, d, rd, [&](int n) {
+            if (j > 0 && n < slots) update(n);
+            if (n == 3 && j + 1 < kPB) {                // column j + 1 leaves the slots
+#pragma unroll
+                for (int k = 0; k < kSlots; ++k)
+                    if (32 * k < live(j) && 32 * k + 32 > live(j + 1) && lane + 32 * k >= live(j + 1) &&
+                        lane + 32 * k < live(j))
+                        *at[k] = v[k];
+            }
+        });
+        __syncwarp();
+        if (j + 1 < kPB) b = Ac[r * LDS + j + 1];       // rows above it are not used
+        l = a * rd;
+        if (lane < kPB && r >= j) Ac[r * LDS + j] = r == j ? d : l;
+        if (lane == 0) rdiag[c0 + j] = rd;
+        if (j + 1 < kPB) a = fma_ordered(-l, __shfl_sync(0xffffffffu, l, j + 1), b);
+        __syncwarp();
     }
     return false;
 }
@@ -560,13 +625,15 @@ __device__ __forceinline__ void inverse_block(const double* A, double* X, const 
 // columns j < r0, kept transposed in X's upper triangle (e: rows i, i + 8 of kCols columns),
 // then X(i, j) = -sum_q X(i, r0 + q) T(r0 + q, j) (e: row i of kCols columns). FP32 is bound
 // by its shared loads here and takes two columns at a time, FP64 by how evenly the
-// warps' instructions are dealt out (with two columns 134k cycles a tile, with one 130k).
+// warps' instructions are dealt out (with two columns 134k cycles a tile, with one 130k); a
+// warp takes eight rows of four neighbouring columns, whose sums are about equally long (as two
+// rows of sixteen columns 23% of its instructions had idle lanes).
 template <class T> constexpr int kCols = sizeof(T) == 4 ? 2 : 1;
 
 template <class T>
 __device__ __forceinline__ void inverse_sums(const T* A, T* X, int r0, int e) {
-    constexpr int C = kCols<T>, per = kPB * kPB / (2 * C);
-    const int i = r0 + (e % per) / (kPB / C), j = (e / per) * kPB + C * (e % (kPB / C));
+    constexpr int C = kCols<T>;
+    const int i = r0 + (e & 7), j = C * (e >> 3);
     const T* a = A + i * LDS;
     T u[C], v[C];
 #pragma unroll
@@ -619,15 +686,18 @@ __device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, T* F, T* _
     const int w = min(T64, pd.sn_ncols[s] - k0);
     T* Fs = F + pd.F_off[s];
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-#pragma unroll 4
-    for (int it = 0; it < 16; ++it) {
-        const int idx = tid + it * 256;
-        const int r = idx & 63, c = idx >> 6;
-        if (c > r) continue;
-        T x = T(0);
-        if (r < w && c < w) x = Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD];
-        else if (r == c) x = T(1);
-        A[r * LDS + c] = x;
+    {
+        T x[16];                          // all of a thread's entries in flight together
+#pragma unroll
+        for (int it = 0; it < 16; ++it) {
+            const int r = tid & 63, c = (tid >> 6) + 4 * it;
+            x[it] = c <= r && r < w ? Fs[(k0 + r) + static_cast<int64_t>(k0 + c) * LD] : r == c ? T(1) : T(0);
+        }
+#pragma unroll
+        for (int it = 0; it < 16; ++it) {
+            const int r = tid & 63, c = (tid >> 6) + 4 * it;
+            if (c <= r) A[r * LDS + c] = x[it];
+        }
     }
     if (tid < 12) next[tid] = 0;
     tile_sync();
@@ -649,22 +719,34 @@ __device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, T* F, T* _
         const bool helper = (wid & 3) != 0;
         if (wid == 0 && factor_block(A, rdiag, c0)) report_pivot(s, pd, err);
         if (c0 > 0) {
-            if (helper) {
-                inverse_block(A, X, rdiag, c0 - kPB, ht);
-                helper_sync();
-                if (c0 > kPB) share(counter, (c0 - kPB) * kPB / kCols<T>, [&](int e) { inverse_rows(X, c0 - kPB, e); });
-            }
             if (wid != 4) {
-                // warp 0 joins once its block is done and the inverse's last block row is there
-                if (helper) { helper_sync(); inverse_arrive(); }
-                else inverse_wait();
-                share(counter + 1, c0 * kPB / (2 * kCols<T>), [&](int e) { inverse_sums(A, X, c0, e); });
-                // less the diagonal block's entries or squares
-                constexpr int C = kCols<T>, kDone = kPB / C * (kPB / C + 1) / 2;
-                share(counter + 2, (nt + kPB) / C * ((nt + kPB) / C + 1) / 2 - kDone, [&](int e) {
-                    if constexpr (C == 2) trail_square(A, c0 - kPB, kDone + e);
-                    else trail_entry(A, c0 - kPB, kDone + e);
-                });
+                auto sums = [&] {
+                    share(counter + 1, c0 * kPB / (2 * kCols<T>), [&](int e) { inverse_sums(A, X, c0, e); });
+                };
+                auto trail = [&] {                     // less the diagonal block's entries or squares
+                    constexpr int C = kCols<T>, kDone = kPB / C * (kPB / C + 1) / 2;
+                    share(counter + 2, (nt + kPB) / C * ((nt + kPB) / C + 1) / 2 - kDone, [&](int e) {
+                        if constexpr (C == 2) trail_square(A, c0 - kPB, kDone + e);
+                        else trail_entry(A, c0 - kPB, kDone + e);
+                    });
+                };
+                // the inverse's block row: by four warps while the others update, by all six in the
+                // last block, where there is nothing else
+                const int ni = nt > 0 ? 128 : 192;
+                if (helper && ht < ni) {
+                    inverse_block(A, X, rdiag, c0 - kPB, ht);
+                    inverse_sync(ni);
+                    if (c0 > kPB)
+                        share(counter, (c0 - kPB) * kPB / kCols<T>, [&](int e) { inverse_rows(X, c0 - kPB, e); });
+                    inverse_sync(ni);
+                    inverse_arrive();
+                    sums();
+                    trail();
+                } else {
+                    trail();
+                    inverse_wait();
+                    sums();
+                }
             }
         }
         tile_sync();
@@ -679,7 +761,7 @@ __device__ __noinline__ void potrf_tile(int s, int kstep, PlanDev pd, T* F, T* _
     for (int e = tid; e < (T64 - kPB) * kPB / kCols<T>; e += 256) inverse_rows(X, T64 - kPB, e);
     tile_sync();
     T* Li = Linv + inv_off[s] + static_cast<int64_t>(kstep) * T64 * T64;
-#pragma unroll 4
+#pragma unroll
     for (int it = 0; it < 16; ++it) {
         const int idx = tid + it * 256;
         const int r = idx & 63, c = idx >> 6;
@@ -1310,8 +1392,8 @@ __device__ __forceinline__ int block_row_of(int lb) {
 // kept apart in neighbouring groups of columns and have no branch between them. The block
 // with a front's first tile factors the next diagonal tile and waits for it without polling.
 // As 128 x 32 tiles of blocks that copied, multiplied and subtracted in turn, two on an SM, a
-// tile's half took 29,000 cycles: mean step at m = 4740 85 -> 78 us (there the diagonal tile's
-// 64 us are the limit), of 40 LPs (54,000 rows) 161 -> 115 us. Waits are bounded: on a
+// tile's half took 29,000 cycles: mean step at m = 4740 85 -> 69 us (there the diagonal tile is
+// the limit), of 40 LPs (54,000 rows) 161 -> 110 us. Waits are bounded: on a
 // time-out the block records err[2], takes no further tile, waits once more for what it issued
 // and frees its TMEM.
 constexpr size_t kOzSmemU = kOzDigits * (2 * kOzA + 4 * kOzB) + 512;
