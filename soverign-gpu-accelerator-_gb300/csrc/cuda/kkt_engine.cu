@@ -297,14 +297,16 @@ __global__ void k_asm_cols_dense(int M, const int* __restrict__ rp, const int* _
 constexpr int kPB = 16;
 constexpr int kPBTri = kPB * (kPB + 1) / 2;
 
+// These barriers count whole warps, which therefore meet first: a thread that reported a bad
+// pivot, or left a loop early, may still be on its own.
 // The barrier of the warps that extend the inverse, and the one on which the others wait for
 // its block row.
-__device__ __forceinline__ void inverse_sync(int threads) { asm volatile("bar.sync 1, %0;" :: "r"(threads) : "memory"); }
-__device__ __forceinline__ void inverse_arrive() { asm volatile("bar.arrive 2, 224;" ::: "memory"); }
-__device__ __forceinline__ void inverse_wait() { asm volatile("bar.sync 2, 224;" ::: "memory"); }
+__device__ __forceinline__ void inverse_sync(int threads) { __syncwarp(); asm volatile("bar.sync 1, %0;" :: "r"(threads) : "memory"); }
+__device__ __forceinline__ void inverse_arrive() { __syncwarp(); asm volatile("bar.arrive 2, 224;" ::: "memory"); }
+__device__ __forceinline__ void inverse_wait() { __syncwarp(); asm volatile("bar.sync 2, 224;" ::: "memory"); }
 
 // The 256 threads of a diagonal tile (the update's block has one more warp).
-__device__ __forceinline__ void tile_sync() { asm volatile("bar.sync 3, 256;" ::: "memory"); }
+__device__ __forceinline__ void tile_sync() { __syncwarp(); asm volatile("bar.sync 3, 256;" ::: "memory"); }
 
 __device__ __noinline__ void report_pivot(int s, const PlanDev& pd, int* err) {
     if ((threadIdx.x & 31) != 0) return;
@@ -1156,7 +1158,7 @@ constexpr uint32_t kOzLbo = 128;                       // bytes between K-adjace
 constexpr uint32_t kOzSbo = 512;                       // bytes between 8-row groups (32 bf16 per row and half)
 constexpr size_t kOzA = 128 * 64;                      // 128 rows of one plane and half: 8 KB
 constexpr size_t kOzB = 64 * 64;                       // 64 rows: 4 KB
-constexpr int kOzSpin = 1 << 22;
+constexpr long long kOzCycles = 1LL << 31;             // how long a copy or an MMA batch may take: a second
 // instruction descriptors (kind::f16): D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1),
 // both K-major, N >> 3 at bits 17-22 (added per product), M >> 4 at bits 24-28 (M = 128)
 constexpr uint32_t kOzIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
@@ -1172,15 +1174,17 @@ __device__ __forceinline__ double oz_pow2(int p) {       // 2^p, 0 below the nor
     if (p < -1022) return 0.0;
     return __longlong_as_double(static_cast<long long>(p + 1023) << 52);
 }
-__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity = 0, int limit = kOzSpin,
+__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity = 0, long long limit = kOzCycles,
                                         int polls = 4096) {
     uint32_t done = 0;
-    for (int spin = 0; spin < limit && !done; ++spin) {
+    const long long start = clock64();
+    for (int spin = 0; !done; ++spin) {
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         // back-to-back polls first: a copy or an MMA batch of one tile completes within
         // microseconds, and a sleep per poll adds its own latency to every tile
         if (!done && spin >= polls) __nanosleep(polls ? 32 : 1000);
+        if (!done && (spin & 15) == 15 && clock64() - start > limit) break;
     }
     return done != 0;
 }
@@ -1425,12 +1429,11 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
     const uint32_t bA = smem_addr(bars), bB = bA + 16, bTile = bA + 48, bLo = bA + 80, bHi = bA + 88,
                    bLoFree = bA + 104, bHiFree = bA + 112, bTri = bA + 120;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    constexpr int kLimit = 2 * kOzSpin;   // waits for other warps, whose own waits end before
     if (tid == 0) {
         for (int b = 0; b < 16; ++b)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bA + 8 * b), "r"(b < 13 ? 1 : 8));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *fail = 0;
+        *fail = *reinterpret_cast<volatile int*>(err + 2);   // an earlier step's time-out: no more tiles
     }
     if (wid == 8) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_addr(tslot)));
@@ -1440,6 +1443,17 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
+    // for another warp, whose own waits end before
+    auto wait_warp = [&](uint32_t bar, int n, int code, int polls = 4096) {
+        bool done = oz_wait(bar, n & 1, 2 * kOzCycles, polls);
+        done = __all_sync(0xffffffffu, done);         // the warp goes on together
+        if (!done && lane == 0) {
+            *fail = 1;
+            atomicExch(err + 2, code);
+        }
+        __syncwarp();
+        return done;
+    };
     // a copy or an MMA batch that does not complete
     auto wait_async = [&](uint32_t bar, int n) {      // the n-th phase of a barrier
         bool done = *fail == 0 && oz_wait(bar, n & 1);
@@ -1448,6 +1462,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             *fail = 1;
             atomicExch(err + 2, 1);
         }
+        __syncwarp();
         return done;
     };
     if (wid == 9) {
@@ -1459,7 +1474,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
         bool first = false;                           // the tile before was a first one
         for (int t = 0;; ++t) {
             // the diagonal tile needs the SM's issue slots: no polling beside it
-            if (first) oz_wait(bTri, tri++ & 1, kLimit, 0);
+            if (first) wait_warp(bTri, tri++, 2, 0);
             OzTile w;
             w.s = -1;
             while (u < total && w.s < 0) {
@@ -1494,7 +1509,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                 rows = bi;
             }
             const int buf = t & 1;
-            bool ok = w.s >= 0;
+            bool ok = w.s >= 0 && *fail == 0;
             if (ok && t > 1) ok = wait_async(bHi + 8 * buf, (t - 2) >> 1);              // B's buffer is no longer read
             if (ok)
                 for (int h = 0; h < 2; ++h)
@@ -1514,15 +1529,15 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             if (!ok) break;
         }
         if (*fail != 0)                               // what may still be in flight
-            for (int b = 0; b < 6; ++b) oz_wait(bA + 8 * b, 0, 1 << 12);
+            for (int b = 0; b < 6; ++b) oz_wait(bA + 8 * b, 0, kOzCycles / 64);
     } else if (wid == 8) {
         const uint32_t sa = smem_addr(As);
         int na = 0;
         for (int t = 0;; ++t) {
-            if (!oz_wait(bTile + 8 * (t & 3), (t >> 2) & 1, kLimit, t > 0 && slot[(t - 1) & 3].first ? 0 : 4096) ||
+            if (!wait_warp(bTile + 8 * (t & 3), t >> 2, 3, t > 0 && slot[(t - 1) & 3].first ? 0 : 4096) ||
                 slot[t & 3].s < 0) break;
             na += slot[t & 3].fresh;
-            if (t > 0) oz_wait(bLoFree, (t - 1) & 1, kLimit);
+            if (t > 0) wait_warp(bLoFree, t - 1, 4);
             const uint32_t sb = smem_addr(Bs) + (t & 1) * 2 * kB;
             bool ok = true;
             for (int h = 0; h < 2; ++h) {
@@ -1531,7 +1546,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                 if (ok && lane == 0) oz_products(tmem, sa + h * kA, sb + h * kB, h, 3, kOzDigits);
             }
             if (lane == 0) oz_commit(bLo);
-            if (t > 0) oz_wait(bHiFree, (t - 1) & 1, kLimit);
+            if (t > 0) wait_warp(bHiFree, t - 1, 5);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (lane == 0) {
                 if (ok)
@@ -1544,7 +1559,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
         const int row = 32 * (wid & 3) + lane, ch = 32 * (wid >> 2);      // this thread's row and columns
         const uint32_t tl = tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch);
         for (int t = 0;; ++t) {
-            if (!oz_wait(bTile + 8 * (t & 3), (t >> 2) & 1, kLimit)) break;
+            if (!wait_warp(bTile + 8 * (t & 3), t >> 2, 6)) break;
             const OzTile w = slot[t & 3];
             if (w.s < 0) break;
             const int r = w.r0 + row;
@@ -1552,8 +1567,8 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             const int nj = r < w.N ? min(32, min(w.N, r + 1) - (w.c0 + ch)) : 0;
             double* C = F + w.F + r + static_cast<int64_t>(w.c0 + ch) * w.LD;
             const int ea = dexp[w.qa + row] - 52, eb = dexp[w.qb + ch + lane];
-            const bool plain = oz_plain(ea + __reduce_min_sync(0xffffffffu, eb)) &&
-                               oz_plain(ea + __reduce_max_sync(0xffffffffu, eb));
+            const int elo = __reduce_min_sync(0xffffffffu, eb), ehi = __reduce_max_sync(0xffffffffu, eb);
+            const bool plain = oz_plain(ea + elo) && oz_plain(ea + ehi);
             double cv[2][16];
             auto load_c = [&](int h) {
 #pragma unroll
@@ -1561,7 +1576,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                     cv[h][j] = 16 * h + j < nj ? C[static_cast<int64_t>(16 * h + j) * w.LD] : 0.0;
             };
             load_c(0);
-            oz_wait(bLo, t & 1, kLimit);
+            wait_warp(bLo, t, 7);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             long long lo[32];
             {
@@ -1578,7 +1593,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
 #pragma unroll
                 for (int j = 0; j < 32; ++j) lo[j] = oz_lower(v + j, 32);
             }
-            oz_wait(bHi + 8 * (t & 1), (t >> 1) & 1, kLimit);
+            wait_warp(bHi + 8 * (t & 1), t >> 1, 8);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int last = *fail == 0 ? nj : 0;
             // Eight columns at a time; their subtractions are issued between the integer work of
@@ -1616,6 +1631,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                         const int e = ea + __shfl_sync(0xffffffffu, eb, 8 * g + q);
                         if (any) x[g & 1][q] = oz_value_any(u[q], e);
                     }
+                    __syncwarp();
                 }
                 if (g == 0) load_c(1);
             }
@@ -2097,7 +2113,7 @@ __global__ void k_fwd_gather(int n, const int* __restrict__ dst, const int* __re
 // there: with two of them in registers the FP32 solves of 40 LPs take 206 -> 110 us forward
 // and 133 -> 93 us backward.
 
-constexpr int kSpinLimit = 1 << 24;
+constexpr long long kAwaitCycles = 1LL << 32;      // two seconds
 constexpr int kReadyBlocks = 16;   // column blocks taken per pass once they are there
 
 __device__ __forceinline__ float peek(const float* p) {
@@ -2122,10 +2138,12 @@ __device__ __forceinline__ void publish(double* p, double v) {
 // *p once it is there; false on time-out or when another task gave up.
 template <class T>
 __device__ __forceinline__ bool await(const T* p, T& v, int* err) {
+    const long long start = clock64();
     for (int spins = 0;; ++spins) {
         v = peek(p);
         if (!Pending<T>::is(v)) return true;
-        if (spins > kSpinLimit || ((spins & 255) == 255 && *reinterpret_cast<volatile int*>(err) != 0)) {
+        if ((spins & 255) == 255 &&
+            (clock64() - start > kAwaitCycles || *reinterpret_cast<volatile int*>(err) != 0)) {
             atomicExch(err, 1);
             return false;
         }
