@@ -512,9 +512,11 @@ int sk_kkt_solve_device(sk_kkt* k, double* d_rhs, double tol) {
         const double t = tol * std::max(1.0, rn_rhs);
         E.apply_inverse(d_rhs, k->out.ptr);
         auto resid = [&]() {
-            E.apply_normal(k->theta.ptr, k->out.ptr, k->tmp.ptr);
-            dev::vec_diff(m, d_rhs, k->tmp.ptr, k->r.ptr, st);
-            return dev::absmax_device(m, k->r.ptr, k->scratch.ptr, st);
+            E.residual(k->theta.ptr, d_rhs, k->out.ptr, k->r.ptr, k->scratch.ptr);
+            double rn = 0.0;
+            SK_CUDA(cudaMemcpyAsync(&rn, k->scratch.ptr, sizeof(rn), cudaMemcpyDeviceToHost, st));
+            SK_CUDA(cudaStreamSynchronize(st));
+            return rn;
         };
         double rn = resid();
         const int max_ir = k->precision == SK_PREC_MIXED ? 30 : 10;

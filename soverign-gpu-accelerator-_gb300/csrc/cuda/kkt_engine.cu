@@ -2477,14 +2477,91 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
 
 // ------------------------------------------------------- normal-matrix apply
 
-__global__ void k_spmv_rows(int rows, const int* __restrict__ rp, const int* __restrict__ ci,
-                            const double* __restrict__ v, const double* __restrict__ x,
-                            const double* __restrict__ scale, double* __restrict__ y) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
+// What a row's product becomes: y = scale .* (A x), and r = b - A x with its largest entry.
+// A NaN does not count as an entry (fmax), and |r| >= 0 orders like its bits.
+__device__ __forceinline__ void absmax_add(double v, unsigned long long* mx) {
+    unsigned long long m = static_cast<unsigned long long>(oz_abs(v));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(mx, m);
+}
+struct RowScaled {
+    const double* scale;               // may be null
+    double* y;
+    unsigned long long* clear;         // may be null: the next product's maximum
+    __device__ void operator()(int r, bool valid, double acc) const {
+        if (valid) y[r] = scale ? acc * scale[r] : acc;
+        if (clear && r == 0) *clear = 0;
+    }
+};
+struct RowResidual {
+    const double* b;
+    double* res;
+    unsigned long long* mx;
+    __device__ void operator()(int r, bool valid, double acc) const {
+        const double d = valid ? b[r] - acc : 0.0;
+        if (valid) res[r] = d;
+        absmax_add(d, mx);
+    }
+};
+
+// A x, each row summed by one lane in its entries' order. The sums are as long as the longest
+// row (64 cycles an entry), so a block takes only 32 rows; their entries come through shared
+// memory, 32 of every row at a time: four warps load whole row segments of the next tile
+// while warp 0 sums one (a lane's own loads, one row each, made the product latency bound: A^T y,
+// A x, residual and its maximum 70 us at m = 4740 with 47 and 120 entries a row, now 24).
+// Rows of fewer than kRowSegment entries on average would leave most lanes of a segment idle,
+// and a lane loads its own: A^T y with 6 entries a row 3.1 us, by segments 3.7.
+constexpr int kRowSegment = 8;
+template <bool Staged, class Epi>
+__global__ void __launch_bounds__(Staged ? 160 : 256) k_row_sums(int rows, const int* __restrict__ rp,
+                                                                 const int* __restrict__ ci,
+                                                                 const double* __restrict__ v,
+                                                                 const double* __restrict__ x, Epi epi) {
+    const int row = Staged ? blockIdx.x * 32 + (threadIdx.x & 31) : blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = row < rows;
+    const int q0 = valid ? rp[row] : 0, n = valid ? rp[row + 1] - q0 : 0;
     double acc = 0.0;
-    for (int q = rp[r]; q < rp[r + 1]; ++q) acc += v[q] * x[ci[q]];
-    y[r] = scale ? acc * scale[r] : acc;
+    if constexpr (Staged) {
+        constexpr int S = 33;
+        __shared__ double vs[2][32 * S], xs[2][32 * S];
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        const int len = __reduce_max_sync(0xffffffffu, n), tiles = (len + 31) / 32;   // the same in every warp
+        for (int t = 0; t <= tiles; ++t) {
+            if (wid > 0 && t < tiles) {               // tile t: eight rows a warp
+                const int k = 32 * t + lane, r0 = 8 * (wid - 1);
+                int c[8];
+                double a[8], g[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const bool in = k < __shfl_sync(0xffffffffu, n, r0 + i);
+                    const int q = __shfl_sync(0xffffffffu, q0, r0 + i) + k;
+                    c[i] = in ? ci[q] : -1;
+                    a[i] = in ? v[q] : 0.0;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) g[i] = c[i] >= 0 ? x[c[i]] : 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    vs[t & 1][(r0 + i) * S + lane] = a[i];
+                    xs[t & 1][(r0 + i) * S + lane] = g[i];
+                }
+            }
+            if (wid == 0 && t > 0) {
+                const double* va = vs[(t - 1) & 1] + lane * S;
+                const double* xa = xs[(t - 1) & 1] + lane * S;
+                const int m = min(32, n - 32 * (t - 1));
+#pragma unroll 8
+                for (int k = 0; k < 32; ++k)
+                    if (k < m) acc += va[k] * xa[k];
+            }
+            __syncthreads();
+        }
+        if (wid > 0) return;
+    } else {
+        for (int q = q0; q < q0 + n; ++q) acc += v[q] * x[ci[q]];
+    }
+    epi(row, valid, acc);
 }
 
 inline int blocks_for(int64_t n, int t) { return static_cast<int>((n + t - 1) / t); }
@@ -3093,11 +3170,30 @@ int KktEngine::failed_lp() const {
     return failed_sn_ >= 0 && failed_sn_ < static_cast<int>(sn_lp_h_.size()) ? sn_lp_h_[failed_sn_] : -1;
 }
 
+namespace {
+template <class Epi>
+void row_sums(int rows, int64_t nnz, const int* rp, const int* ci, const double* v, const double* x, Epi epi,
+              cudaStream_t st) {
+    if (rows <= 0) return;
+    if (nnz >= static_cast<int64_t>(kRowSegment) * rows)
+        k_row_sums<true><<<blocks_for(rows, 32), 160, 0, st>>>(rows, rp, ci, v, x, epi);
+    else
+        k_row_sums<false><<<blocks_for(rows, 256), 256, 0, st>>>(rows, rp, ci, v, x, epi);
+    SK_CUDA(cudaGetLastError());
+}
+}  // namespace
+
 void KktEngine::apply_normal(const double* d_theta, const double* d_src, double* d_dst) {
     // t = theta .* (A^T src); dst = A t
-    k_spmv_rows<<<blocks_for(lp_.N, 256), 256, 0, st_>>>(lp_.N, lp_.t_rp, lp_.t_ci, lp_.t_v, d_src, d_theta, tn_.ptr);
-    k_spmv_rows<<<blocks_for(lp_.M, 256), 256, 0, st_>>>(lp_.M, lp_.a_rp, lp_.a_ci, lp_.a_v, tn_.ptr, nullptr, d_dst);
-    SK_CUDA(cudaGetLastError());
+    row_sums(lp_.N, lp_.nnz, lp_.t_rp, lp_.t_ci, lp_.t_v, d_src, RowScaled{d_theta, tn_.ptr, nullptr}, st_);
+    row_sums(lp_.M, lp_.nnz, lp_.a_rp, lp_.a_ci, lp_.a_v, tn_.ptr, RowScaled{nullptr, d_dst, nullptr}, st_);
+}
+
+void KktEngine::residual(const double* d_theta, const double* d_b, const double* d_x, double* d_res, double* d_max) {
+    unsigned long long* mx = reinterpret_cast<unsigned long long*>(d_max);
+    if (lp_.N <= 0) SK_CUDA(cudaMemsetAsync(d_max, 0, sizeof(double), st_));
+    row_sums(lp_.N, lp_.nnz, lp_.t_rp, lp_.t_ci, lp_.t_v, d_x, RowScaled{d_theta, tn_.ptr, mx}, st_);
+    row_sums(lp_.M, lp_.nnz, lp_.a_rp, lp_.a_ci, lp_.a_v, tn_.ptr, RowResidual{d_b, d_res, mx}, st_);
 }
 
 void KktEngine::profile(const double* d_theta, double delta, bool fp32, const double* d_rhs, double* d_out,
@@ -3220,10 +3316,6 @@ __global__ void k_absmax_partial(int n, const double* __restrict__ a, double* __
         part[blockIdx.x] = r;
     }
 }
-__global__ void k_axpy_diff(int n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = a[i] - b[i];
-}
 __global__ void k_add(int n, const double* __restrict__ a, double* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] += a[i];
@@ -3238,11 +3330,6 @@ double absmax_device(int n, const double* a, double* scratch64, cudaStream_t st)
     double r = 0.0;
     for (double v : h) r = std::max(r, v);
     return r;
-}
-
-void vec_diff(int n, const double* a, const double* b, double* out, cudaStream_t st) {
-    k_axpy_diff<<<(n + 255) / 256, 256, 0, st>>>(n, a, b, out);
-    SK_CUDA(cudaGetLastError());
 }
 
 void vec_add(int n, const double* a, double* out, cudaStream_t st) {

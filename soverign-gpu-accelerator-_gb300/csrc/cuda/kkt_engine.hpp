@@ -47,6 +47,8 @@ public:
     void apply_inverse(const double* d_src, double* d_dst);
     // dst = A diag(theta) A^T src (FP64, matrix-free).
     void apply_normal(const double* d_theta, const double* d_src, double* d_dst);
+    // res = b - A theta A^T x, and its largest |entry| (NaNs aside) in *d_max
+    void residual(const double* d_theta, const double* d_b, const double* d_x, double* d_res, double* d_max);
     // Which LPs of the batch are still being solved: factorisation and solves skip
     // the fronts of the others (their solve output rows are 0). All on initially.
     // apply_inverse then uses the last factor's precision for every LP.
@@ -177,7 +179,6 @@ namespace sankhya {
 namespace dev {
 // max |a_i| over n entries (synchronises; scratch64 holds 64 doubles).
 double absmax_device(int n, const double* a, double* scratch64, cudaStream_t st);
-void vec_diff(int n, const double* a, const double* b, double* out, cudaStream_t st);   // out = a - b
 void vec_add(int n, const double* a, double* out, cudaStream_t st);                      // out += a
 }  // namespace dev
 }  // namespace sankhya
