@@ -67,8 +67,12 @@ struct sk_kkt {
     cudaStream_t st = nullptr;
     dev::Arena arena;
     dev::Slot<int> a_rp, a_ci, t_rp, t_ci, row_lp, col_lp;
-    dev::Slot<double> a_v, t_v, theta, out, r, corr, bak, tmp, scratch, hostio;
+    dev::Slot<double> a_v, t_v, theta, out, r, corr, bak, scratch, hostio;
     dev::DeviceLP lp;
+    // the host's side of the copies: [0] the residual's largest entry, [1 ..] the right-hand side's 64
+    // partial ones, [65] the solve's error flag, [66 ..] a vector
+    dev::Pinned<double> pin;
+    static constexpr int kPinFlag = 65, kPinVec = 66;
     std::unique_ptr<dev::KktEngine> eng;
     bool factored = false;
     ~sk_kkt() {
@@ -452,12 +456,12 @@ int sk_kkt_create(int m, int n, const int* row_ptrs, const int* col_idx, const d
         dev::reserve(ar, k->a_rp, m + 1); dev::reserve(ar, k->a_ci, nz); dev::reserve(ar, k->a_v, nz);
         dev::reserve(ar, k->t_rp, n + 1); dev::reserve(ar, k->t_ci, nz); dev::reserve(ar, k->t_v, nz);
         dev::reserve(ar, k->row_lp, m); dev::reserve(ar, k->col_lp, n);
-        for (auto* s : {&k->out, &k->r, &k->corr, &k->bak, &k->tmp, &k->hostio}) dev::reserve(ar, *s, m);
+        for (auto* s : {&k->out, &k->r, &k->corr, &k->bak, &k->hostio}) dev::reserve(ar, *s, m);
         dev::reserve(ar, k->theta, n);
-        dev::reserve(ar, k->scratch, 64);
+        dev::reserve(ar, k->scratch, 65);
         ar.commit();
         for (auto* s : {&k->a_rp, &k->a_ci, &k->t_rp, &k->t_ci, &k->row_lp, &k->col_lp}) dev::bind(ar, *s);
-        for (auto* s : {&k->a_v, &k->t_v, &k->out, &k->r, &k->corr, &k->bak, &k->tmp, &k->hostio, &k->theta,
+        for (auto* s : {&k->a_v, &k->t_v, &k->out, &k->r, &k->corr, &k->bak, &k->hostio, &k->theta,
                         &k->scratch})
             dev::bind(ar, *s);
         dev::upload(k->a_rp, A.row_ptrs, k->st); dev::upload(k->a_ci, A.col_indices, k->st);
@@ -465,6 +469,7 @@ int sk_kkt_create(int m, int n, const int* row_ptrs, const int* col_idx, const d
         dev::upload(k->t_v, cv, k->st);
         SK_CUDA(cudaMemsetAsync(k->row_lp.ptr, 0, sizeof(int) * m, k->st));
         SK_CUDA(cudaMemsetAsync(k->col_lp.ptr, 0, sizeof(int) * n, k->st));
+        k->pin.alloc(static_cast<size_t>(sk_kkt::kPinVec) + std::max(m, n));
         auto& lp = k->lp;
         lp.nlp = 1; lp.M = m; lp.N = n; lp.nnz = nz;
         lp.a_rp = k->a_rp.ptr; lp.a_ci = k->a_ci.ptr; lp.a_v = k->a_v.ptr;
@@ -479,25 +484,70 @@ int sk_kkt_create(int m, int n, const int* row_ptrs, const int* col_idx, const d
     }
 }
 
+// Factorisation for the weights in k->theta.
+static int kkt_factor(sk_kkt* k) {
+    const bool fp32 = k->precision == SK_PREC_MIXED;
+    double delta = fp32 ? 1e-7 : 1e-9;
+    for (int retry = 0; retry < 5; ++retry, delta *= 10.0) {
+        if (k->eng->factor(k->theta.ptr, delta, fp32)) {
+            k->factored = true;
+            return SK_OK;
+        }
+    }
+    k->factored = false;
+    api::set_error("factorisation failed: matrix is not positive definite for any regularisation");
+    return SK_ERR_NUMERICAL;
+}
+
 int sk_kkt_factorize_device(sk_kkt* k, const double* d_theta) {
     api::clear_error();
     if (!k || !d_theta) return SK_ERR_INVALID;
     try {
         SK_CUDA(cudaMemcpyAsync(k->theta.ptr, d_theta, sizeof(double) * k->n, cudaMemcpyDeviceToDevice, k->st));
-        const bool fp32 = k->precision == SK_PREC_MIXED;
-        double delta = fp32 ? 1e-7 : 1e-9;
-        for (int retry = 0; retry < 5; ++retry, delta *= 10.0) {
-            if (k->eng->factor(k->theta.ptr, delta, fp32)) {
-                k->factored = true;
-                return SK_OK;
-            }
-        }
-        k->factored = false;
-        api::set_error("factorisation failed: matrix is not positive definite for any regularisation");
-        return SK_ERR_NUMERICAL;
+        return kkt_factor(k);
     } catch (...) {
         return api::status_of_current_exception();
     }
+}
+
+// Solve with iterative refinement into k->out; d_rhs stays. The host waits once per residual:
+// the right-hand side's largest entry comes with the first one, and a step's sum goes to a
+// second vector, which becomes the solution if it is better.
+static int kkt_solve(sk_kkt* k, const double* d_rhs, double tol) {
+    const int m = k->m;
+    cudaStream_t st = k->st;
+    auto& E = *k->eng;
+    dev::absmax_partials(m, d_rhs, k->scratch.ptr + 1, st);
+    E.apply_inverse(d_rhs, k->out.ptr);
+    auto resid = [&](const double* x, int count) {
+        E.residual(k->theta.ptr, d_rhs, x, k->r.ptr, k->scratch.ptr);
+        SK_CUDA(cudaMemcpyAsync(k->pin.ptr, k->scratch.ptr, count * sizeof(double), cudaMemcpyDeviceToHost, st));
+        SK_CUDA(cudaStreamSynchronize(st));
+        return k->pin.ptr[0];
+    };
+    double rn = resid(k->out.ptr, 65);
+    double rn_rhs = 0.0;
+    for (int q = 1; q <= 64; ++q) rn_rhs = std::max(rn_rhs, k->pin.ptr[q]);
+    const double t = tol * std::max(1.0, rn_rhs);
+    const int max_ir = k->precision == SK_PREC_MIXED ? 30 : 10;
+    for (int it = 0; it < max_ir && rn > t; ++it) {
+        E.apply_inverse(k->r.ptr, k->corr.ptr);
+        dev::vec_sum(m, k->out.ptr, k->corr.ptr, k->bak.ptr, st);
+        const double rn2 = resid(k->bak.ptr, 1);
+        if (rn2 >= rn) break;
+        std::swap(k->out.ptr, k->bak.ptr);
+        rn = rn2;
+    }
+    return rn <= t ? SK_OK : SK_ERR_NUMERICAL;
+}
+
+// Waits for the stream; false if a task of a triangular solve timed out.
+static bool kkt_finish(sk_kkt* k) {
+    int* flag = reinterpret_cast<int*>(k->pin.ptr + sk_kkt::kPinFlag);
+    k->eng->read_solve_error(flag);
+    SK_CUDA(cudaStreamSynchronize(k->st));
+    if (*flag) api::set_error("triangular solve: a task timed out waiting for a dependency");
+    return *flag == 0;
 }
 
 int sk_kkt_solve_device(sk_kkt* k, double* d_rhs, double tol) {
@@ -505,39 +555,9 @@ int sk_kkt_solve_device(sk_kkt* k, double* d_rhs, double tol) {
     if (!k || !d_rhs) return SK_ERR_INVALID;
     if (!k->factored) { api::set_error("solve before a successful factorisation"); return SK_ERR_INVALID; }
     try {
-        const int m = k->m;
-        cudaStream_t st = k->st;
-        auto& E = *k->eng;
-        const double rn_rhs = dev::absmax_device(m, d_rhs, k->scratch.ptr, st);
-        const double t = tol * std::max(1.0, rn_rhs);
-        E.apply_inverse(d_rhs, k->out.ptr);
-        auto resid = [&]() {
-            E.residual(k->theta.ptr, d_rhs, k->out.ptr, k->r.ptr, k->scratch.ptr);
-            double rn = 0.0;
-            SK_CUDA(cudaMemcpyAsync(&rn, k->scratch.ptr, sizeof(rn), cudaMemcpyDeviceToHost, st));
-            SK_CUDA(cudaStreamSynchronize(st));
-            return rn;
-        };
-        double rn = resid();
-        const int max_ir = k->precision == SK_PREC_MIXED ? 30 : 10;
-        for (int it = 0; it < max_ir && rn > t; ++it) {
-            SK_CUDA(cudaMemcpyAsync(k->bak.ptr, k->out.ptr, sizeof(double) * m, cudaMemcpyDeviceToDevice, st));
-            E.apply_inverse(k->r.ptr, k->corr.ptr);
-            dev::vec_add(m, k->corr.ptr, k->out.ptr, st);
-            const double rn2 = resid();
-            if (rn2 >= rn) {
-                SK_CUDA(cudaMemcpyAsync(k->out.ptr, k->bak.ptr, sizeof(double) * m, cudaMemcpyDeviceToDevice, st));
-                break;
-            }
-            rn = rn2;
-        }
-        SK_CUDA(cudaMemcpyAsync(d_rhs, k->out.ptr, sizeof(double) * m, cudaMemcpyDeviceToDevice, st));
-        SK_CUDA(cudaStreamSynchronize(st));
-        if (E.solve_error()) {
-            api::set_error("triangular solve: a task timed out waiting for a dependency");
-            return SK_ERR_CUDA;
-        }
-        return rn <= t ? SK_OK : SK_ERR_NUMERICAL;
+        const int rc = kkt_solve(k, d_rhs, tol);
+        SK_CUDA(cudaMemcpyAsync(d_rhs, k->out.ptr, sizeof(double) * k->m, cudaMemcpyDeviceToDevice, k->st));
+        return kkt_finish(k) ? rc : SK_ERR_CUDA;
     } catch (...) {
         return api::status_of_current_exception();
     }
@@ -547,14 +567,10 @@ int sk_kkt_factorize(sk_kkt* k, const double* theta) {
     api::clear_error();
     if (!k || !theta) return SK_ERR_INVALID;
     try {
-        dev::Arena tmp;
-        dev::Slot<double> th;
-        dev::reserve(tmp, th, k->n);
-        tmp.commit();
-        dev::bind(tmp, th);
-        SK_CUDA(cudaMemcpyAsync(th.ptr, theta, sizeof(double) * k->n, cudaMemcpyHostToDevice, k->st));
-        SK_CUDA(cudaStreamSynchronize(k->st));
-        return sk_kkt_factorize_device(k, th.ptr);
+        double* v = k->pin.ptr + sk_kkt::kPinVec;
+        std::memcpy(v, theta, sizeof(double) * k->n);
+        SK_CUDA(cudaMemcpyAsync(k->theta.ptr, v, sizeof(double) * k->n, cudaMemcpyHostToDevice, k->st));
+        return kkt_factor(k);
     } catch (...) {
         return api::status_of_current_exception();
     }
@@ -563,13 +579,15 @@ int sk_kkt_factorize(sk_kkt* k, const double* theta) {
 int sk_kkt_solve(sk_kkt* k, double* rhs, double tol) {
     api::clear_error();
     if (!k || !rhs) return SK_ERR_INVALID;
+    if (!k->factored) { api::set_error("solve before a successful factorisation"); return SK_ERR_INVALID; }
     try {
-        SK_CUDA(cudaMemcpyAsync(k->hostio.ptr, rhs, sizeof(double) * k->m, cudaMemcpyHostToDevice, k->st));
-        SK_CUDA(cudaStreamSynchronize(k->st));
-        const int rc = sk_kkt_solve_device(k, k->hostio.ptr, tol);
-        if (rc != SK_OK && rc != SK_ERR_NUMERICAL) return rc;
-        SK_CUDA(cudaMemcpyAsync(rhs, k->hostio.ptr, sizeof(double) * k->m, cudaMemcpyDeviceToHost, k->st));
-        SK_CUDA(cudaStreamSynchronize(k->st));
+        double* v = k->pin.ptr + sk_kkt::kPinVec;
+        std::memcpy(v, rhs, sizeof(double) * k->m);
+        SK_CUDA(cudaMemcpyAsync(k->hostio.ptr, v, sizeof(double) * k->m, cudaMemcpyHostToDevice, k->st));
+        const int rc = kkt_solve(k, k->hostio.ptr, tol);
+        SK_CUDA(cudaMemcpyAsync(v, k->out.ptr, sizeof(double) * k->m, cudaMemcpyDeviceToHost, k->st));
+        if (!kkt_finish(k)) return SK_ERR_CUDA;
+        std::memcpy(rhs, v, sizeof(double) * k->m);
         return rc;
     } catch (...) {
         return api::status_of_current_exception();

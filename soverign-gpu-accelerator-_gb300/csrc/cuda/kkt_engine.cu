@@ -2624,6 +2624,7 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
     int dev = 0;
     SK_CUDA(cudaGetDevice(&dev));
     SK_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
+    host_flags_.alloc(4);
     // tile-inverse offsets and per-level column-block prefixes of the backward pass
     std::vector<int64_t> inv_off(static_cast<size_t>(p.ns), 0);
     inv_size_ = 0;
@@ -2957,10 +2958,13 @@ void KktEngine::launch_solve(const T* F, const T* Linv, Prof* prof) {
 }
 
 int KktEngine::solve_error() {
-    int h = 0;
-    SK_CUDA(cudaMemcpyAsync(&h, solve_err_.ptr, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    read_solve_error(host_flags_.ptr + 3);
     SK_CUDA(cudaStreamSynchronize(st_));
-    return h;
+    return host_flags_.ptr[3];
+}
+
+void KktEngine::read_solve_error(int* host) {
+    SK_CUDA(cudaMemcpyAsync(host, solve_err_.ptr, sizeof(int), cudaMemcpyDeviceToHost, st_));
 }
 
 void KktEngine::ensure_fronts(bool fp32) {
@@ -3049,8 +3053,8 @@ bool KktEngine::factor(const double* d_theta, double delta, bool fp32) {
         SK_CUDA(cudaGraphLaunch(gfac_[q], st_));
         SK_CUDA(cudaEventRecord(fev_[1], st_));
     }
-    int herr[3];
-    SK_CUDA(cudaMemcpyAsync(herr, err_.ptr, sizeof(herr), cudaMemcpyDeviceToHost, st_));
+    const int* herr = host_flags_.ptr;
+    SK_CUDA(cudaMemcpyAsync(host_flags_.ptr, err_.ptr, 3 * sizeof(int), cudaMemcpyDeviceToHost, st_));
     SK_CUDA(cudaStreamSynchronize(st_));
     float fms = 0.f;
     SK_CUDA(cudaEventElapsedTime(&fms, fev_[0], fev_[1]));
@@ -3316,24 +3320,19 @@ __global__ void k_absmax_partial(int n, const double* __restrict__ a, double* __
         part[blockIdx.x] = r;
     }
 }
-__global__ void k_add(int n, const double* __restrict__ a, double* __restrict__ out) {
+__global__ void k_sum(int n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += a[i];
+    if (i < n) out[i] = a[i] + b[i];
 }
 }  // namespace
 
-double absmax_device(int n, const double* a, double* scratch64, cudaStream_t st) {
-    k_absmax_partial<<<64, 256, 0, st>>>(n, a, scratch64);
-    double h[64];
-    SK_CUDA(cudaMemcpyAsync(h, scratch64, sizeof(h), cudaMemcpyDeviceToHost, st));
-    SK_CUDA(cudaStreamSynchronize(st));
-    double r = 0.0;
-    for (double v : h) r = std::max(r, v);
-    return r;
+void absmax_partials(int n, const double* a, double* part64, cudaStream_t st) {
+    k_absmax_partial<<<64, 256, 0, st>>>(n, a, part64);
+    SK_CUDA(cudaGetLastError());
 }
 
-void vec_add(int n, const double* a, double* out, cudaStream_t st) {
-    k_add<<<(n + 255) / 256, 256, 0, st>>>(n, a, out);
+void vec_sum(int n, const double* a, const double* b, double* out, cudaStream_t st) {
+    k_sum<<<(n + 255) / 256, 256, 0, st>>>(n, a, b, out);
     SK_CUDA(cudaGetLastError());
 }
 

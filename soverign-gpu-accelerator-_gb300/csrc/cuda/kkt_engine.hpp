@@ -16,6 +16,20 @@
 namespace sankhya {
 namespace dev {
 
+// Page-locked host memory: a copy to or from pageable memory goes through the driver's staging
+// buffer and costs about as much again as a small kernel.
+template <class T>
+struct Pinned {
+    T* ptr = nullptr;
+    void alloc(size_t n) { SK_CUDA(cudaMallocHost(&ptr, n * sizeof(T))); }
+    Pinned() = default;
+    Pinned(const Pinned&) = delete;
+    Pinned& operator=(const Pinned&) = delete;
+    ~Pinned() {
+        if (ptr) cudaFreeHost(ptr);
+    }
+};
+
 struct PlanDev;
 
 class KktEngine {
@@ -91,6 +105,7 @@ public:
     // Non-zero when a triangular-solve task gave up waiting for a dependency
     // (synchronises). The solve result is then invalid.
     int solve_error();
+    void read_solve_error(int* host);           // the same, asynchronously into pinned memory
     // Work vectors of length N available to callers between calls.
     double* scratch_n() const { return tn_.ptr; }
 
@@ -153,6 +168,7 @@ private:
     // numeric work
     Slot<double> D_, Mdiag_, zp_, xp_, zsol_, fvec_, tn_, params_;
     Slot<int> err_;
+    Pinned<int> host_flags_;                    // err_ as the host reads it, and solve_err_
     Slot<int> oz_cnt_;                          // per front: parts of the next diagonal tile updated; then the tile counter
     bool fp32_ = false;
     int failed_sn_ = -1;
@@ -178,7 +194,7 @@ private:
 namespace sankhya {
 namespace dev {
 // max |a_i| over n entries (synchronises; scratch64 holds 64 doubles).
-double absmax_device(int n, const double* a, double* scratch64, cudaStream_t st);
-void vec_add(int n, const double* a, double* out, cudaStream_t st);                      // out += a
+void absmax_partials(int n, const double* a, double* part64, cudaStream_t st);   // max |a| over 64 parts of a
+void vec_sum(int n, const double* a, const double* b, double* out, cudaStream_t st);   // out = a + b
 }  // namespace dev
 }  // namespace sankhya
