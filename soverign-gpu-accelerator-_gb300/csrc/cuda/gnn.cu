@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 namespace sankhya {
 namespace dev {
@@ -440,7 +441,10 @@ __global__ void __launch_bounds__(256, NPT == 1 ? 3 : 4) k_layer_bwd(Side side, 
 // (og, kg) keeps 4 outputs x 8 of the 128 columns in registers (32 multiply-adds per three
 // 16-byte shared loads); the next 32 nodes are loaded while the present ones are summed. One
 // output column group per thread with the operands from the L1 took 182 us a matrix at
-// 19,000 / 48,000 nodes; now 20 us for both. Sums of 32 nodes are added up separately.
+// 19,000 / 48,000 nodes; now 20 us for both. Sums of 32 nodes are added up separately. A
+// masked gradient (0) leaves its node's features out whatever they are: a stage with an
+// infinity or a NaN among its features, which 0 times it would spread, is summed with a
+// choice at each product (the sum of a thread's features is not finite in such a stage).
 __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const float* __restrict__ g,
                                                 const float* __restrict__ x1, const float* __restrict__ x2,
                                                 float* __restrict__ dW1, float* __restrict__ dW2,
@@ -467,18 +471,19 @@ __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const floa
     };
     load(n0);
     for (int n = n0; n < n1; n += S) {
+        float all[4];                              // sums of this thread's features
 #pragma unroll
         for (int u = 0; u < 2; ++u) reinterpret_cast<float4*>(gs)[tid + 256 * u] = pg[u];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int e = tid + 256 * (u & 1);
             reinterpret_cast<float4*>(xs)[(e >> 4) * 32 + (u < 2 ? 0 : 16) + (e & 15)] = px[u];
+            all[u] = (px[u].x + px[u].y) + (px[u].z + px[u].w);
         }
-        __syncthreads();
+        const bool choose = __syncthreads_or(!isfinite((all[0] + all[1]) + (all[2] + all[3])));
         if (n + S < n1) load(n + S);
         float acc[4][8] = {}, accb[4] = {};
-#pragma unroll 4
-        for (int nn = 0; nn < S; ++nn) {
+        auto add = [&](int nn, auto masked) {
             float gv[4], xv[8];
             *reinterpret_cast<float4*>(gv) = *reinterpret_cast<const float4*>(gs + nn * H + 4 * og);
             *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(xs + nn * 2 * H + 8 * kg);
@@ -487,8 +492,16 @@ __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const floa
             for (int o = 0; o < 4; ++o) {
                 accb[o] += gv[o];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) acc[o][c] += gv[o] * xv[c];
+                for (int c = 0; c < 8; ++c)
+                    if (!masked || gv[o] != 0.f) acc[o][c] += gv[o] * xv[c];
             }
+        };
+        if (choose) {
+#pragma unroll 1
+            for (int nn = 0; nn < S; ++nn) add(nn, std::true_type{});
+        } else {
+#pragma unroll 4
+            for (int nn = 0; nn < S; ++nn) add(nn, std::false_type{});
         }
 #pragma unroll
         for (int o = 0; o < 4; ++o) {
@@ -510,7 +523,8 @@ __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const floa
 
 // Embeddings backward, columns in the first `col_blocks` blocks (their gradient d plus the
 // messages of the first layer's rows), then rows: g = d masked with h0 > 0, dE[o][k] += g[o]
-// f[k], de[o] += g[o]. Half a warp takes every sixteenth node of the block's kEmbedNodes.
+// f[k], de[o] += g[o]; a masked gradient (0) leaves its node's features out, which may be
+// infinite or no numbers. Half a warp takes every sixteenth node of the block's kEmbedNodes.
 struct EmbedGrad {
     int nodes;
     const float *d, *h, *f;
@@ -545,10 +559,10 @@ __global__ void __launch_bounds__(256) k_embed_bwd(EmbedGrad cols, EmbedGrad row
         g = mask_positive(g, y);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            s[0][k] += g.x * f[k];
-            s[1][k] += g.y * f[k];
-            s[2][k] += g.z * f[k];
-            s[3][k] += g.w * f[k];
+            if (g.x != 0.f) s[0][k] += g.x * f[k];
+            if (g.y != 0.f) s[1][k] += g.y * f[k];
+            if (g.z != 0.f) s[2][k] += g.z * f[k];
+            if (g.w != 0.f) s[3][k] += g.w * f[k];
         }
     }
 #pragma unroll
