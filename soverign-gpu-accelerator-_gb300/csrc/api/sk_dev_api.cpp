@@ -972,8 +972,10 @@ int sk_gnn_train_step(sk_gnn* g, sk_gnn_batch* bt, float lr, double* loss) {
         g->net->forward(bt->lp, g->st, nullptr, nullptr, nullptr, bt->tlx.ptr, bt->tls.ptr, bt->ty.ptr);
         g->net->backward(bt->lp, g->st, nullptr);
         g->net->adam_step(g->st, lr);
-        const double l = g->net->loss();       // the gradient and the step still run
-        if (loss) *loss = l;
+        if (loss) *loss = g->net->loss();
+        // the step is over when this returns: parameters are read and set, and other handles predict
+        // with this network, on streams that do not wait for this one
+        SK_CUDA(cudaStreamSynchronize(g->st));
         return SK_OK;
     } catch (...) {
         return api::status_of_current_exception();
