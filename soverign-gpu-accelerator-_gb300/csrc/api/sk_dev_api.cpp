@@ -512,7 +512,9 @@ int sk_kkt_factorize_device(sk_kkt* k, const double* d_theta) {
 
 // Solve with iterative refinement into k->out; d_rhs stays. The host waits once per residual:
 // the right-hand side's largest entry comes with the first one, and a step's sum goes to a
-// second vector, which becomes the solution if it is better.
+// second vector, which becomes the solution if it is better. A residual with an entry that is
+// not finite (a right-hand side or a solution with one, or beyond the fronts' range) is no
+// success, whatever the tolerance.
 static int kkt_solve(sk_kkt* k, const double* d_rhs, double tol) {
     const int m = k->m;
     cudaStream_t st = k->st;
@@ -534,11 +536,11 @@ static int kkt_solve(sk_kkt* k, const double* d_rhs, double tol) {
         E.apply_inverse(k->r.ptr, k->corr.ptr);
         dev::vec_sum(m, k->out.ptr, k->corr.ptr, k->bak.ptr, st);
         const double rn2 = resid(k->bak.ptr, 1);
-        if (rn2 >= rn) break;
+        if (!(rn2 < rn)) break;
         std::swap(k->out.ptr, k->bak.ptr);
         rn = rn2;
     }
-    return rn <= t ? SK_OK : SK_ERR_NUMERICAL;
+    return std::isfinite(rn) && rn <= t ? SK_OK : SK_ERR_NUMERICAL;
 }
 
 // Waits for the stream; false if a task of a triangular solve timed out.

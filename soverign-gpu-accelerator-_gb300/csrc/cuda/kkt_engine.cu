@@ -2478,9 +2478,9 @@ __global__ void __launch_bounds__(256, 2) k_bwd_tasks(const int2* __restrict__ t
 // ------------------------------------------------------- normal-matrix apply
 
 // What a row's product becomes: y = scale .* (A x), and r = b - A x with its largest entry.
-// A NaN does not count as an entry (fmax), and |r| >= 0 orders like its bits.
+// |r| orders like its bits, with a NaN above every number: one NaN makes the largest entry one.
 __device__ __forceinline__ void absmax_add(double v, unsigned long long* mx) {
-    unsigned long long m = static_cast<unsigned long long>(oz_abs(v));
+    unsigned long long m = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffULL;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(mx, m);

@@ -61,7 +61,7 @@ public:
     void apply_inverse(const double* d_src, double* d_dst);
     // dst = A diag(theta) A^T src (FP64, matrix-free).
     void apply_normal(const double* d_theta, const double* d_src, double* d_dst);
-    // res = b - A theta A^T x, and its largest |entry| (NaNs aside) in *d_max
+    // res = b - A theta A^T x, and its largest |entry| (a NaN if there is one) in *d_max
     void residual(const double* d_theta, const double* d_b, const double* d_x, double* d_res, double* d_max);
     // Which LPs of the batch are still being solved: factorisation and solves skip
     // the fronts of the others (their solve output rows are 0). All on initially.
