@@ -13,6 +13,8 @@
 // decoded with a binary search over a prefix of per-front tile counts.
 #include "cuda/kkt_engine.hpp"
 
+#include "cuda/oz_pipeline.hpp"
+
 #include <algorithm>
 #include <cmath>
 #include <stdexcept>
@@ -1398,8 +1400,8 @@ __device__ __forceinline__ int block_row_of(int lb) {
 // As 128 x 32 tiles of blocks that copied, multiplied and subtracted in turn, two on an SM, a
 // tile's half took 29,000 cycles: mean step at m = 4740 85 -> 69 us (there the diagonal tile is
 // the limit), of 40 LPs (54,000 rows) 161 -> 110 us. Waits are bounded: on a
-// time-out the block records err[2], takes no further tile, waits once more for what it issued
-// and frees its TMEM.
+// time-out the block records err[2] and takes no further tile; at its end it waits, again with a
+// limit, for the copies and MMAs that it has issued, and frees its TMEM.
 constexpr size_t kOzSmemU = kOzDigits * (2 * kOzA + 4 * kOzB) + 512;
 
 struct OzTile {
@@ -1472,6 +1474,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
         int item = -1, rows = -1;                     // whose rows are in As
         int tri = 0;
         bool first = false;                           // the tile before was a first one
+        PhaseLog copies;                              // barriers 0, 1: A; 2 .. 5: B
         for (int t = 0;; ++t) {
             // the diagonal tile needs the SM's issue slots: no polling beside it
             if (first) wait_warp(bTri, tri++, 2, 0);
@@ -1512,13 +1515,17 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             bool ok = w.s >= 0 && *fail == 0;
             if (ok && t > 1) ok = wait_async(bHi + 8 * buf, (t - 2) >> 1);              // B's buffer is no longer read
             if (ok)
-                for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < 2; ++h) {
                     oz_copy_rows(h, bB + 16 * buf + 8 * h, Bs + (2 * buf + h) * kB, dig, plane, w.qb, 64);
+                    copies.start(2 + 2 * buf + h);
+                }
             if (ok && w.fresh) {
                 if (t > 0) ok = wait_async(bHi + 8 * (buf ^ 1), (t - 1) >> 1);                // nor are A's rows
                 if (ok)
-                    for (int h = 0; h < 2; ++h)
+                    for (int h = 0; h < 2; ++h) {
                         oz_copy_rows(h, bA + 8 * h, As + h * kA, dig, plane, w.qa, 128);
+                        copies.start(h);
+                    }
             }
             if (!ok) w.s = -1;
             first = w.first;
@@ -1528,11 +1535,12 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             }
             if (!ok) break;
         }
-        if (*fail != 0)                               // what may still be in flight
-            for (int b = 0; b < 6; ++b) oz_wait(bA + 8 * b, 0, kOzCycles / 64);
+        for (int b = 0; b < 6; ++b)                   // none is in flight when the block ends
+            if (copies.any(b)) oz_wait(bA + 8 * b, copies.last_parity(b));
     } else if (wid == 8) {
         const uint32_t sa = smem_addr(As);
         int na = 0;
+        PhaseLog batches;                             // 0: the lower levels; 1, 2: the upper ones
         for (int t = 0;; ++t) {
             if (!wait_warp(bTile + 8 * (t & 3), t >> 2, 3, t > 0 && slot[(t - 1) & 3].first ? 0 : 4096) ||
                 slot[t & 3].s < 0) break;
@@ -1546,6 +1554,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                 if (ok && lane == 0) oz_products(tmem, sa + h * kA, sb + h * kB, h, 3, kOzDigits);
             }
             if (lane == 0) oz_commit(bLo);
+            batches.start(0);
             if (t > 0) wait_warp(bHiFree, t - 1, 5);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (lane == 0) {
@@ -1553,8 +1562,11 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                     for (int h = 0; h < 2; ++h) oz_products(tmem, sa + h * kA, sb + h * kB, h, 0, 3);
                 oz_commit(bHi + 8 * (t & 1));
             }
+            batches.start(1 + (t & 1));
             __syncwarp();
         }
+        for (int b = 0; b < 3; ++b)
+            if (batches.any(b)) oz_wait(b == 0 ? bLo : bHi + 8 * (b - 1), batches.last_parity(b));
     } else {
         const int row = 32 * (wid & 3) + lane, ch = 32 * (wid >> 2);      // this thread's row and columns
         const uint32_t tl = tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch);
