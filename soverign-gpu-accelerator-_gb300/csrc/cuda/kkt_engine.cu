@@ -1401,7 +1401,8 @@ __device__ __forceinline__ int block_row_of(int lb) {
 // tile's half took 29,000 cycles: mean step at m = 4740 85 -> 69 us (there the diagonal tile is
 // the limit), of 40 LPs (54,000 rows) 161 -> 110 us. Waits are bounded: on a
 // time-out the block records err[2] and takes no further tile; at its end it waits, again with a
-// limit, for the copies and MMAs that it has issued, and frees its TMEM.
+// limit, for the copies and MMAs that it has issued, and frees its TMEM. The barriers of the
+// diagonal tile have no limit, so the eight warps go there together or not at all (join()).
 constexpr size_t kOzSmemU = kOzDigits * (2 * kOzA + 4 * kOzB) + 512;
 
 struct OzTile {
@@ -1424,7 +1425,8 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
     OzTile* slot = reinterpret_cast<OzTile*>(bars + 16);              // [4]
     uint32_t* tslot = reinterpret_cast<uint32_t*>(slot + 4);
     volatile int* fail = reinterpret_cast<volatile int*>(tslot + 1);
-    int* go = reinterpret_cast<int*>(tslot + 2);
+    int* joined = reinterpret_cast<int*>(tslot + 2);
+    static_assert(16 * 8 + 4 * sizeof(OzTile) + 12 <= 512, "kOzSmemU");
     // A's halves, B's buffers and halves, the slots' descriptions; a tile's lower sums done, an
     // even and an odd tile's upper ones (the copying warp may look after the next is done too),
     // their accumulators free again, the diagonal tile factored
@@ -1436,6 +1438,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bA + 8 * b), "r"(b < 13 ? 1 : 8));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *fail = *reinterpret_cast<volatile int*>(err + 2);   // an earlier step's time-out: no more tiles
+        *joined = 0;
     }
     if (wid == 8) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_addr(tslot)));
@@ -1570,10 +1573,18 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
     } else {
         const int row = 32 * (wid & 3) + lane, ch = 32 * (wid >> 2);      // this thread's row and columns
         const uint32_t tl = tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch);
-        for (int t = 0;; ++t) {
-            if (!wait_warp(bTile + 8 * (t & 3), t >> 2, 6)) break;
+        auto swap_joined = [&](int n, int v) {        // by lane 0, for the warp
+            int old = 0;
+            if (lane == 0) old = atomicCAS(joined, n, v);
+            return __shfl_sync(0xffffffffu, old, 0);
+        };
+        bool left = false;
+        for (int t = 0, tri = 0;; ++t) {
+            while (!left && !wait_warp(bTile + 8 * (t & 3), t >> 2, 6)) left = leave(tri, swap_joined);
+            if (left) break;
             const OzTile w = slot[t & 3];
             if (w.s < 0) break;
+            const bool tri_tile = w.first && join(tri++, swap_joined);
             const int r = w.r0 + row;
             // columns c0 + ch + j of row r for j < nj
             const int nj = r < w.N ? min(32, min(w.N, r + 1) - (w.c0 + ch)) : 0;
@@ -1652,10 +1663,10 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             store(3);
             if (w.first) {
                 __threadfence();                      // C, before the other warps read it
-                tile_sync();
-                if (tid == 0) *go = *fail == 0;
-                tile_sync();
-                if (*go) potrf_tile(w.s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
+                if (tri_tile) {
+                    tile_sync();
+                    potrf_tile(w.s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
+                }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // before A is copied there again
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bTri);

@@ -1,6 +1,7 @@
 """The failure path of the emulated-FP64 update without a GPU: which copies and MMA batches are
-still in flight when it gives up (cuda/oz_pipeline.hpp, run by a C++ program against a model of
-the barriers), and that the kernel waits for them."""
+still in flight when it gives up, and that its warps enter the diagonal tile together or not at
+all (cuda/oz_pipeline.hpp, run by a C++ program against a model of the barriers); and that the
+kernel keeps to both."""
 import json
 import os
 import re
@@ -10,9 +11,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "soverign-gpu-accelerator-_gb300", "csrc")
 
 
-def test_phases(tmp_path):
+def test_phases_and_joins(tmp_path):
     exe = os.path.join(str(tmp_path), "oz_pipeline")
-    p = subprocess.run(["g++", "-O1", "-std=c++17", "-I" + CSRC,
+    p = subprocess.run(["g++", "-O1", "-std=c++17", "-pthread", "-I" + CSRC,
                         os.path.join(HERE, "cpp", "oz_pipeline.cpp"), "-o", exe], capture_output=True, text=True)
     assert p.returncode == 0, p.stderr
     p = subprocess.run([exe], capture_output=True, text=True, timeout=300)
@@ -20,6 +21,7 @@ def test_phases(tmp_path):
     res = json.loads(p.stdout)
     assert res["failed"] == 0 and res["checks"] > 100000
     assert res["fixed_parity_leaves"] > 1000            # a wait with a fixed parity ends too early
+    assert res["together"] > 1000 and res["apart"] > 100
 
 
 def _kernel(name):
@@ -34,3 +36,7 @@ def test_the_kernel_waits_for_what_it_issued():
     assert body.count("oz_copy_rows(") == body.count("copies.start(") == 2
     assert body.count("oz_commit(") == body.count("batches.start(") == 2
     assert "copies.last_parity(b)" in body and "batches.last_parity(b)" in body
+    # the barriers without a limit are reached by all of the eight warps that joined, or by none
+    assert "bar.sync" not in body and body.count("tile_sync()") == body.count("potrf_tile(") == 1
+    assert re.search(r"if \(tri_tile\) \{\s*tile_sync\(\);\s*potrf_tile\(", body)
+    assert "tri_tile = w.first && join(" in body and "left = leave(" in body
