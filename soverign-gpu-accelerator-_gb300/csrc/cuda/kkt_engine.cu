@@ -1603,6 +1603,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             long long lo[32];
             {
+                __syncwarp();
                 uint32_t v[4 * 32];
 #pragma unroll
                 for (int L = 0; L < 4; ++L) {
@@ -1629,6 +1630,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             };
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
+                __syncwarp();                         // the TMEM loads take a converged warp
                 uint32_t v[3 * 8];
 #pragma unroll
                 for (int L = 0; L < 3; ++L) tmem_load8(v + 8 * L, tl + static_cast<uint32_t>(64 * L + 8 * g));
@@ -1676,6 +1678,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (wid == 8) {
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" :: "r"(tmem));
     }
@@ -1726,6 +1729,7 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
     const double* Li = Linv + inv_off[s] + static_cast<int64_t>(a.k) * T64 * T64;   // column-major 64 x 64
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     if (wid == 0) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(smem_addr(tslot)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -1794,6 +1798,7 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
         const int er = ea[row];
 #pragma unroll
         for (int c8 = 0; c8 < 2; ++c8) {
+            __syncwarp();                              // the TMEM loads take a converged warp
             long long u[8];
             oz_read8(tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch + 8 * c8), u);
             bool any = false;
@@ -1803,9 +1808,12 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
                 any |= !oz_plain(e);
                 v[8 * c8 + q] = oz_value(u[q], e, any);
             }
-            if (any)
+            if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
-                for (int q = 0; q < 8; ++q) v[8 * c8 + q] = oz_value_any(u[q], er + eb[ch + 8 * c8 + q] - 52);
+                for (int q = 0; q < 8; ++q)
+                    if (any) v[8 * c8 + q] = oz_value_any(u[q], er + eb[ch + 8 * c8 + q] - 52);
+                __syncwarp();
+            }
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int j = 8 * c8 + q, col = ch + j;
@@ -1819,6 +1827,7 @@ __global__ void __launch_bounds__(512, 1) k_panel_oz(StepArgs a, const int* __re
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (wid == 0) {
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" :: "r"(tmem));
     }
@@ -1937,6 +1946,7 @@ __global__ void __launch_bounds__(256, 2) k_update_tcs(StepArgs a, const int* __
                          :: "r"(smem_addr(dst[c])), "l"(src[c]), "r"(len[c]), "r"(b0) : "memory");
     }
     if (wid == 0) {
+        __syncwarp();                                  // thread 0 has been on its own
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" :: "r"(smem_addr(tslot)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -1991,6 +2001,7 @@ __global__ void __launch_bounds__(256, 2) k_update_tcs(StepArgs a, const int* __
     if (ok) {
 #pragma unroll
         for (int c16 = 0; c16 < 2; ++c16) {
+            __syncwarp();                              // the TMEM loads take a converged warp
             uint32_t v[16];
             const uint32_t taddr = tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) +
                                    static_cast<uint32_t>(ch + 16 * c16);
@@ -2011,6 +2022,7 @@ __global__ void __launch_bounds__(256, 2) k_update_tcs(StepArgs a, const int* __
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (wid == 0) {
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" :: "r"(tmem));
     }
