@@ -585,35 +585,34 @@ __global__ void k_adam(int n, float* __restrict__ w, const float* __restrict__ g
 }
 
 // Launches of the layer kernels: 16 nodes a block while that leaves at most four blocks per
-// SM, then 32 (half the weight loads per node). 5000 nodes: 16 a block.
-constexpr int kSms = 152;
-inline bool wide_layer(int nodes) { return nodes > kSms * 4 * 16; }
-inline int layer_blocks(int nodes, int per) { return std::min((nodes + per - 1) / per, kSms * 4); }
+// SM, then 32 (half the weight loads per node). 5000 nodes on 152 SMs: 16 a block.
+inline bool wide_layer(int nodes, int sms) { return nodes > sms * 4 * 16; }
+inline int layer_blocks(int nodes, int per, int sms) { return std::min((nodes + per - 1) / per, sms * 4); }
 
 void layer_forward(const Side& side, const float* inv_deg, const float* other, const float* x1, const uint16_t* W1,
-                   const uint16_t* W2, const uint16_t* b, float* mout, float* out, cudaStream_t st) {
-    if (wide_layer(side.nodes))
-        k_layer<2><<<layer_blocks(side.nodes, 32), 256, layer_smem(32, 2), st>>>(side, inv_deg, other, x1, W1, W2, b,
-                                                                                 mout, out);
+                   const uint16_t* W2, const uint16_t* b, float* mout, float* out, int sms, cudaStream_t st) {
+    if (wide_layer(side.nodes, sms))
+        k_layer<2><<<layer_blocks(side.nodes, 32, sms), 256, layer_smem(32, 2), st>>>(side, inv_deg, other, x1, W1,
+                                                                                      W2, b, mout, out);
     else
-        k_layer<1><<<layer_blocks(side.nodes, 16), 256, layer_smem(16, 2), st>>>(side, inv_deg, other, x1, W1, W2, b,
-                                                                                 mout, out);
+        k_layer<1><<<layer_blocks(side.nodes, 16, sms), 256, layer_smem(16, 2), st>>>(side, inv_deg, other, x1, W1,
+                                                                                      W2, b, mout, out);
 }
 
 template <bool Gather>
 void layer_backward(const Side& side, const float* scale_in, const float* src, float* d, const float* y,
-                    const uint16_t* W1, const uint16_t* W2, float* dx1, float* dx2, cudaStream_t st) {
-    if (wide_layer(side.nodes))
-        k_layer_bwd<Gather, 2><<<layer_blocks(side.nodes, 32), 256, layer_smem(32, 1), st>>>(side, scale_in, src, d, y,
-                                                                                             W1, W2, dx1, dx2);
+                    const uint16_t* W1, const uint16_t* W2, float* dx1, float* dx2, int sms, cudaStream_t st) {
+    if (wide_layer(side.nodes, sms))
+        k_layer_bwd<Gather, 2><<<layer_blocks(side.nodes, 32, sms), 256, layer_smem(32, 1), st>>>(
+            side, scale_in, src, d, y, W1, W2, dx1, dx2);
     else
-        k_layer_bwd<Gather, 1><<<layer_blocks(side.nodes, 16), 256, layer_smem(16, 1), st>>>(side, scale_in, src, d, y,
-                                                                                             W1, W2, dx1, dx2);
+        k_layer_bwd<Gather, 1><<<layer_blocks(side.nodes, 16, sms), 256, layer_smem(16, 1), st>>>(
+            side, scale_in, src, d, y, W1, W2, dx1, dx2);
 }
 
 void grad_weights(int nodes, const float* g, const float* x1, const float* x2, float* dW1, float* dW2, float* db,
-                  cudaStream_t st) {
-    const int chunk = std::max(64, ((nodes + kSms - 1) / kSms + 31) / 32 * 32);
+                  int sms, cudaStream_t st) {
+    const int chunk = std::max(64, ((nodes + sms - 1) / sms + 31) / 32 * 32);
     k_grad_w<<<(nodes + chunk - 1) / chunk, 256, 0, st>>>(nodes, chunk, g, x1, x2, dW1, dW2, db);
 }
 
@@ -623,13 +622,16 @@ inline int nb(int64_t n, int t = 256) { return static_cast<int>((n + t - 1) / t)
 
 Gnn::Gnn(unsigned long long seed) {
     nparams_ = kLay.total;
+    int device = 0;
+    SK_CUDA(cudaGetDevice(&device));
+    SK_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device));
     SK_CUDA(cudaMalloc(&master_, sizeof(float) * nparams_));
     SK_CUDA(cudaMalloc(&wbf_, sizeof(uint16_t) * nparams_));
     SK_CUDA(cudaMalloc(&grad_, sizeof(float) * nparams_));
     SK_CUDA(cudaMalloc(&adam_m_, sizeof(float) * nparams_));
     SK_CUDA(cudaMalloc(&adam_v_, sizeof(float) * nparams_));
     SK_CUDA(cudaMalloc(&loss_, sizeof(double)));
-    SK_CUDA(cudaMallocHost(&loss_host_, sizeof(double)));
+    loss_host_.alloc(1);
     SK_CUDA(cudaEventCreateWithFlags(&loss_ready_, cudaEventDisableTiming));
     for (auto* f : {k_layer<1>, k_layer<2>})
         SK_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -670,7 +672,6 @@ Gnn::~Gnn() {
                     static_cast<void*>(dr_), static_cast<void*>(dm_), static_cast<void*>(dt_),
                     static_cast<void*>(inv_deg_r_), static_cast<void*>(inv_deg_c_)})
         if (p) cudaFree(p);
-    if (loss_host_) cudaFreeHost(loss_host_);
     if (loss_ready_) cudaEventDestroy(loss_ready_);
 }
 
@@ -725,9 +726,9 @@ void Gnn::forward(const DeviceLP& lp, cudaStream_t st, double* out_logx, double*
         float* hcl = hc_ + l * NH;
         float* hrl = hr_ + l * MH;
         layer_forward(rows, inv_deg_r_, hcl, hrl, w + kLay.Wrr[l], w + kLay.Wrm[l], w + kLay.br[l],
-                      keep ? mr_ + l * MH : nullptr, hrl + MH, st);
+                      keep ? mr_ + l * MH : nullptr, hrl + MH, sms_, st);
         layer_forward(cols, inv_deg_c_, hrl + MH, hcl, w + kLay.Wcc[l], w + kLay.Wcm[l], w + kLay.bc[l],
-                      keep ? mc_ + l * NH : nullptr, hcl + NH, st);
+                      keep ? mc_ + l * NH : nullptr, hcl + NH, sms_, st);
     }
     k_heads<<<all, 256, 0, st>>>(N, M, hc_ + L * NH, hr_ + L * MH, w + kLay.Hc, w + kLay.oc, w + kLay.Hr,
                                  w + kLay.orr, oc_, or_, out_logx, out_logs, out_y);
@@ -736,13 +737,13 @@ void Gnn::forward(const DeviceLP& lp, cudaStream_t st, double* out_logx, double*
     SK_CUDA(cudaMemsetAsync(loss_, 0, sizeof(double), st));
     // d_oc -> dm_ (N x 2), d_or -> dt_ (M)
     k_loss<<<nb(static_cast<int64_t>(N) + M), 256, 0, st>>>(N, M, oc_, or_, t_logx, t_logs, t_y, dm_, dt_, loss_);
-    SK_CUDA(cudaMemcpyAsync(loss_host_, loss_, sizeof(double), cudaMemcpyDeviceToHost, st));
+    SK_CUDA(cudaMemcpyAsync(loss_host_.ptr, loss_, sizeof(double), cudaMemcpyDeviceToHost, st));
     SK_CUDA(cudaEventRecord(loss_ready_, st));
 }
 
 double Gnn::loss() const {
     SK_CUDA(cudaEventSynchronize(loss_ready_));
-    return *loss_host_;
+    return *loss_host_.ptr;
 }
 
 void Gnn::backward(const DeviceLP& lp, cudaStream_t st, float* grad_host) {
@@ -768,15 +769,16 @@ void Gnn::backward(const DeviceLP& lp, cudaStream_t st, float* grad_host) {
         // (mr[l+1] = diag(inv_deg_r) A hc[l+1]); d mc[l] -> dm_
         if (l == L - 1)
             layer_backward<false>(cols, nullptr, nullptr, dhc, hcl + NH, w + kLay.Wcc[l], w + kLay.Wcm[l], dhc2, dm_,
-                                  st);
+                                  sms_, st);
         else
             layer_backward<true>(cols, inv_deg_r_, dt_, dhc, hcl + NH, w + kLay.Wcc[l], w + kLay.Wcm[l], dhc2, dm_,
-                                 st);
-        grad_weights(N, dhc, hcl, mc_ + l * NH, gr + kLay.Wcc[l], gr + kLay.Wcm[l], gr + kLay.bc[l], st);
+                                 sms_, st);
+        grad_weights(N, dhc, hcl, mc_ + l * NH, gr + kLay.Wcc[l], gr + kLay.Wcm[l], gr + kLay.bc[l], sms_, st);
         // hr[l+1] = relu(Wrr hr[l] + Wrm mr[l] + br), and mc[l] = diag(inv_deg_c) A^T hr[l+1];
         // d mr[l] -> dt_
-        layer_backward<true>(rows, inv_deg_c_, dm_, dhr, hrl + MH, w + kLay.Wrr[l], w + kLay.Wrm[l], dhr2, dt_, st);
-        grad_weights(M, dhr, hrl, mr_ + l * MH, gr + kLay.Wrr[l], gr + kLay.Wrm[l], gr + kLay.br[l], st);
+        layer_backward<true>(rows, inv_deg_c_, dm_, dhr, hrl + MH, w + kLay.Wrr[l], w + kLay.Wrm[l], dhr2, dt_,
+                             sms_, st);
+        grad_weights(M, dhr, hrl, mr_ + l * MH, gr + kLay.Wrr[l], gr + kLay.Wrm[l], gr + kLay.br[l], sms_, st);
         std::swap(dhc, dhc2);
         std::swap(dhr, dhr2);
     }

@@ -60,8 +60,9 @@ private:
     float *oc_ = nullptr, *or_ = nullptr;                 // N x 2, M x 1
     float *dc_ = nullptr, *dr_ = nullptr, *dm_ = nullptr, *dt_ = nullptr;  // gradient work
     float *inv_deg_r_ = nullptr, *inv_deg_c_ = nullptr;
+    int sms_ = 0;                     // of the device
     double* loss_ = nullptr;
-    double* loss_host_ = nullptr;     // pinned
+    Pinned<double> loss_host_;
     cudaEvent_t loss_ready_ = nullptr;
 };
 

@@ -16,20 +16,6 @@
 namespace sankhya {
 namespace dev {
 
-// Page-locked host memory: a copy to or from pageable memory goes through the driver's staging
-// buffer and costs about as much again as a small kernel.
-template <class T>
-struct Pinned {
-    T* ptr = nullptr;
-    void alloc(size_t n) { SK_CUDA(cudaMallocHost(&ptr, n * sizeof(T))); }
-    Pinned() = default;
-    Pinned(const Pinned&) = delete;
-    Pinned& operator=(const Pinned&) = delete;
-    ~Pinned() {
-        if (ptr) cudaFreeHost(ptr);
-    }
-};
-
 struct PlanDev;
 
 class KktEngine {
