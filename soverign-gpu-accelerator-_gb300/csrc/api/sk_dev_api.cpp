@@ -76,6 +76,7 @@ struct sk_kkt {
     std::unique_ptr<dev::KktEngine> eng;
     bool factored = false;
     ~sk_kkt() {
+        if (st) cudaStreamSynchronize(st);       // nothing uses pin any more
         eng.reset();
         if (st) cudaStreamDestroy(st);
     }

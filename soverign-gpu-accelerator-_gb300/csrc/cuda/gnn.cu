@@ -672,7 +672,10 @@ Gnn::~Gnn() {
                     static_cast<void*>(dr_), static_cast<void*>(dm_), static_cast<void*>(dt_),
                     static_cast<void*>(inv_deg_r_), static_cast<void*>(inv_deg_c_)})
         if (p) cudaFree(p);
-    if (loss_ready_) cudaEventDestroy(loss_ready_);
+    if (loss_ready_) {
+        cudaEventSynchronize(loss_ready_);                    // nothing uses loss_host_ any more
+        cudaEventDestroy(loss_ready_);
+    }
 }
 
 void Gnn::get_params(float* out) const {

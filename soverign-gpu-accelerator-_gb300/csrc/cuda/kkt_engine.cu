@@ -2820,6 +2820,7 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
 }
 
 KktEngine::~KktEngine() {
+    cudaStreamSynchronize(st_);                  // nothing uses host_flags_ any more
     for (int q = 0; q < 2; ++q)
         if (fev_[q]) cudaEventDestroy(fev_[q]);
     for (int q = 0; q < 4; ++q)
