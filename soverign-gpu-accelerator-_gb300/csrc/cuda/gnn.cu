@@ -218,7 +218,8 @@ __global__ void __launch_bounds__(256, NPT == 1 ? 3 : 4) k_layer(Side side, cons
             const size_t at = static_cast<size_t>(node) * (H / 4) + (lane & 15);
             float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
             if (on) x = reinterpret_cast<const float4*>(x1)[at];
-            float4 m = gather_row<NPT == 1 ? 8 : 4>(on ? side.rp[node] : 0, on ? side.rp[node + 1] : 0, side.ci, side.v, nullptr, other);
+            float4 m = gather_row<NPT == 1 ? 8 : 4>(on ? side.rp[node] : 0, on ? side.rp[node + 1] : 0, side.ci,
+                                                    side.v, nullptr, other);
             const float so = on ? inv_deg[node] : 0.f;
             m = make_float4(so * m.x, so * m.y, so * m.z, so * m.w);
             if (on && mout) reinterpret_cast<float4*>(mout)[at] = m;
@@ -393,8 +394,8 @@ __global__ void __launch_bounds__(256, NPT == 1 ? 3 : 4) k_layer_bwd(Side side, 
                 yv = reinterpret_cast<const float4*>(y)[at];
             }
             if (Gather) {
-                const float4 m = gather_row<NPT == 1 ? 8 : 4>(on ? side.rp[node] : 0, on ? side.rp[node + 1] : 0, side.ci, side.v,
-                                            scale_in, src);
+                const float4 m = gather_row<NPT == 1 ? 8 : 4>(on ? side.rp[node] : 0, on ? side.rp[node + 1] : 0,
+                                                              side.ci, side.v, scale_in, src);
                 g = make_float4(g.x + m.x, g.y + m.y, g.z + m.z, g.w + m.w);
             }
             g = mask_positive(g, yv);
@@ -465,8 +466,8 @@ __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const floa
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int e = tid + 256 * (u & 1), node = n + (e >> 4);
-            px[u] = node < n1 ? reinterpret_cast<const float4*>(u < 2 ? x1 : x2)[static_cast<size_t>(node) * 16 + (e & 15)]
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4* x = reinterpret_cast<const float4*>(u < 2 ? x1 : x2);
+            px[u] = node < n1 ? x[static_cast<size_t>(node) * 16 + (e & 15)] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
     load(n0);
@@ -552,8 +553,8 @@ __global__ void __launch_bounds__(256) k_embed_bwd(EmbedGrad cols, EmbedGrad row
             for (int k = 0; k < 3; ++k) f[k] = e.f[node * 3 + k];
         }
         if (col) {
-            const float4 m = gather_row<4>(on ? side.rp[node] : 0, on ? side.rp[node + 1] : 0, side.ci, side.v, scale_in,
-                                        src);
+            const float4 m = gather_row<4>(on ? side.rp[node] : 0, on ? side.rp[node + 1] : 0, side.ci, side.v,
+                                           scale_in, src);
             g = make_float4(g.x + m.x, g.y + m.y, g.z + m.z, g.w + m.w);
         }
         g = mask_positive(g, y);

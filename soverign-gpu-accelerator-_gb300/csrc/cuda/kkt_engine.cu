@@ -2,15 +2,23 @@
 //
 // Kernels, in the order one factorisation + solve runs them:
 //   assembly    k_asm_*          D (A Theta A^T) D + delta I into the fronts
-//   factor      k_potrf          Cholesky of one 64x64 diagonal tile per front
-//               k_trsm           panel rows below the tile: X L^T = B
-//               k_update         trailing update C -= L_i L_j^T (tiles of 64x64)
+//   factor      k_potrf          Cholesky and inverse of a level's first 64x64 diagonal tiles; later
+//                                ones are factored by the update before them (potrf_tile)
+//               panel rows below the tile, X = B Linv^T:
+//               k_trsm           FP32
+//               k_trsm_rows      FP64 on the FP64 pipe
+//               k_panel_oz       FP64 with BF16 digits on the tensor cores
+//               trailing update C -= X_i X_j^T:
+//               k_tc_split, k_update_tcs  FP32 on the tensor cores (TF32 x3); k_update without
+//               k_update_split   FP64 on the FP64 pipe
+//               k_update_oz      FP64 with BF16 digits on the tensor cores
 //               k_extend_add     child update matrix into the parent front
 //   solve       k_fwd_gather     frontal right-hand sides of one level
 //               k_fwd_tasks      L z = r, dependency-driven 64-row block tasks
 //               k_bwd_tasks      L^T x = z, same scheme in reverse
-// Factorisation grids are lists of (front, tile) work items of one level / step,
-// decoded with a binary search over a prefix of per-front tile counts.
+//   products    k_row_sums       A Theta A^T x and residuals
+// Factorisation grids are lists of (front, tile) work items of one level / step, decoded by a
+// warp-wide search over a prefix of per-front tile counts (find_item).
 #include "cuda/kkt_engine.hpp"
 
 #include "cuda/oz_pipeline.hpp"
@@ -282,8 +290,8 @@ __global__ void k_asm_cols_dense(int M, const int* __restrict__ rp, const int* _
 // triangular solves), stored column-major in Linv. A partial tile is padded with the
 // identity. This runs in one block on the critical path of every 64-column step, by blocks
 // of 16 columns: the 16x16 diagonal block, the rows below it, the trailing update. Every
-// entry keeps its own ascending sequence of fused multiply-adds and correctly rounded roots
-// and reciprocals, so the result does not depend on how the work is dealt out:
+// entry keeps its own ascending sequence of fused multiply-adds, roots and reciprocals, so the
+// result does not depend on how the work is dealt out:
 //  * FP32 is bound by the latency of the pivot chain, FP64 also by the SM's FP64 pipe: a
 //    warp's FP64 instruction takes 64 cycles of its SM quarter whatever its active lanes, a
 //    dependent one follows at once, and shuffles and shared loads queue with it (measured:
@@ -303,12 +311,24 @@ constexpr int kPBTri = kPB * (kPB + 1) / 2;
 // pivot, or left a loop early, may still be on its own.
 // The barrier of the warps that extend the inverse, and the one on which the others wait for
 // its block row.
-__device__ __forceinline__ void inverse_sync(int threads) { __syncwarp(); asm volatile("bar.sync 1, %0;" :: "r"(threads) : "memory"); }
-__device__ __forceinline__ void inverse_arrive() { __syncwarp(); asm volatile("bar.arrive 2, 224;" ::: "memory"); }
-__device__ __forceinline__ void inverse_wait() { __syncwarp(); asm volatile("bar.sync 2, 224;" ::: "memory"); }
+__device__ __forceinline__ void inverse_sync(int threads) {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" :: "r"(threads) : "memory");
+}
+__device__ __forceinline__ void inverse_arrive() {
+    __syncwarp();
+    asm volatile("bar.arrive 2, 224;" ::: "memory");
+}
+__device__ __forceinline__ void inverse_wait() {
+    __syncwarp();
+    asm volatile("bar.sync 2, 224;" ::: "memory");
+}
 
-// The 256 threads of a diagonal tile (the update's block has one more warp).
-__device__ __forceinline__ void tile_sync() { __syncwarp(); asm volatile("bar.sync 3, 256;" ::: "memory"); }
+// The 256 threads of a diagonal tile (the emulated update's block has two more warps).
+__device__ __forceinline__ void tile_sync() {
+    __syncwarp();
+    asm volatile("bar.sync 3, 256;" ::: "memory");
+}
 
 __device__ __noinline__ void report_pivot(int s, const PlanDev& pd, int* err) {
     if ((threadIdx.x & 31) != 0) return;
@@ -342,9 +362,10 @@ __device__ __forceinline__ void pivot_root(float p, float& d, float& rd, Fill fi
 // FP64: y ~ p^(-1/2) to about 2^-45 without the FP64 pipe: the mantissa m in [1, 4) as two
 // floats, the approximate unit's seed y0, e = 1 - m y0^2 with the square's low part, and one
 // third-order step, whose correction is added to y0's bits as an integer. Then d0 = p y, the
-// residual corrections d = d0 + (p - d0^2) y / 2 and rd = y + (1 - d y) y (Markstein 1990),
-// whose last rounding is the correct one unless the exact value lies within about 2^-90 of a
-// rounding boundary.
+// residual corrections d = d0 + (p - d0^2) y / 2 and rd = y + (1 - d y) y (Markstein 1990).
+// Their last rounding is the correct one unless the exact value lies within about 2^-90 of a
+// rounding boundary, where it may be the other neighbour: the reciprocal of 1 - j 2^-53, j odd
+// and small, lies j^2 2^-106 from one and comes out a place low.
 template <class Fill>
 __device__ __forceinline__ void pivot_root(double p, double& d, double& rd, Fill fill) {
     const int hi = __double2hiint(p), lo = __double2loint(p);
@@ -404,7 +425,8 @@ __device__ __noinline__ bool factor_rest(T* A, T* rdiag, int c0, int j) {
 }
 
 // Warp 0: the diagonal block at c0. Leaves L in A and 1 / L(c, c) in rdiag. Result: a pivot was
-// not positive (it counts as 1). FP32: lane (r, h) holds the columns 2k + h of row r. Column j updates column j + 1 at once and the others while the next pivot's root forms.
+// not positive (it counts as 1). FP32: lane (r, h) holds the columns 2k + h of row r. Column j
+// updates column j + 1 at once and the others while the next pivot's root forms.
 __device__ __forceinline__ bool factor_block(float* A, float* rdiag, int c0) {
     const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
     float v[8];
@@ -789,7 +811,7 @@ __global__ void __launch_bounds__(256) k_potrf(StepArgs a, const int* __restrict
     potrf_tile(s, a.k, pd, F, Linv, inv_off, err, smraw);
 }
 
-// Panel rows below the diagonal tile: X = B L_kk^{-float} = B Linv^float (a small GEMM).
+// FP32 panel rows below the diagonal tile: X = B L_kk^{-T} = B Linv^T (a small GEMM).
 __global__ void __launch_bounds__(256) k_trsm(StepArgs a, const int* __restrict__ items,
                                               const int* __restrict__ prefix, PlanDev pd, float* F,
                                               const float* __restrict__ Linv, const int64_t* __restrict__ inv_off) {
@@ -1393,9 +1415,11 @@ __device__ __forceinline__ int block_row_of(int lb) {
 // two buffers). Warp 9 fetches tiles and copies, warp 8 issues the MMAs, warps 0..7 take the
 // sums from TMEM (448 columns) to C, 32 columns a thread. The lower levels are multiplied
 // first: their accumulators are free for the next tile as soon as they are in registers, while
-// the upper levels' products run. Bound by the epilogue: of an SM quarter 5,500 cycles of
-// integer instructions a tile, 4,100 of FP64 subtractions, 3,700 of conversions, so these are
-// kept apart in neighbouring groups of columns and have no branch between them. The block
+// the upper levels' products run. Bound by the epilogue: of the 16,000 cycles that a tile takes
+// at 3,260 rows an SM quarter's FP64 subtractions need 4,100 (64 cycles an instruction), its integer
+// instructions 4,600 and its conversions 2,600, one after the other in each warp, so these are kept
+// apart in neighbouring groups of columns and have no branch between them; the tensor pipe is busy
+// for 22% of the time. The block
 // with a front's first tile factors the next diagonal tile and waits for it without polling.
 // As 128 x 32 tiles of blocks that copied, multiplied and subtracted in turn, two on an SM, a
 // tile's half took 29,000 cycles: mean step at m = 4740 85 -> 69 us (there the diagonal tile is
@@ -2606,15 +2630,22 @@ inline int blocks_for(int64_t n, int t) { return static_cast<int>((n + t - 1) / 
 // ------------------------------------------------------------------ engine
 
 // FP64 updates of fewer 64x64 tiles than this take 16x16 parts (about two waves of the 152
-// SMs): m = 500 LP 16.5 ms, with 32x32 parts from 12 tiles on 16.8 ms.
+// SMs): m = 500 LP 16.5 ms, with 32x32 parts from 12 tiles on 16.8 ms; one front of 130 rows 257 us
+// with 32x32 parts, 232 with these. It counts the tiles of all fronts together, and several fronts
+// with that few would rather have 32x32 parts (ten fronts of 100 rows 198 us, 181 with those; 16
+// of 512 rows 1157, 1101).
 constexpr int kSplit16Tiles = 24;
 // Fewer tiles than this run one block per SM, so that the next diagonal tile has an SM to
-// itself: m = 1447 3.12 -> 2.89 ms; with 800 here m = 4001 loses 1 %.
+// itself: m = 1447 3.12 -> 2.89 ms; with 800 here m = 4001 loses 1 %. With many fronts, too: 40 of
+// 100 rows 232 -> 194 us, 100 of 192 rows 558 -> 508, 60 of 320 rows 1031 -> 992, the same from
+// 150 fronts of 100 rows on.
 constexpr int kAloneTiles = 300;
 // Panel solves of fewer 64-row units than this take 8 rows a block instead of 16: m = 500
-// LP 17.5 -> 16.0 ms, one warp then has an SM quarter to itself; more blocks than SMs only
-// load the diagonal tile more often.
+// LP 17.5 -> 16.0 ms, one front of 130 rows 243 -> 232 us, one warp then has an SM quarter to
+// itself; more blocks than SMs only load the diagonal tile more often (10 to 400 fronts of 100 to
+// 700 rows: the same either way, within 2 %).
 constexpr int kTr4Tiles = 76;
+
 struct KktEngine::Prof {
     cudaStream_t st;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> ev;
@@ -2786,7 +2817,9 @@ KktEngine::KktEngine(const ipm::FrontPlan& plan, const DeviceLP& lp, cudaStream_
     bnd(ch_list_); bnd(perm_); bnd(sn_F_off_); bnd(sn_f_off_); bnd(sn_rows_off_); bnd(ea_off_); bnd(step_items_);
     bnd(step_prefix_); bnd(round_items_); bnd(round_prefix_); bnd(level_sn_); bnd(slot_pos_); bnd(w_ptr_);
     bnd(slot_i_); bnd(slot_j_); bnd(w_col_); bnd(w_val_); bnd(inv_off_); bnd(fwd_tasks_);
-    bnd(bwd_tasks_); bnd(g_dst_); bnd(g_zp_); bnd(g_ptr_); bnd(g_src_); bnd(sn_lp_); bnd(on32_); bnd(on64_); bnd(q_lp_); bnd(zc_sn_); bnd(zc_len_); bnd(zc_off_); bnd(counters_); bnd(solve_err_); bnd(D_); bnd(Mdiag_);
+    bnd(bwd_tasks_); bnd(g_dst_); bnd(g_zp_); bnd(g_ptr_); bnd(g_src_); bnd(sn_lp_); bnd(on32_);
+    bnd(on64_); bnd(q_lp_); bnd(zc_sn_); bnd(zc_len_); bnd(zc_off_); bnd(counters_); bnd(solve_err_); bnd(D_);
+    bnd(Mdiag_);
     bnd(zp_); bnd(xp_); bnd(zsol_); bnd(fvec_); bnd(tn_); bnd(params_); bnd(err_); bnd(lp_fail_); bnd(oz_cnt_);
     for (auto& sb : sub_) { bnd(sb.d_items); bnd(sb.d_prefix); }
     upload(sn_first_, p.sn_first, st_); upload(sn_ncols_, p.sn_ncols, st_); upload(sn_nrows_, p.sn_nrows, st_);
@@ -2922,14 +2955,15 @@ void KktEngine::launch_factor(T* F, T* Linv, Prof* prof, const SubSteps* sub) {
                     if (tc) return;
                     const int tiles = static_cast<int>(st.upd_tiles);
                     if constexpr (std::is_same<T, float>::value)
-                        k_update<<<st.nitems + tiles, 256, potrf_smem(sizeof(T)), st_>>>(a, items, prefix, pdv, F, Linv,
-                                                                             inv_off_.ptr, err_.ptr);
+                        k_update<<<st.nitems + tiles, 256, potrf_smem(sizeof(T)), st_>>>(
+                            a, items, prefix, pdv, F, Linv, inv_off_.ptr, err_.ptr);
                     else if (tiles < kSplit16Tiles)
-                        k_update_split<16><<<(st.nitems + tiles) * 16, 256, split_smem<16>(), st_>>>(a, items, prefix, pdv, F, Linv,
-                                                                                       inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
+                        k_update_split<16><<<(st.nitems + tiles) * 16, 256, split_smem<16>(), st_>>>(
+                            a, items, prefix, pdv, F, Linv, inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
                     else
-                        k_update_split<32><<<(st.nitems + tiles) * 4, 256, tiles < kAloneTiles ? kSplitAlone : split_smem<32>(),
-                                             st_>>>(a, items, prefix, pdv, F, Linv, inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
+                        k_update_split<32><<<(st.nitems + tiles) * 4, 256,
+                                             tiles < kAloneTiles ? kSplitAlone : split_smem<32>(), st_>>>(
+                            a, items, prefix, pdv, F, Linv, inv_off_.ptr, oz_cnt_.ptr, err_.ptr);
                 });
                 if (prof) {
                     for (int it = 0; it < st.nitems; ++it) {
