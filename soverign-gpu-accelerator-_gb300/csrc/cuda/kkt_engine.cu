@@ -1425,7 +1425,7 @@ __device__ __forceinline__ int block_row_of(int lb) {
 // tile's half took 29,000 cycles: mean step at m = 4740 85 -> 69 us (there the diagonal tile is
 // the limit), of 40 LPs (54,000 rows) 161 -> 110 us. Waits are bounded: on a
 // time-out the block records err[2] and takes no further tile; at its end it waits, again with a
-// limit, for the copies and MMAs that it has issued, and frees its TMEM. The barriers of the
+// limit, for the copies and MMAs that it has in flight, and frees its TMEM. The barriers of the
 // diagonal tile have no limit, so the eight warps go there together or not at all (join()).
 constexpr size_t kOzSmemU = kOzDigits * (2 * kOzA + 4 * kOzB) + 512;
 
@@ -1494,6 +1494,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
         __syncwarp();
         return done;
     };
+    PhaseLog issued;      // by warp 9: copies, on A's (0, 1) and B's (2 .. 5) barriers; by warp 8: batches, on bLo, bHi
     if (wid == 9) {
         const int* up = prefix + a.up3_off;
         const int grid = gridDim.x, total = a.nitems + up[a.nitems];
@@ -1501,7 +1502,6 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
         int item = -1, rows = -1;                     // whose rows are in As
         int tri = 0;
         bool first = false;                           // the tile before was a first one
-        PhaseLog copies;                              // barriers 0, 1: A; 2 .. 5: B
         for (int t = 0;; ++t) {
             // the diagonal tile needs the SM's issue slots: no polling beside it
             if (first) wait_warp(bTri, tri++, 2, 0);
@@ -1544,14 +1544,14 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             if (ok)
                 for (int h = 0; h < 2; ++h) {
                     oz_copy_rows(h, bB + 16 * buf + 8 * h, Bs + (2 * buf + h) * kB, dig, plane, w.qb, 64);
-                    copies.start(2 + 2 * buf + h);
+                    issued.start(2 + 2 * buf + h);
                 }
             if (ok && w.fresh) {
                 if (t > 0) ok = wait_async(bHi + 8 * (buf ^ 1), (t - 1) >> 1);                // nor are A's rows
                 if (ok)
                     for (int h = 0; h < 2; ++h) {
                         oz_copy_rows(h, bA + 8 * h, As + h * kA, dig, plane, w.qa, 128);
-                        copies.start(h);
+                        issued.start(h);
                     }
             }
             if (!ok) w.s = -1;
@@ -1562,12 +1562,9 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             }
             if (!ok) break;
         }
-        for (int b = 0; b < 6; ++b)                   // none is in flight when the block ends
-            if (copies.any(b)) oz_wait(bA + 8 * b, copies.last_parity(b));
     } else if (wid == 8) {
         const uint32_t sa = smem_addr(As);
         int na = 0;
-        PhaseLog batches;                             // 0: the lower levels; 1, 2: the upper ones
         for (int t = 0;; ++t) {
             if (!wait_warp(bTile + 8 * (t & 3), t >> 2, 3, t > 0 && slot[(t - 1) & 3].first ? 0 : 4096) ||
                 slot[t & 3].s < 0) break;
@@ -1581,7 +1578,7 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                 if (ok && lane == 0) oz_products(tmem, sa + h * kA, sb + h * kB, h, 3, kOzDigits);
             }
             if (lane == 0) oz_commit(bLo);
-            batches.start(0);
+            issued.start(0);
             if (t > 0) wait_warp(bHiFree, t - 1, 5);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (lane == 0) {
@@ -1589,11 +1586,9 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                     for (int h = 0; h < 2; ++h) oz_products(tmem, sa + h * kA, sb + h * kB, h, 0, 3);
                 oz_commit(bHi + 8 * (t & 1));
             }
-            batches.start(1 + (t & 1));
+            issued.start(1 + (t & 1));
             __syncwarp();
         }
-        for (int b = 0; b < 3; ++b)
-            if (batches.any(b)) oz_wait(b == 0 ? bLo : bHi + 8 * (b - 1), batches.last_parity(b));
     } else {
         const int row = 32 * (wid & 3) + lane, ch = 32 * (wid >> 2);      // this thread's row and columns
         const uint32_t tl = tmem + (static_cast<uint32_t>(32 * (wid & 3)) << 16) + static_cast<uint32_t>(ch);
@@ -1608,7 +1603,6 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             if (left) break;
             const OzTile w = slot[t & 3];
             if (w.s < 0) break;
-            const bool tri_tile = w.first && join(tri++, swap_joined);
             const int r = w.r0 + row;
             // columns c0 + ch + j of row r for j < nj
             const int nj = r < w.N ? min(32, min(w.N, r + 1) - (w.c0 + ch)) : 0;
@@ -1627,7 +1621,6 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             long long lo[32];
             {
-                __syncwarp();
                 uint32_t v[4 * 32];
 #pragma unroll
                 for (int L = 0; L < 4; ++L) {
@@ -1645,7 +1638,10 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int last = *fail == 0 ? nj : 0;
             // Eight columns at a time; their subtractions are issued between the integer work of
-            // the next eight, which they would otherwise wait for and hold up.
+            // the next eight, which they would otherwise wait for and hold up. The vote at the end
+            // of each comes after every access that is not the same for all lanes: it brings the
+            // warp together for the next TMEM loads, which take a converged one (a __syncwarp before
+            // them instead cost the 512-LP batch 0.8 %).
             double x[2][8];
             auto store = [&](int g) {
 #pragma unroll
@@ -1654,11 +1650,11 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
             };
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                __syncwarp();                         // the TMEM loads take a converged warp
                 uint32_t v[3 * 8];
 #pragma unroll
                 for (int L = 0; L < 3; ++L) tmem_load8(v + 8 * L, tl + static_cast<uint32_t>(64 * L + 8 * g));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (g == 1) load_c(1);
                 if (g == 3) {
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
@@ -1682,14 +1678,16 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
                     }
                     __syncwarp();
                 }
-                if (g == 0) load_c(1);
             }
 #pragma unroll
             for (int q = 0; q < 8; ++q) x[1][q] = cv[1][8 + q] - x[1][q];
             store(3);
             if (w.first) {
+                int in = 0;
+                if (lane == 0) in = join(tri, [&](int n, int v) { return atomicCAS(joined, n, v); });
+                ++tri;
                 __threadfence();                      // C, before the other warps read it
-                if (tri_tile) {
+                if (__shfl_sync(0xffffffffu, in, 0)) {
                     tile_sync();
                     potrf_tile(w.s, a.k + 1, pd, F, Linv, inv_off, err, smraw);
                 }
@@ -1701,6 +1699,12 @@ __global__ void __launch_bounds__(320, 1) k_update_oz(StepArgs a, const int* __r
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*fail != 0 && wid >= 8) {                     // what may still be in flight (else all was waited for)
+        const uint32_t base = wid == 9 ? bA : bLo;
+#pragma unroll 1
+        for (int b = 0; b < 6; ++b)
+            if (issued.any(b)) oz_wait(base + 8 * b, issued.last_parity(b));
+    }
     if (wid == 8) {
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -106,9 +106,8 @@ void tiles(std::mt19937& rng, long& together, long& apart, long& kept) {
                     stays.fetch_add(1);
                     if (published.load() <= t) stuck.fetch_add(1);     // must not be
                 }
-                const bool in = first[t] && join(tri++, cas);
                 if (trouble > 0 && r() % 4 == 0) nap(r() % 300);
-                if (in) {
+                if (first[t] && join(tri++, cas)) {
                     went[w][t] = 1;
                     at_barrier[t].fetch_add(1);
                     long k = 0;

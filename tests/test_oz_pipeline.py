@@ -32,11 +32,14 @@ def _kernel(name):
 
 def test_the_kernel_waits_for_what_it_issued():
     body = _kernel("k_update_oz")
-    # every copy and every batch of MMAs is logged where it is issued, and waited for at the end
-    assert body.count("oz_copy_rows(") == body.count("copies.start(") == 2
-    assert body.count("oz_commit(") == body.count("batches.start(") == 2
-    assert "copies.last_parity(b)" in body and "batches.last_parity(b)" in body
+    # every copy and every batch of MMAs is logged where it is issued, and waited for once every
+    # warp is through, if any of them gave up
+    assert body.count("oz_copy_rows(") + body.count("oz_commit(") == body.count("issued.start(") == 4
+    end = body[body.rindex("__syncthreads();"):]
+    assert re.search(r"if \(\*fail != 0 && wid >= 8\)", end) and "issued.last_parity(b)" in end
+    assert end.index("issued.last_parity(b)") < end.index("tcgen05.dealloc")
     # the barriers without a limit are reached by all of the eight warps that joined, or by none
     assert "bar.sync" not in body and body.count("tile_sync()") == body.count("potrf_tile(") == 1
-    assert re.search(r"if \(tri_tile\) \{\s*tile_sync\(\);\s*potrf_tile\(", body)
-    assert "tri_tile = w.first && join(" in body and "left = leave(" in body
+    assert re.search(r"in = join\(tri,.*?if \(__shfl_sync\(0xffffffffu, in, 0\)\) \{\s*tile_sync\(\);\s*potrf_tile\(",
+                     body, re.S)
+    assert "left = leave(tri, swap_joined)" in body
