@@ -5,7 +5,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <type_traits>
 
 namespace sankhya {
 namespace dev {
@@ -437,15 +436,34 @@ __global__ void __launch_bounds__(256, NPT == 1 ? 3 : 4) k_layer_bwd(Side side, 
     }
 }
 
+// k_grad_w's sums over the nodes n0 .. n1 - 1, with a choice at each product (any values).
+__device__ __noinline__ void grad_w_masked(int n0, int n1, const float* __restrict__ g, const float* __restrict__ x1,
+                                           const float* __restrict__ x2, float* __restrict__ dW1,
+                                           float* __restrict__ dW2, float* __restrict__ db) {
+    const int o = threadIdx.x & 63, k0 = (threadIdx.x >> 6) * 32;       // output o, 32 of the 128 columns
+    const float* x = k0 < H ? x1 + k0 : x2 + k0 - H;
+    float sum[32] = {}, sumb = 0.f;
+    for (int n = n0; n < n1; ++n) {
+        const float gv = g[static_cast<size_t>(n) * H + o];
+        sumb += gv;
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+            if (gv != 0.f) sum[c] += gv * x[static_cast<size_t>(n) * H + c];
+    }
+    float* dW = (k0 < H ? dW1 + k0 : dW2 + k0 - H) + o * H;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) atomicAdd(dW + c, sum[c]);
+    if (k0 == 0) atomicAdd(db + o, sumb);
+}
+
 // dW1[o][k] += sum_node g[node][o] x1[node][k], dW2 with x2, db[o] += sum_node g[node][o] over
 // `chunk` nodes a block: a 64 x 128 product with the nodes as its inner dimension. Thread
 // (og, kg) keeps 4 outputs x 8 of the 128 columns in registers (32 multiply-adds per three
 // 16-byte shared loads); the next 32 nodes are loaded while the present ones are summed. One
 // output column group per thread with the operands from the L1 took 182 us a matrix at
 // 19,000 / 48,000 nodes; now 20 us for both. Sums of 32 nodes are added up separately. A
-// masked gradient (0) leaves its node's features out whatever they are: a stage with an
-// infinity or a NaN among its features, which 0 times it would spread, is summed with a
-// choice at each product (the sum of a thread's features is not finite in such a stage).
+// masked gradient (0) leaves its node's features out whatever they are: a block with a sum that
+// is not finite, where 0 may have met an infinity or a NaN, adds up once more by grad_w_masked().
 __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const float* __restrict__ g,
                                                 const float* __restrict__ x1, const float* __restrict__ x2,
                                                 float* __restrict__ dW1, float* __restrict__ dW2,
@@ -472,19 +490,18 @@ __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const floa
     };
     load(n0);
     for (int n = n0; n < n1; n += S) {
-        float all[4];                              // sums of this thread's features
 #pragma unroll
         for (int u = 0; u < 2; ++u) reinterpret_cast<float4*>(gs)[tid + 256 * u] = pg[u];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int e = tid + 256 * (u & 1);
             reinterpret_cast<float4*>(xs)[(e >> 4) * 32 + (u < 2 ? 0 : 16) + (e & 15)] = px[u];
-            all[u] = (px[u].x + px[u].y) + (px[u].z + px[u].w);
         }
-        const bool choose = __syncthreads_or(!isfinite((all[0] + all[1]) + (all[2] + all[3])));
+        __syncthreads();
         if (n + S < n1) load(n + S);
         float acc[4][8] = {}, accb[4] = {};
-        auto add = [&](int nn, auto masked) {
+#pragma unroll 4
+        for (int nn = 0; nn < S; ++nn) {
             float gv[4], xv[8];
             *reinterpret_cast<float4*>(gv) = *reinterpret_cast<const float4*>(gs + nn * H + 4 * og);
             *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(xs + nn * 2 * H + 8 * kg);
@@ -493,16 +510,8 @@ __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const floa
             for (int o = 0; o < 4; ++o) {
                 accb[o] += gv[o];
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    if (!masked || gv[o] != 0.f) acc[o][c] += gv[o] * xv[c];
+                for (int c = 0; c < 8; ++c) acc[o][c] += gv[o] * xv[c];
             }
-        };
-        if (choose) {
-#pragma unroll 1
-            for (int nn = 0; nn < S; ++nn) add(nn, std::true_type{});
-        } else {
-#pragma unroll 4
-            for (int nn = 0; nn < S; ++nn) add(nn, std::false_type{});
         }
 #pragma unroll
         for (int o = 0; o < 4; ++o) {
@@ -511,6 +520,15 @@ __global__ void __launch_bounds__(256) k_grad_w(int nodes, int chunk, const floa
             for (int c = 0; c < 8; ++c) sum[o][c] += acc[o][c];
         }
         __syncthreads();
+    }
+    float none = 0.f;                              // stays 0 over finite sums
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) none += 0.f * sum[o][c];
+    if (__syncthreads_or(none != 0.f)) {
+        grad_w_masked(n0, n1, g, x1, x2, dW1, dW2, db);
+        return;
     }
     float* dW = (kg < 8 ? dW1 : dW2) + 8 * (kg & 7);
 #pragma unroll

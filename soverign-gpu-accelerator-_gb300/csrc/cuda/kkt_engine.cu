@@ -1417,7 +1417,7 @@ __device__ __forceinline__ int block_row_of(int lb) {
 // first: their accumulators are free for the next tile as soon as they are in registers, while
 // the upper levels' products run. Bound by the epilogue: of the 16,000 cycles that a tile takes
 // at 3,260 rows an SM quarter's FP64 subtractions need 4,100 (64 cycles an instruction), its integer
-// instructions 4,600 and its conversions 2,600, one after the other in each warp, so these are kept
+// instructions 4,700 and its conversions 2,600, one after the other in each warp, so these are kept
 // apart in neighbouring groups of columns and have no branch between them; the tensor pipe is busy
 // for 22% of the time. The block
 // with a front's first tile factors the next diagonal tile and waits for it without polling.
